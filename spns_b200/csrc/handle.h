@@ -299,20 +299,6 @@ int spns_fail(spns_handle *h, int code, const char *fmt, ...);
             return spns_fail(h, SPNS_ERR_CUDA, "launch failed: %s (%s:%d)", cudaGetErrorString(e_), __FILE__, __LINE__); \
     } while (0)
 
-#define DISPATCH(Lval, call)                                                                 \
-    switch (Lval) {                                                                          \
-    case 48: { constexpr int LL = 48; call; } break;                                         \
-    case 72: { constexpr int LL = 72; call; } break;                                         \
-    case 96: { constexpr int LL = 96; call; } break;                                         \
-    case 144: { constexpr int LL = 144; call; } break;                                       \
-    case 192: { constexpr int LL = 192; call; } break;                                       \
-    case 288: { constexpr int LL = 288; call; } break;                                       \
-    case 384: { constexpr int LL = 384; call; } break;                                       \
-    case 768: { constexpr int LL = 768; call; } break;                                       \
-    case 1536: { constexpr int LL = 1536; call; } break;                                     \
-    default: return spns_fail(h, SPNS_ERR_UNSUPPORTED_SIZE, "FFT length %d is not compiled", Lval); \
-    }
-
 // Twiddle table w_L^m = exp(-2 pi i m / L), computed in extended precision, followed
 // by the per-stage sub-tables w_n^m = w_L^{m L/n} (copies of base entries) for every
 // divisor n < L of L, in increasing n (spns::tw_sub_offset), and the power tables
@@ -369,16 +355,30 @@ struct PrecOps {
 };
 
 // Lengths with batched pass kernels (ensembles of small boxes).
-#define SPNS_DISPATCH_BATCH(Lval, call)                                                     \
-    switch (Lval) {                                                                          \
-    case 48: { constexpr int LL = 48; call; } break;                                         \
-    case 72: { constexpr int LL = 72; call; } break;                                         \
-    case 96: { constexpr int LL = 96; call; } break;                                         \
-    case 144: { constexpr int LL = 144; call; } break;                                       \
-    case 192: { constexpr int LL = 192; call; } break;                                       \
-    default: return spns_fail(h, SPNS_ERR_UNSUPPORTED_SIZE, "no batched kernels at FFT length %d", Lval); \
+constexpr bool spns_batch_length(int L) { return L == 48 || L == 72 || L == 96 || L == 144 || L == 192; }
+// Launches of the pass kernels of one FFT length in one precision (len_launch.cuh;
+// one object file per pair).
+struct LenTable {
+    // pass k (1..5) of `mode` on the handle's stream; select: in the shape the handle chose
+    cudaError_t (*pass)(spns_handle *h, int k, int mode, bool select, double *phys);
+    // the same for the n members of a batched class
+    cudaError_t (*batch)(spns_handle *h, const spns::BatchMember *tab, int n, cudaStream_t st, int k, int mode);
+    // batched 1-D transforms of contiguous lines / of the strided axis of [nbatch][L][ncols] arrays
+    cudaError_t (*lines)(spns_handle *h, void *data, long long batch, bool inv);
+    cudaError_t (*cols)(spns_handle *h, void *data, int ncols, int nbatch, bool inv);
+};
+#define SPNS_LEN_DECL(n) extern const LenTable spns_len_f64_##n, spns_len_f32_##n;
+SPNS_FOR_EACH_LENGTH(SPNS_LEN_DECL)
+#undef SPNS_LEN_DECL
+// Table of a compiled length (spns_create refuses the others).
+template <typename T> inline const LenTable *spns_len_table(int L) {
+    switch (L) {
+#define SPNS_LEN_CASE(n) case n: return sizeof(T) == 8 ? &spns_len_f64_##n : &spns_len_f32_##n;
+    SPNS_FOR_EACH_LENGTH(SPNS_LEN_CASE)
+#undef SPNS_LEN_CASE
+    default: return nullptr;
     }
-inline bool spns_batch_length(int L) { return L == 48 || L == 72 || L == 96 || L == 144 || L == 192; }
+}
 extern const PrecOps spns_ops_f64;
 extern const PrecOps spns_ops_f32;
 inline const PrecOps &spns_ops(const spns_handle *h) { return h->prec == SPNS_FP64 ? spns_ops_f64 : spns_ops_f32; }

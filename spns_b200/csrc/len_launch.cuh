@@ -1,0 +1,331 @@
+// len_launch.cuh -- launches of the pass kernels of one FFT length, templated on the
+// arithmetic type T of the transforms (double: FP64 form; float: compensated FP32
+// hi/lo form).  spns_len.cu instantiates one (precision, length) per object, so the
+// lengths compile in parallel, and exports its LenTable; passes.cuh runs the step
+// through those tables.
+#pragma once
+#include "handle.h"
+
+#include <cudaTypedefs.h>
+
+#include <algorithm>
+
+template <typename T> struct LenLaunch {
+    using C = spns::cx<T>;
+
+    static C *U(spns_handle *h, int f = 0) { return (C *)h->U + (long long)f * h->g.S0; }
+    static const C *tw(spns_handle *h, int L) { return (const C *)h->tw[L]; }
+
+    template <int L, int MODE, int ALT = 0> static cudaError_t launch_k1(spns_handle *h) {
+        using S = ShapeK1A<T, L, ALT>;
+        auto kern = spns::k1_inv_x<T, L, S::E, S::P, MODE>;
+        cudaError_t e = spns_set_smem(kern, S::SMEM_ROW);
+        if (e != cudaSuccess) return e;
+        dim3 grid((h->g.Kz + S::P - 1) / S::P, h->g.Ky);
+        kern<<<grid, S::THREADS, S::SMEM_ROW, h->st>>>(h->g, U(h, 0), U(h, 1), U(h, 2), (C *)h->B1, tw(h, L));
+        return cudaGetLastError();
+    }
+    // ---- x/y passes with TMA-moved tiles (double precision, axis_tma.cuh) ----
+    // Tensor map {2*Kz doubles, rows, lines, fields} over an input buffer, cached per
+    // (pass, buffer) in the handle.  Box {2P, R, 1, 1}.
+    static cudaError_t axis_map(spns_handle *h, int pass, const void *in, int rows, int lines, int fields, long long row_stride,
+                                long long line_stride, long long field_stride, int P, int R, const CUtensorMap **out) {
+        const auto key = std::make_pair(pass, in);
+        auto it = h->tmaps.find(key);
+        if (it == h->tmaps.end()) {
+            static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
+            if (!encode) {
+                void *fn = nullptr;
+                cudaDriverEntryPointQueryResult q;
+                cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q);
+                if (e != cudaSuccess || q != cudaDriverEntryPointSuccess || !fn) return e != cudaSuccess ? e : cudaErrorNotSupported;
+                encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
+            }
+            const size_t cs = sizeof(C);
+            cuuint64_t dims[4] = {(cuuint64_t)(2 * h->g.Kz), (cuuint64_t)rows, (cuuint64_t)lines, (cuuint64_t)fields};
+            cuuint64_t strides[3] = {(cuuint64_t)(row_stride * cs), (cuuint64_t)(line_stride * cs), (cuuint64_t)(field_stride * cs)};
+            cuuint32_t box[4] = {(cuuint32_t)(2 * P), (cuuint32_t)R, 1u, 1u};
+            cuuint32_t estr[4] = {1u, 1u, 1u, 1u};
+            CUtensorMap m;
+            CUresult r = encode(&m, sizeof(T) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
+                                const_cast<void *>(in), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+            if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
+            it = h->tmaps.emplace(key, m).first;
+        }
+        *out = &it->second;
+        return cudaSuccess;
+    }
+    // Persistent launch of k_axis_tma: one wave of blocks (one per SM at this shared memory).
+    template <int L, bool INV>
+    static cudaError_t launch_axis_tma(spns_handle *h, const CUtensorMap *map, const spns::AxisArgs &a, C *out) {
+        using S = AxisTmaShape<T, L>;
+        auto kern = spns::k_axis_tma<T, L, S::E, S::P, INV>;
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
+        if (e != cudaSuccess) return e;
+        constexpr int THREADS = S::P * (L / S::E);
+        int per_sm = 0;
+        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, THREADS, S::SMEM)) != cudaSuccess) return e;
+        if (per_sm < 1) return cudaErrorInvalidConfiguration;
+        const long long items = (long long)((a.Kz + S::P - 1) / S::P) * a.lines;
+        const long long blocks = std::min<long long>(items, (long long)h->sms * per_sm);
+        kern<<<(unsigned)blocks, THREADS, S::SMEM, h->st>>>(*map, a, out, tw(h, L), h->ds);
+        return cudaGetLastError();
+    }
+    // Shared-memory placement of an inverse tile needs the boxes from both ends not to overlap.
+    template <int L> static bool axis_tma_fits(int hh) {
+        const int R = SPNS_AX_TMA_R;
+        const int npos = (hh + R) / R, nneg = (hh + R - 1) / R;
+        return hh >= 1 && 2 * hh + 1 <= L && L - nneg * R >= npos * R;
+    }
+    template <int L, int MODE> static cudaError_t launch_k2_tma(spns_handle *h) {
+        using S = AxisTmaShape<T, L>;
+        const spns::Geo &g = h->g;
+        const int nin = (h->B1 == h->inv_B1 || MODE == spns::MODE_INV) ? 6 : h->nB1;
+        const CUtensorMap *map = nullptr;
+        cudaError_t e = axis_map(h, 2, h->B1, g.Ky, g.Mx, nin, (long long)g.Mx * g.Kz, g.Kz, g.S1, S::P, SPNS_AX_TMA_R, &map);
+        if (e != cudaSuccess) return e;
+        spns::AxisArgs a{};
+        a.h = g.hy; a.Kc = g.Ky; a.lines = g.Mx; a.Kz = g.Kz; a.nout = spns::Fields<MODE>::K2;
+        for (int f = 0; f < a.nout; f++) a.src |= (unsigned long long)(f < 6 ? f : f - 6) << (4 * f);
+        a.deriv_from = (MODE == spns::MODE_VEL || MODE == spns::MODE_ROT) ? 99 : 6;
+        a.s = g.sy; a.o_row = (long long)g.Mx * g.Kz; a.o_line = g.Kz; a.o_field = g.S2; a.rbox = SPNS_AX_TMA_R;
+        return launch_axis_tma<L, true>(h, map, a, (C *)h->B2);
+    }
+    template <int L, int MODE> static cudaError_t launch_k4_tma(spns_handle *h) {
+        using S = AxisTmaShape<T, L>;
+        const spns::Geo &g = h->g;
+        const int nin = MODE == spns::MODE_INV ? 9 : h->nB2;
+        const CUtensorMap *map = nullptr;
+        cudaError_t e = axis_map(h, 4, h->B2, g.My, g.Mx, nin, (long long)g.Mx * g.Kz, g.Kz, g.S2, S::P, SPNS_AX_TMA_R, &map);
+        if (e != cudaSuccess) return e;
+        spns::AxisArgs a{};
+        a.h = g.hy; a.Kc = g.Ky; a.lines = g.Mx; a.Kz = g.Kz; a.nout = spns::Fields<MODE>::NOUT;
+        for (int f = 0; f < a.nout; f++) a.src |= (unsigned long long)spns::k4_in_field<MODE>(f) << (4 * f);
+        a.deriv_from = 99;
+        a.s = g.sy; a.o_row = (long long)g.Mx * g.Kz; a.o_line = g.Kz; a.o_field = g.S1; a.rbox = SPNS_AX_TMA_R;
+        return launch_axis_tma<L, false>(h, map, a, (C *)h->B1);
+    }
+    template <int L, int MODE> static cudaError_t launch_k5_tma(spns_handle *h) {
+        using S = AxisTmaShape<T, L>;
+        const spns::Geo &g = h->g;
+        const int nin = MODE == spns::MODE_INV ? 6 : h->nB1;
+        const CUtensorMap *map = nullptr;
+        cudaError_t e = axis_map(h, 5, h->B1, g.Mx, g.Ky, nin, g.Kz, (long long)g.Mx * g.Kz, g.S1, S::P, SPNS_AX_TMA_R, &map);
+        if (e != cudaSuccess) return e;
+        spns::AxisArgs a{};
+        a.h = g.hx; a.Kc = g.Kx; a.lines = g.Ky; a.Kz = g.Kz; a.nout = spns::Fields<MODE>::NOUT;
+        for (int f = 0; f < a.nout; f++) a.src |= (unsigned long long)f << (4 * f);
+        a.deriv_from = 99;
+        a.s = g.sx; a.o_row = g.Kz; a.o_line = (long long)g.Kx * g.Kz; a.o_field = g.S0; a.rbox = SPNS_AX_TMA_R;
+        return launch_axis_tma<L, false>(h, map, a, (C *)h->B2);
+    }
+
+    template <int L, int MODE, int ALT = 0> static cudaError_t launch_k2(spns_handle *h) {
+        if constexpr (AxisTmaShape<T, L>::ON && ALT == 0)
+            if (axis_tma_fits<L>(h->g.hy)) return launch_k2_tma<L, MODE>(h);
+        using S = ShapeK2A<T, L, ALT>;
+        auto kern = spns::k2_inv_y<T, L, S::E, S::P, MODE>;
+        cudaError_t e = spns_set_smem(kern, S::SMEM_ROW);
+        if (e != cudaSuccess) return e;
+        dim3 grid((h->g.Kz + S::P - 1) / S::P, h->g.Mx);
+        kern<<<grid, S::THREADS, S::SMEM_ROW, h->st>>>(h->g, (const C *)h->B1, (C *)h->B2, tw(h, L));
+        return cudaGetLastError();
+    }
+    // Rotational z pass staged pair by pair with bulk copies (zpass_staged.cuh),
+    // persistent: one wave of blocks over the SMs.
+    template <int L> static cudaError_t launch_k3_staged(spns_handle *h) {
+        using ZS = ZStagedShape<T, L>;
+        using LY = spns::ZStagedLayout<T, L, ZS::E, ZS::PB, ZS::SLOTS>;
+        auto kern = spns::k3_rot_staged<T, L, ZS::E, ZS::PB, ZS::SLOTS, ZS::MINB>;
+        const size_t smem = LY::smem_bytes(h->g.Kz);
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        constexpr int THREADS = ZS::PB * LY::Q;
+        int dev = 0, sms = 0, per_sm = 0;
+        if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+        if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, THREADS, smem)) != cudaSuccess) return e;
+        if (per_sm < 1) return cudaErrorInvalidConfiguration;
+        const long long groups = ((long long)h->g.Mx * h->g.My + ZS::PB - 1) / ZS::PB;
+        long long blocks = (long long)sms * per_sm;
+        if (blocks > groups) blocks = groups;
+        kern<<<(unsigned)blocks, THREADS, smem, h->st>>>(h->g, (C *)h->B2, h->c, h->ds, tw(h, L));
+        return cudaGetLastError();
+    }
+    template <int L, int MODE, int ALT = 0> static cudaError_t launch_k3(spns_handle *h, double *phys) {
+        if constexpr (MODE == spns::MODE_ROT && ALT == 0 && ZStagedShape<T, L>::ON) return launch_k3_staged<L>(h);
+        using S3 = Shape3<T, L, MODE, ALT>;
+        constexpr bool STAGE_ROT = MODE == spns::MODE_ROT && ShapeSel<T>::Z_STAGE;
+        constexpr bool STAGE_LES = MODE == spns::MODE_LES && sizeof(T) == 4 && SPNS_F32_Z_STAGE_LES;
+        constexpr bool STAGE = STAGE_ROT || STAGE_LES;
+        auto kern = spns::k3_z<T, L, S3::E, S3::P, MODE, STAGE>;
+        constexpr size_t stage_fields = STAGE_ROT ? 2 * spns::K3StagePairs<T>::N : STAGE_LES ? 9 : 0;
+        // the staging is sized by Kz at run time: at most L/2+1 values per field and pencil
+        static_assert(S3::SMEM + (size_t)S3::P * stage_fields * (L / 2 + 1) * sizeof(C) <= 227 * 1024,
+                      "z-pass shared memory (exchange, physical slots and staging) exceeds 227 KB for this shape");
+        const size_t smem = S3::SMEM + (size_t)S3::P * stage_fields * h->g.Kz * sizeof(C);
+        cudaError_t e = spns_set_smem(kern, smem);
+        if (e != cudaSuccess) return e;
+        const long long npen = (long long)h->g.Mx * h->g.My;
+        dim3 grid((unsigned)((npen + S3::P - 1) / S3::P));
+        kern<<<grid, S3::THREADS, smem, h->st>>>(h->g, (C *)h->B2, h->c, h->ds, phys, tw(h, L));
+        return cudaGetLastError();
+    }
+    template <int L, int MODE, int ALT = 0> static cudaError_t launch_k4(spns_handle *h) {
+        if constexpr (AxisTmaShape<T, L>::ON && ALT == 0 && MODE != spns::MODE_LES)
+            if (2 * h->g.hy + 1 <= L) return launch_k4_tma<L, MODE>(h);
+        using S = ShapeK2A<T, L, ALT>;
+        auto kern = spns::k4_fwd_y<T, L, S::E, S::P, MODE>;
+        cudaError_t e = spns_set_smem(kern, S::SMEM_ROW);
+        if (e != cudaSuccess) return e;
+        dim3 grid((h->g.Kz + S::P - 1) / S::P, h->g.Mx);
+        kern<<<grid, S::THREADS, S::SMEM_ROW, h->st>>>(h->g, (const C *)h->B2, (C *)h->B1, tw(h, L));
+        return cudaGetLastError();
+    }
+    template <int L, int MODE, int ALT = 0> static cudaError_t launch_k5(spns_handle *h) {
+        if constexpr (AxisTmaShape<T, L>::ON && ALT == 0 && MODE != spns::MODE_LES)
+            if (2 * h->g.hx + 1 <= L) return launch_k5_tma<L, MODE>(h);
+        using S = ShapeK5A<T, L, ALT>;
+        auto kern = spns::k5_fwd_x<T, L, S::E, S::P, MODE>;
+        cudaError_t e = spns_set_smem(kern, S::SMEM_ROW);
+        if (e != cudaSuccess) return e;
+        dim3 grid((h->g.Kz + S::P - 1) / S::P, h->g.Ky);
+        kern<<<grid, S::THREADS, S::SMEM_ROW, h->st>>>(h->g, (const C *)h->B1, (C *)h->B2, tw(h, L));
+        return cudaGetLastError();
+    }
+    // Launch of pass K1..K5 in the shape the handle selected (shape_alt).
+#define SPNS_SELECT(name, idx, ...)                                                              \
+    template <int L, int MODE> static cudaError_t sel_##name(spns_handle *h) {                    \
+        if constexpr (shape_alt_ok<L, MODE>())                                                    \
+            if (h->shape_alt[idx]) return launch_##name<L, MODE, 1>(h __VA_ARGS__);               \
+        return launch_##name<L, MODE, 0>(h __VA_ARGS__);                                          \
+    }
+    SPNS_SELECT(k1, 1)
+    SPNS_SELECT(k2, 2)
+    SPNS_SELECT(k3, 3, , nullptr)
+    SPNS_SELECT(k4, 4)
+    SPNS_SELECT(k5, 5)
+#undef SPNS_SELECT
+
+    // Batched 1-D FFTs for the 2-D edge planes.
+    template <int L, bool INV> static cudaError_t launch_lines(spns_handle *h, C *data, long long batch) {
+        using S = Shape<T, L>;
+        auto kern = spns::k_lines<T, L, S::E, S::P, INV>;
+        cudaError_t e = spns_set_smem(kern, S::SMEM_PEN);
+        if (e != cudaSuccess) return e;
+        kern<<<(unsigned)((batch + S::P - 1) / S::P), S::THREADS, S::SMEM_PEN, h->st>>>(data, batch, tw(h, L));
+        return cudaGetLastError();
+    }
+    template <int L, bool INV> static cudaError_t launch_cols(spns_handle *h, C *data, int ncols, int nbatch) {
+        using S = Shape<T, L>;
+        auto kern = spns::k_cols<T, L, S::E, S::P, INV>;
+        cudaError_t e = spns_set_smem(kern, S::SMEM_ROW);
+        if (e != cudaSuccess) return e;
+        dim3 grid((ncols + S::P - 1) / S::P, nbatch);
+        kern<<<grid, S::THREADS, S::SMEM_ROW, h->st>>>(data, ncols, tw(h, L));
+        return cudaGetLastError();
+    }
+    // ---- batched launches: one per pass for the members of a table, all of h0's class ----
+    template <int L, int MODE, int ALT> static cudaError_t launch_k1b(spns_handle *h, const spns::BatchMember *tab, int n, cudaStream_t st) {
+        using S = ShapeK1A<T, L, ALT>;
+        auto kern = spns::k1_inv_x_batch<T, L, S::E, S::P, MODE>;
+        cudaError_t e = spns_set_smem(kern, S::SMEM_ROW);
+        if (e != cudaSuccess) return e;
+        kern<<<dim3((h->g.Kz + S::P - 1) / S::P, h->g.Ky, n), S::THREADS, S::SMEM_ROW, st>>>(h->g, tab, tw(h, L));
+        return cudaGetLastError();
+    }
+    template <int L, int MODE, int ALT> static cudaError_t launch_k2b(spns_handle *h, const spns::BatchMember *tab, int n, cudaStream_t st) {
+        using S = ShapeK2A<T, L, ALT>;
+        auto kern = spns::k2_inv_y_batch<T, L, S::E, S::P, MODE>;
+        cudaError_t e = spns_set_smem(kern, S::SMEM_ROW);
+        if (e != cudaSuccess) return e;
+        kern<<<dim3((h->g.Kz + S::P - 1) / S::P, h->g.Mx, n), S::THREADS, S::SMEM_ROW, st>>>(h->g, tab, tw(h, L));
+        return cudaGetLastError();
+    }
+    template <int L, int MODE, int ALT> static cudaError_t launch_k3b(spns_handle *h, const spns::BatchMember *tab, int n, cudaStream_t st) {
+        using S3 = Shape3<T, L, MODE, ALT>;
+        constexpr bool STAGE = MODE == spns::MODE_LES && sizeof(T) == 4 && SPNS_F32_Z_STAGE_LES;
+        auto kern = spns::k3_z_batch<T, L, S3::E, S3::P, MODE, STAGE>;
+        const size_t smem = S3::SMEM + (size_t)S3::P * (STAGE ? 9 : 0) * h->g.Kz * sizeof(C);
+        cudaError_t e = spns_set_smem(kern, smem);
+        if (e != cudaSuccess) return e;
+        const long long npen = (long long)h->g.Mx * h->g.My;
+        kern<<<dim3((unsigned)((npen + S3::P - 1) / S3::P), 1, n), S3::THREADS, smem, st>>>(h->g, tab, tw(h, L));
+        return cudaGetLastError();
+    }
+    template <int L, int MODE, int ALT> static cudaError_t launch_k4b(spns_handle *h, const spns::BatchMember *tab, int n, cudaStream_t st) {
+        using S = ShapeK2A<T, L, ALT>;
+        auto kern = spns::k4_fwd_y_batch<T, L, S::E, S::P, MODE>;
+        cudaError_t e = spns_set_smem(kern, S::SMEM_ROW);
+        if (e != cudaSuccess) return e;
+        kern<<<dim3((h->g.Kz + S::P - 1) / S::P, h->g.Mx, n), S::THREADS, S::SMEM_ROW, st>>>(h->g, tab, tw(h, L));
+        return cudaGetLastError();
+    }
+    template <int L, int MODE, int ALT> static cudaError_t launch_k5b(spns_handle *h, const spns::BatchMember *tab, int n, cudaStream_t st) {
+        using S = ShapeK5A<T, L, ALT>;
+        auto kern = spns::k5_fwd_x_batch<T, L, S::E, S::P, MODE>;
+        cudaError_t e = spns_set_smem(kern, S::SMEM_ROW);
+        if (e != cudaSuccess) return e;
+        kern<<<dim3((h->g.Kz + S::P - 1) / S::P, h->g.Ky, n), S::THREADS, S::SMEM_ROW, st>>>(h->g, tab, tw(h, L));
+        return cudaGetLastError();
+    }
+#define SPNS_SELECT_B(name, idx)                                                                                       \
+    template <int L, int MODE> static cudaError_t sel_##name(spns_handle *h, const spns::BatchMember *tab, int n, cudaStream_t st) { \
+        if constexpr (shape_alt_ok<L, MODE>())                                                                         \
+            if (h->shape_alt[idx]) return launch_##name<L, MODE, 1>(h, tab, n, st);                                    \
+        return launch_##name<L, MODE, 0>(h, tab, n, st);                                                               \
+    }
+    SPNS_SELECT_B(k1b, 1)
+    SPNS_SELECT_B(k2b, 2)
+    SPNS_SELECT_B(k3b, 3)
+    SPNS_SELECT_B(k4b, 4)
+    SPNS_SELECT_B(k5b, 5)
+#undef SPNS_SELECT_B
+
+    // ---- the table of one length ----
+    // Pass k (1..5: K1..K5) of `mode`; `select`: in the shape the handle chose for it
+    // (steps), else in the default shape.  `phys` goes to the z pass.
+    template <int L, int MODE> static cudaError_t run_mode(spns_handle *h, int k, bool select, double *phys) {
+        switch (k) {
+        case 1: return select ? sel_k1<L, MODE>(h) : launch_k1<L, MODE>(h);
+        case 2: return select ? sel_k2<L, MODE>(h) : launch_k2<L, MODE>(h);
+        case 3: return select ? sel_k3<L, MODE>(h) : launch_k3<L, MODE>(h, phys);
+        case 4: return select ? sel_k4<L, MODE>(h) : launch_k4<L, MODE>(h);
+        default: return select ? sel_k5<L, MODE>(h) : launch_k5<L, MODE>(h);
+        }
+    }
+    template <int L> static cudaError_t run_vel(spns_handle *h, int k, double *phys) {
+        return k == 1 ? launch_k1<L, spns::MODE_VEL>(h) : k == 2 ? launch_k2<L, spns::MODE_VEL>(h) : launch_k3<L, spns::MODE_VEL>(h, phys);
+    }
+    template <int L> static cudaError_t pass(spns_handle *h, int k, int mode, bool select, double *phys) {
+        switch (mode) {
+        case spns::MODE_VEL: return run_vel<L>(h, k, phys);
+        case spns::MODE_ROT: return run_mode<L, spns::MODE_ROT>(h, k, select, phys);
+        case spns::MODE_ADV: return run_mode<L, spns::MODE_ADV>(h, k, select, phys);
+        case spns::MODE_LES: return run_mode<L, spns::MODE_LES>(h, k, select, phys);
+        default: return run_mode<L, spns::MODE_INV>(h, k, select, phys);
+        }
+    }
+    template <int L, int MODE> static cudaError_t batch_mode(spns_handle *h, const spns::BatchMember *tab, int n, cudaStream_t st, int k) {
+        switch (k) {
+        case 1: return sel_k1b<L, MODE>(h, tab, n, st);
+        case 2: return sel_k2b<L, MODE>(h, tab, n, st);
+        case 3: return sel_k3b<L, MODE>(h, tab, n, st);
+        case 4: return sel_k4b<L, MODE>(h, tab, n, st);
+        default: return sel_k5b<L, MODE>(h, tab, n, st);
+        }
+    }
+    template <int L> static cudaError_t batch(spns_handle *h, const spns::BatchMember *tab, int n, cudaStream_t st, int k, int mode) {
+        if constexpr (spns_batch_length(L))
+            return mode == spns::MODE_LES ? batch_mode<L, spns::MODE_LES>(h, tab, n, st, k) : batch_mode<L, spns::MODE_ADV>(h, tab, n, st, k);
+        return cudaErrorNotSupported;
+    }
+    template <int L> static cudaError_t lines(spns_handle *h, void *data, long long batch, bool inv) {
+        return inv ? launch_lines<L, true>(h, (C *)data, batch) : launch_lines<L, false>(h, (C *)data, batch);
+    }
+    template <int L> static cudaError_t cols(spns_handle *h, void *data, int ncols, int nbatch, bool inv) {
+        return inv ? launch_cols<L, true>(h, (C *)data, ncols, nbatch) : launch_cols<L, false>(h, (C *)data, ncols, nbatch);
+    }
+    template <int L> static constexpr LenTable table() { return LenTable{&pass<L>, &batch<L>, &lines<L>, &cols<L>}; }
+};
