@@ -208,8 +208,12 @@ __host__ __device__ constexpr int tw_pow_offset(int L, int n, int r) {
 }
 __host__ __device__ constexpr int tw_full_size(int L) { return 4 * tw_table_size(L); }
 
-template <bool WARP> __device__ __forceinline__ void stage_barrier() {
-    if constexpr (WARP) __syncwarp(); else __syncthreads();
+// Barrier of an exchange: the block's (WARP 0), the whole warp's (1), or that of the lanes
+// of the mask WARP, the only ones that run the transform.
+template <unsigned WARP> __device__ __forceinline__ void stage_barrier() {
+    if constexpr (WARP == 0) __syncthreads();
+    else if constexpr (WARP == 1) __syncwarp();
+    else __syncwarp(WARP);
 }
 
 // Single precision: the powers w^r of a butterfly's twiddle.  With SPNS_F32_TW_POW the
@@ -234,7 +238,7 @@ __device__ __forceinline__ void twiddle_powers(cx<T> (&wp)[R], const cx<T> *__re
     }
 }
 
-template <typename T, int L, int E, bool INV, bool WARP, int S, class SM>
+template <typename T, int L, int E, bool INV, unsigned WARP, int S, class SM>
 __device__ __forceinline__ void fft_run(cx<T> (&v)[E], SM sm, int q, const cx<T> *__restrict__ tw) {
     using PL = Plan<L, E, INV>;
     constexpr int R = PL::radix(S);
@@ -367,16 +371,23 @@ template <int L, int E, bool INV> __device__ __forceinline__ int out_row(int q, 
     return q + PL::Q * (e / R) + (e % R) * (L / R);
 }
 
+// Opaque copy of an index: the row and address arithmetic that depends on it is
+// recomputed where it is used instead of being hoisted out of a loop over fields or
+// pencils and kept live in registers for every register slot.
+__device__ __forceinline__ int opaque(int q) {
+    int r;
+    asm volatile("mov.b32 %0, %1;" : "=r"(r) : "r"(q));
+    return r;
+}
+
 // The thread index goes through an opaque move so that the shared-memory
 // addresses of the stages are recomputed per transform instead of being kept
 // live across every transform of a kernel (which exhausts the register file).
 // WARP=true only where each pencil's threads lie in one warp (Q divides 32 in a
 // pencil-major thread layout).
-template <typename T, int L, int E, bool INV, class SM, bool WARP = false>
+template <typename T, int L, int E, bool INV, class SM, unsigned WARP = 0>
 __device__ __forceinline__ void fft(cx<T> (&v)[E], SM sm, int q, const cx<T> *__restrict__ tw) {
-    int qq;
-    asm volatile("mov.b32 %0, %1;" : "=r"(qq) : "r"(q));
-    fft_run<T, L, E, INV, WARP, 0, SM>(v, sm, qq, tw);
+    fft_run<T, L, E, INV, WARP, 0, SM>(v, sm, opaque(q), tw);
 }
 
 // Accessor: tile of P pencils stored row-major [row][P] (pencil index fastest).

@@ -9,6 +9,7 @@
 #include "edge_kernels.cuh"
 #include "zpass_staged.cuh"
 #include "axis_tma.cuh"
+#include "zpass_field.cuh"
 
 #include <cuda_runtime.h>
 
@@ -213,6 +214,58 @@ template <typename T, int L, int MODE, int ALT = 0> struct Shape3 {
     static constexpr int P = P0 <= PMAX ? P0 : PMAX >= 16 ? 16 : PMAX >= 8 ? 8 : PMAX >= 4 ? 4 : PMAX >= 2 ? 2 : 1;
     static constexpr int THREADS = P * Q;
     static constexpr size_t SMEM = PER_PEN * P;
+};
+
+// z pass with the fields transformed side by side (k3_field, zpass_field.cuh).  E values
+// per thread, NT teams of Q = L/E threads (a whole number of warps), PB pencils per block,
+// and the register budget that sets the resident blocks.
+#ifndef SPNS_ZF_E_LONG
+#define SPNS_ZF_E_LONG 12
+#endif
+#ifndef SPNS_ZF_R24
+#define SPNS_ZF_R24 168
+#endif
+#ifndef SPNS_ZF_R12
+#define SPNS_ZF_R12 112
+#endif
+#ifndef SPNS_ZF_R6
+#define SPNS_ZF_R6 80
+#endif
+#ifndef SPNS_F32_ZF_E_LONG
+#define SPNS_F32_ZF_E_LONG 12
+#endif
+#ifndef SPNS_ZF_E144
+#define SPNS_ZF_E144 12
+#endif
+#ifndef SPNS_F32_ZF_R24
+#define SPNS_F32_ZF_R24 104
+#endif
+#ifndef SPNS_F32_ZF_R12
+#define SPNS_F32_ZF_R12 80
+#endif
+#ifndef SPNS_F32_ZF_R6
+#define SPNS_F32_ZF_R6 64
+#endif
+#ifndef SPNS_ZF_ROT
+#define SPNS_ZF_ROT 0
+#endif
+template <typename T, int L, int MODE, int ALT = 0> struct ZFieldShape {
+    static constexpr bool D = sizeof(T) == 8;
+    static constexpr int E = ALT ? SPNS_ALT_E : L >= 768 ? 24 : L == 384 ? (D ? SPNS_ZF_E_LONG : SPNS_F32_ZF_E_LONG) : L == 144 ? SPNS_ZF_E144 : 12;
+    static constexpr int Q = L / E;
+    static constexpr int NPAIR = spns::ZFieldForm<MODE>::NPAIR;
+    static constexpr bool INV = MODE == spns::MODE_INV;
+    // three warps of teams (five for the five pairs of the invariants)
+    static constexpr int TPW = Q < 32 ? 32 / Q : 1;
+    static constexpr int NT = Q >= 32 ? NPAIR : (INV ? 5 : 3) * TPW;
+    static constexpr int lcm(int a, int b) { int m = a; while (m % b) m += a; return m; }
+    static constexpr int PB = lcm(NT, NPAIR) / NPAIR;
+    using LY = spns::ZFieldLayout<T, L, E, PB, NT, MODE>;
+    static constexpr int THREADS = LY::THREADS;
+    static constexpr int REGS = E == 24 ? (D ? SPNS_ZF_R24 : SPNS_F32_ZF_R24) : E == 12 ? (D ? SPNS_ZF_R12 : SPNS_F32_ZF_R12) : (D ? SPNS_ZF_R6 : SPNS_F32_ZF_R6);
+    static constexpr int B0 = 65536 / (REGS * THREADS);
+    static constexpr int MINB = B0 < 1 ? 1 : B0;
+    static_assert(THREADS % 32 == 0 && LY::SMEM <= 227 * 1024, "whole warps and at most 227 KB of shared memory");
 };
 
 // ---------------------------------------------------------------------------

@@ -153,7 +153,28 @@ template <typename T> struct LenLaunch {
         kern<<<(unsigned)blocks, THREADS, smem, h->st>>>(h->g, (C *)h->B2, h->c, h->ds, tw(h, L));
         return cudaGetLastError();
     }
+    // Persistent launch of k3_field: one wave of blocks.
+    template <int L, int MODE, int ALT> static cudaError_t launch_k3_field(spns_handle *h, double *nut) {
+        using S = ZFieldShape<T, L, MODE, ALT>;
+        auto kern = spns::k3_field<T, L, S::E, S::PB, S::NT, MODE, S::MINB>;
+        unsigned blocks = 0;
+        cudaError_t e = wave_of_blocks(h, kern, S::THREADS, S::LY::SMEM, ((long long)h->g.Mx * h->g.My + S::PB - 1) / S::PB, &blocks);
+        if (e != cudaSuccess) return e;
+        kern<<<blocks, S::THREADS, S::LY::SMEM, h->st>>>(h->g, (C *)h->B2, h->c, h->ds, nut, tw(h, L));
+        return cudaGetLastError();
+    }
+    // Shared-memory opt-in and grid of a persistent kernel over n work items.
+    template <class K> static cudaError_t wave_of_blocks(spns_handle *h, K kern, int threads, size_t smem, long long n, unsigned *blocks) {
+        cudaError_t e = spns_set_smem(kern, smem);
+        if (e != cudaSuccess) return e;
+        int per_sm = 0;
+        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem)) != cudaSuccess) return e;
+        if (per_sm < 1) return cudaErrorInvalidConfiguration;
+        *blocks = (unsigned)std::min<long long>(n, (long long)h->sms * per_sm);
+        return cudaSuccess;
+    }
     template <int L, int MODE, int ALT = 0> static cudaError_t launch_k3(spns_handle *h, double *phys) {
+        if constexpr (MODE != spns::MODE_VEL && (MODE != spns::MODE_ROT || SPNS_ZF_ROT)) return launch_k3_field<L, MODE, ALT>(h, phys);
         if constexpr (MODE == spns::MODE_ROT && ALT == 0 && ZStagedShape<T, L>::ON) return launch_k3_staged<L>(h);
         using S3 = Shape3<T, L, MODE, ALT>;
         constexpr bool STAGE_ROT = MODE == spns::MODE_ROT && ShapeSel<T>::Z_STAGE;
@@ -244,14 +265,12 @@ template <typename T> struct LenLaunch {
         return cudaGetLastError();
     }
     template <int L, int MODE, int ALT> static cudaError_t launch_k3b(spns_handle *h, const spns::BatchMember *tab, int n, cudaStream_t st) {
-        using S3 = Shape3<T, L, MODE, ALT>;
-        constexpr bool STAGE = MODE == spns::MODE_LES && sizeof(T) == 4 && SPNS_F32_Z_STAGE_LES;
-        auto kern = spns::k3_z_batch<T, L, S3::E, S3::P, MODE, STAGE>;
-        const size_t smem = S3::SMEM + (size_t)S3::P * (STAGE ? 9 : 0) * h->g.Kz * sizeof(C);
-        cudaError_t e = spns_set_smem(kern, smem);
+        using S = ZFieldShape<T, L, MODE, ALT>;
+        auto kern = spns::k3_field_batch<T, L, S::E, S::PB, S::NT, MODE, S::MINB>;
+        unsigned blocks = 0;
+        cudaError_t e = wave_of_blocks(h, kern, S::THREADS, S::LY::SMEM, ((long long)h->g.Mx * h->g.My + S::PB - 1) / S::PB, &blocks);
         if (e != cudaSuccess) return e;
-        const long long npen = (long long)h->g.Mx * h->g.My;
-        kern<<<dim3((unsigned)((npen + S3::P - 1) / S3::P), 1, n), S3::THREADS, smem, st>>>(h->g, tab, tw(h, L));
+        kern<<<dim3(blocks, n), S::THREADS, S::LY::SMEM, st>>>(h->g, tab, tw(h, L));
         return cudaGetLastError();
     }
     template <int L, int MODE, int ALT> static cudaError_t launch_k4b(spns_handle *h, const spns::BatchMember *tab, int n, cudaStream_t st) {

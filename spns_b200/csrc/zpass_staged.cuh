@@ -97,15 +97,6 @@ __device__ __forceinline__ T &zs_slot(T (&rg)[NREG > 0 ? NREG : 1][E], T *sm_slo
     else return sm_slots[(S - NREG) * pitch + row];
 }
 
-// Opaque copy of the thread index: the row and address arithmetic that depends on
-// it is recomputed where it is used instead of being hoisted out of the pencil
-// loop and kept live in registers for every register slot.
-__device__ __forceinline__ int zs_opaque(int q) {
-    int r;
-    asm volatile("mov.b32 %0, %1;" : "=r"(r) : "r"(q));
-    return r;
-}
-
 template <typename T, int L, int E, int PB, int SLOTS_SM, int MINB>
 __global__ void __launch_bounds__(PB *(L / E), MINB) k3_rot_staged(Geo g, cx<T> *__restrict__ buf, StepConsts c, DevScalars *ds,
                                                                    const cx<T> *__restrict__ tw) {
@@ -173,7 +164,7 @@ __global__ void __launch_bounds__(PB *(L / E), MINB) k3_rot_staged(Geo g, cx<T> 
     long long grp = blockIdx.x;
     if (grp < ngrp) issue(grp, 0, 3);
     for (; grp < ngrp; grp += gridDim.x) {
-        const int q = zs_opaque(q0);
+        const int q = opaque(q0);
         const long long pen = grp * PB + sub;
         const bool ok = pen < npen;
         cx<T> *const B0 = buf + (ok ? pen : 0) * Kz;
