@@ -128,9 +128,24 @@ constexpr int SPNS_ALT_E = 6;
 template <int L, int MODE> constexpr bool shape_alt_ok() {
     return L <= SPNS_ALT_MAX_L && (MODE == spns::MODE_ROT || MODE == spns::MODE_ADV || MODE == spns::MODE_LES);
 }
+// Forward passes of the LES form hold two arrays of values per thread (G_i and the stress
+// folded into it).
+#ifndef SPNS_LES_E
+#define SPNS_LES_E 12
+#endif
+#ifndef SPNS_LES_T4
+#define SPNS_LES_T4 256
+#endif
+#ifndef SPNS_LES_T5
+#define SPNS_LES_T5 256
+#endif
 template <typename T, int L, int ALT> using ShapeK1A = typename std::conditional<ALT != 0, ShapeT<T, L, SPNS_ALT_E, ShapeSel<T>::K1_T>, ShapeK1<T, L>>::type;
 template <typename T, int L, int ALT> using ShapeK2A = typename std::conditional<ALT != 0, ShapeT<T, L, SPNS_ALT_E, ShapeSel<T>::K2_T>, ShapeK2<T, L>>::type;
-template <typename T, int L, int ALT> using ShapeK5A = typename std::conditional<ALT != 0, ShapeT<T, L, SPNS_ALT_E, ShapeSel<T>::K5_T>, ShapeK5<T, L>>::type;
+template <typename T, int L, int MODE, int ALT> using ShapeK4A =
+    typename std::conditional<ALT != 0 || MODE != spns::MODE_LES, ShapeK2A<T, L, ALT>, ShapeT<T, L, SPNS_LES_E, SPNS_LES_T4>>::type;
+template <typename T, int L, int MODE, int ALT> using ShapeK5A =
+    typename std::conditional<ALT != 0, ShapeT<T, L, SPNS_ALT_E, ShapeSel<T>::K5_T>,
+                              typename std::conditional<MODE != spns::MODE_LES, ShapeK5<T, L>, ShapeT<T, L, SPNS_LES_E, SPNS_LES_T5>>::type>::type;
 
 // Rotational z pass with pair-by-pair bulk-copy staging, persistent
 // (k3_rot_staged, zpass_staged.cuh): used at lengths from SPNS_ZS_MIN_L up to 768.

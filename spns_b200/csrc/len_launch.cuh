@@ -19,10 +19,11 @@ template <typename T> struct LenLaunch {
     template <int L, int MODE, int ALT = 0> static cudaError_t launch_k1(spns_handle *h) {
         using S = ShapeK1A<T, L, ALT>;
         auto kern = spns::k1_inv_x<T, L, S::E, S::P, MODE>;
-        cudaError_t e = spns_set_smem(kern, S::SMEM_ROW);
+        constexpr size_t smem = spns::K1Smem<T, L, S::E, S::P, MODE>::BYTES;
+        cudaError_t e = spns_set_smem(kern, smem);
         if (e != cudaSuccess) return e;
         dim3 grid((h->g.Kz + S::P - 1) / S::P, h->g.Ky);
-        kern<<<grid, S::THREADS, S::SMEM_ROW, h->st>>>(h->g, U(h, 0), U(h, 1), U(h, 2), (C *)h->B1, tw(h, L));
+        kern<<<grid, S::THREADS, smem, h->st>>>(h->g, U(h, 0), U(h, 1), U(h, 2), (C *)h->B1, tw(h, L));
         return cudaGetLastError();
     }
     // ---- x/y passes with TMA-moved tiles (double precision, axis_tma.cuh) ----
@@ -196,7 +197,7 @@ template <typename T> struct LenLaunch {
     template <int L, int MODE, int ALT = 0> static cudaError_t launch_k4(spns_handle *h) {
         if constexpr (AxisTmaShape<T, L>::ON && ALT == 0 && MODE != spns::MODE_LES)
             if (2 * h->g.hy + 1 <= L) return launch_k4_tma<L, MODE>(h);
-        using S = ShapeK2A<T, L, ALT>;
+        using S = ShapeK4A<T, L, MODE, ALT>;
         auto kern = spns::k4_fwd_y<T, L, S::E, S::P, MODE>;
         cudaError_t e = spns_set_smem(kern, S::SMEM_ROW);
         if (e != cudaSuccess) return e;
@@ -207,7 +208,7 @@ template <typename T> struct LenLaunch {
     template <int L, int MODE, int ALT = 0> static cudaError_t launch_k5(spns_handle *h) {
         if constexpr (AxisTmaShape<T, L>::ON && ALT == 0 && MODE != spns::MODE_LES)
             if (2 * h->g.hx + 1 <= L) return launch_k5_tma<L, MODE>(h);
-        using S = ShapeK5A<T, L, ALT>;
+        using S = ShapeK5A<T, L, MODE, ALT>;
         auto kern = spns::k5_fwd_x<T, L, S::E, S::P, MODE>;
         cudaError_t e = spns_set_smem(kern, S::SMEM_ROW);
         if (e != cudaSuccess) return e;
@@ -274,7 +275,7 @@ template <typename T> struct LenLaunch {
         return cudaGetLastError();
     }
     template <int L, int MODE, int ALT> static cudaError_t launch_k4b(spns_handle *h, const spns::BatchMember *tab, int n, cudaStream_t st) {
-        using S = ShapeK2A<T, L, ALT>;
+        using S = ShapeK4A<T, L, MODE, ALT>;
         auto kern = spns::k4_fwd_y_batch<T, L, S::E, S::P, MODE>;
         cudaError_t e = spns_set_smem(kern, S::SMEM_ROW);
         if (e != cudaSuccess) return e;
@@ -282,7 +283,7 @@ template <typename T> struct LenLaunch {
         return cudaGetLastError();
     }
     template <int L, int MODE, int ALT> static cudaError_t launch_k5b(spns_handle *h, const spns::BatchMember *tab, int n, cudaStream_t st) {
-        using S = ShapeK5A<T, L, ALT>;
+        using S = ShapeK5A<T, L, MODE, ALT>;
         auto kern = spns::k5_fwd_x_batch<T, L, S::E, S::P, MODE>;
         cudaError_t e = spns_set_smem(kern, S::SMEM_ROW);
         if (e != cudaSuccess) return e;

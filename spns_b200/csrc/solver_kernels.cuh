@@ -94,8 +94,11 @@ __device__ __forceinline__ int ffreq(int a, int M) { return a <= M / 2 ? a : a -
 #ifndef SPNS_F32_AX_MINB
 #define SPNS_F32_AX_MINB 2
 #endif
-template <typename T, int PASS> struct AxisMinBlocks {
-    static constexpr int N = sizeof(T) == 8 ? ((PASS == 2 || PASS == 4) ? SPNS_K2_MINB : PASS == 1 ? SPNS_K1_MINB : SPNS_K5_MINB)
+#ifndef SPNS_LES_MINB
+#define SPNS_LES_MINB 2
+#endif
+template <typename T, int PASS, int MODE> struct AxisMinBlocks {
+    static constexpr int N = MODE == 3 /* LES */ && PASS >= 4 ? SPNS_LES_MINB : sizeof(T) == 8 ? ((PASS == 2 || PASS == 4) ? SPNS_K2_MINB : PASS == 1 ? SPNS_K1_MINB : SPNS_K5_MINB)
                                             : SPNS_F32_AX_MINB;
 };
 
@@ -109,50 +112,69 @@ template <int MODE> struct Fields {
 
 // ===========================================================================
 // K1: inverse transform along x.  Block = (kz chunk, iy).
-//   VEL: u,v,w   ROT: u,v,w and the vorticity w_x=i(ky w-kz v), w_y=i(kz u-kx w),
-//   w_z=i(kx v-ky u) (ky is the block's, kx the row's)   ADV/LES: u,v,w, du/dx, dv/dx, dw/dx
+//   VEL: u,v,w   ROT: u,v,w and the vorticity   ADV/LES: u,v,w, du/dx, dv/dx, dw/dx
+// ky and kz are constant along a line, so of the vorticity w_x = i(ky w - kz v),
+// w_y = i(kz u - kx w), w_z = i(kx v - ky u) only the parts with kx need transforms of
+// their own: five transforms (v, w, u, kx w, kx v) and five reads of the state per point
+// instead of six and nine.  The one transformed field a later output needs (v for w_x, u
+// for w_y and w_z) waits in shared memory, each thread its own values (K1Smem).
 // ===========================================================================
+template <typename T, int L, int E, int P, int MODE> struct K1Smem {
+    static constexpr size_t BYTES = (size_t)L * P * sizeof(cx<T>) * (MODE == MODE_ROT ? 2 : 1);
+};
 template <typename T, int L, int E, int P, int MODE>
 __device__ __forceinline__ void k1_inv_x_body(Geo g, const cx<T> *__restrict__ u, const cx<T> *__restrict__ v,
                                               const cx<T> *__restrict__ w, cx<T> *__restrict__ out, const cx<T> *__restrict__ tw) {
     extern __shared__ __align__(16) unsigned char smraw[];
+    constexpr int THREADS = P * (L / E);
     const int tid = threadIdx.x, p = tid % P, q = tid / P;
     const int iy = blockIdx.y, kz = blockIdx.x * P + p;
     const bool ok = kz < g.Kz;
-    const T kzf = T(g.sz * kz);
-    const T kyf = T(g.sy * ky_mode(g, iy));
     SmRowMajor<T, P> sm{reinterpret_cast<cx<T> *>(smraw), p};
-    const long long rb = (long long)iy * g.Kx;
-#pragma unroll 1
-    for (int f = 0; f < Fields<MODE>::K1; f++) {
-        cx<T> r[E];
+    const long long rb = (long long)iy * g.Kx * g.Kz + kz, ob = (long long)iy * g.Mx * g.Kz + kz;
+    // loads the field into the input rows, times kx where `deriv` (all loads before the first use)
+    auto load = [&](cx<T>(&r)[E], const cx<T> *src, bool deriv) {
 #pragma unroll
         for (int e = 0; e < E; e++) {
-            const int row = in_row<L, E, true>(q, e);
-            const int m1 = ffreq(row, L);
-            cx<T> val = zero<T>();
-            if (ok && m1 <= g.hx && m1 >= -g.hx) {
-                const long long idx = (rb + (m1 >= 0 ? m1 : m1 + g.Kx)) * g.Kz + kz;
-                const T kx = T(g.sx * m1);
-                if (f == 0) val = u[idx];
-                else if (f == 1) val = v[idx];
-                else if (f == 2) val = w[idx];
-                else if (MODE == MODE_ROT) {
-                    if (f == 3) { cx<T> b = v[idx], c = w[idx]; val = mul_i(mk<T>(kyf * c.x - kzf * b.x, kyf * c.y - kzf * b.y)); }
-                    else if (f == 4) { cx<T> a = u[idx], c = w[idx]; val = mul_i(mk<T>(kzf * a.x - kx * c.x, kzf * a.y - kx * c.y)); }
-                    else { cx<T> a = u[idx], b = v[idx]; val = mul_i(mk<T>(kx * b.x - kyf * a.x, kx * b.y - kyf * a.y)); }
-                } else { // x-derivatives
-                    const cx<T> *src = f == 3 ? u : f == 4 ? v : w;
-                    val = mul_i(kx * src[idx]);
-                }
-            }
-            r[e] = val;
+            const int m1 = ffreq(in_row<L, E, true>(q, e), L);
+            r[e] = (ok && m1 <= g.hx && m1 >= -g.hx) ? src[rb + (long long)(m1 >= 0 ? m1 : m1 + g.Kx) * g.Kz] : zero<T>();
         }
-        fft<T, L, E, true>(r, sm, q, tw);
-        if (ok) {
-            cx<T> *o = out + (long long)f * g.S1 + (long long)iy * g.Mx * g.Kz + kz;
+        if (deriv) {
 #pragma unroll
-            for (int e = 0; e < E; e++) o[(long long)out_row<L, E, true>(q, e) * g.Kz] = r[e];
+            for (int e = 0; e < E; e++) r[e] = T(g.sx * ffreq(in_row<L, E, true>(q, e), L)) * r[e];
+        }
+    };
+    auto put = [&](int f, auto value) {
+        if (!ok) return;
+        cx<T> *o = out + (long long)f * g.S1 + ob;
+#pragma unroll
+        for (int e = 0; e < E; e++) o[(long long)out_row<L, E, true>(q, e) * g.Kz] = value(e);
+    };
+    if constexpr (MODE == MODE_ROT) {
+        const T kzf = T(g.sz * kz), kyf = T(g.sy * ky_mode(g, iy));
+        cx<T> *const slot = reinterpret_cast<cx<T> *>(smraw) + L * P + tid;
+#pragma unroll 1
+        for (int s = 0; s < 5; s++) {
+            cx<T> r[E];
+            load(r, s == 2 ? u : (s == 0 || s == 4) ? v : w, s >= 3);
+            fft<T, L, E, true>(r, sm, q, tw);
+            if (s < 3) put(s == 0 ? 1 : s == 1 ? 2 : 0, [&](int e) { return r[e]; });
+            if (s == 1) put(3, [&](int e) { return mul_i(kyf * r[e] - kzf * slot[e * THREADS]); });
+            if (s == 3) put(4, [&](int e) { return mul_i(kzf * slot[e * THREADS] - r[e]); });
+            if (s == 4) put(5, [&](int e) { return mul_i(r[e] - kyf * slot[e * THREADS]); });
+            if (s == 0 || s == 2) {
+#pragma unroll
+                for (int e = 0; e < E; e++) slot[e * THREADS] = r[e];
+            }
+        }
+    } else {
+#pragma unroll 1
+        for (int f = 0; f < Fields<MODE>::K1; f++) {
+            cx<T> r[E];
+            load(r, f % 3 == 0 ? u : f % 3 == 1 ? v : w, f >= 3);
+            fft<T, L, E, true>(r, sm, q, tw);
+            if (f < 3) put(f, [&](int e) { return r[e]; });
+            else put(f, [&](int e) { return mul_i(r[e]); });
         }
     }
 }
@@ -166,37 +188,33 @@ template <typename T, int L, int E, int P, int MODE>
 __device__ __forceinline__ void k2_inv_y_body(Geo g, const cx<T> *__restrict__ in, cx<T> *__restrict__ out,
                                               const cx<T> *__restrict__ tw) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    const int tid = threadIdx.x, p = tid % P, q = tid / P;
+    const int tid = threadIdx.x, p = tid % P, q0 = tid / P;
     const int x = blockIdx.y, kz = blockIdx.x * P + p;
     const bool ok = kz < g.Kz;
-    const T kzf = T(g.sz * kz);
     SmRowMajor<T, P> sm{reinterpret_cast<cx<T> *>(smraw), p};
-    const long long col = (long long)x * g.Kz + kz;
+    // row offsets in 32 bits (a field has fewer than 2^31 elements at every compiled length):
+    // one register and one multiply-add per address instead of a 64-bit chain
+    const unsigned col = (unsigned)x * g.Kz + kz, rs = (unsigned)g.Mx * g.Kz;
 #pragma unroll 1
     for (int f = 0; f < Fields<MODE>::K2; f++) {
+        const int q = opaque(q0);
         cx<T> r[E];
+        const bool deriv = (MODE == MODE_ADV || MODE == MODE_LES || MODE == MODE_INV) && f >= 6;
+        const cx<T> *F = in + (long long)(deriv ? f - 6 : f) * g.S1;
 #pragma unroll
         for (int e = 0; e < E; e++) {
-            const int row = in_row<L, E, true>(q, e);
-            const int m2 = ffreq(row, L);
-            cx<T> val = zero<T>();
-            if (ok && m2 <= g.hy && m2 >= -g.hy) {
-                const cx<T> *F = in + (long long)(m2 >= 0 ? m2 : m2 + g.Ky) * g.Mx * g.Kz + col;
-                const T ky = T(g.sy * m2);
-                if (MODE == MODE_VEL || MODE == MODE_ROT) {
-                    val = F[(long long)f * g.S1];
-                } else {
-                    if (f < 6) val = F[(long long)f * g.S1];
-                    else val = mul_i(ky * F[(long long)(f - 6) * g.S1]);
-                }
-            }
-            r[e] = val;
+            const int m2 = ffreq(in_row<L, E, true>(q, e), L);
+            r[e] = (ok && m2 <= g.hy && m2 >= -g.hy) ? F[col + (unsigned)(m2 >= 0 ? m2 : m2 + g.Ky) * rs] : zero<T>();
+        }
+        if (deriv) {
+#pragma unroll
+            for (int e = 0; e < E; e++) r[e] = mul_i(T(g.sy * ffreq(in_row<L, E, true>(q, e), L)) * r[e]);
         }
         fft<T, L, E, true>(r, sm, q, tw);
         if (ok) {
-            cx<T> *o = out + (long long)f * g.S2 + col;
+            cx<T> *o = out + (long long)f * g.S2;
 #pragma unroll
-            for (int e = 0; e < E; e++) o[(long long)out_row<L, E, true>(q, e) * g.Mx * g.Kz] = r[e];
+            for (int e = 0; e < E; e++) o[col + (unsigned)out_row<L, E, true>(q, e) * rs] = r[e];
         }
     }
 }
@@ -896,54 +914,46 @@ template <typename T, int L, int E, int P, int MODE>
 __device__ __forceinline__ void k4_fwd_y_body(Geo g, const cx<T> *__restrict__ in, cx<T> *__restrict__ out,
                                               const cx<T> *__restrict__ tw) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    const int tid = threadIdx.x, p = tid % P, q = tid / P;
+    const int tid = threadIdx.x, p = tid % P, q0 = tid / P;
     const int x = blockIdx.y, kz = blockIdx.x * P + p;
     const bool ok = kz < g.Kz;
     SmRowMajor<T, P> sm{reinterpret_cast<cx<T> *>(smraw), p};
-    const long long col = (long long)x * g.Kz + kz;
+    const unsigned col = (unsigned)x * g.Kz + kz, rs = (unsigned)g.Mx * g.Kz;
+    constexpr bool LES = MODE == MODE_LES;
+    // LES.  in (S2): 0 G_x, 1 G_y, 2 G_z, 3 t11, 4 t12, 5 t13, 6 t22, 7 t23
+    //       out (S1): 0 G_x + i ky t12, 1 G_y + i ky t22, 2 G_z + i ky t23, 3 t11, 4 t12, 5 t13
+    // Groups: (t12, G_x), (t22, G_y), (t23, G_z), then t11 and t13 alone.
+    constexpr int NG = LES ? 5 : Fields<MODE>::NOUT;
     auto load_fft = [&](cx<T>(&r)[E], int f) {
-        const cx<T> *src = in + (long long)f * g.S2 + col;
+        const int q = opaque(q0);
+        const cx<T> *src = in + (long long)f * g.S2;
 #pragma unroll
-        for (int e = 0; e < E; e++) r[e] = ok ? src[(long long)in_row<L, E, false>(q, e) * g.Mx * g.Kz] : zero<T>();
+        for (int e = 0; e < E; e++) r[e] = ok ? src[col + (unsigned)in_row<L, E, false>(q, e) * rs] : zero<T>();
         fft<T, L, E, false>(r, sm, q, tw);
     };
-    auto store = [&](const cx<T>(&r)[E], int f, const cx<T> *add, bool use_add) {
+    auto store = [&](int f, auto value) {
         if (!ok) return;
-        cx<T> *o = out + (long long)f * g.S1 + col;
+        const int q = opaque(q0);
+        cx<T> *o = out + (long long)f * g.S1;
 #pragma unroll
         for (int e = 0; e < E; e++) {
             const int m2 = ffreq(out_row<L, E, false>(q, e), L);
-            if (m2 <= g.hy && m2 >= -g.hy) {
-                cx<T> val = r[e];
-                if (use_add) val = val + mul_i(T(g.sy * m2) * add[e]);
-                o[(long long)(m2 >= 0 ? m2 : m2 + g.Ky) * g.Mx * g.Kz] = val;
-            }
+            if (m2 <= g.hy && m2 >= -g.hy) o[col + (unsigned)(m2 >= 0 ? m2 : m2 + g.Ky) * rs] = value(e, m2);
         }
     };
-    if constexpr (MODE != MODE_LES) {
 #pragma unroll 1
-        for (int f = 0; f < Fields<MODE>::NOUT; f++) {
-            cx<T> r[E];
-            load_fft(r, k4_in_field<MODE>(f));
-            store(r, f, r, false);
-        }
-    } else {
-        // in (S2): 0 G_x, 1 G_y, 2 G_z, 3 t11, 4 t12, 5 t13, 6 t22, 7 t23
-        // out (S1): 0 G_x + i ky t12, 1 G_y + i ky t22, 2 G_z + i ky t23, 3 t11, 4 t12, 5 t13
-        const int gi[3] = {0, 1, 2}, ti[3] = {4, 6, 7};
-#pragma unroll 1
-        for (int i = 0; i < 3; i++) {
-            cx<T> r[E], t[E];
-            load_fft(r, gi[i]);
-            load_fft(t, ti[i]);
-            store(r, i, t, true);
-            if (i == 0) store(t, 4, t, false);
-        }
-#pragma unroll 1
-        for (int f = 3; f <= 5; f += 2) {
-            cx<T> r[E];
+    for (int grp = 0; grp < NG; grp++) {
+        cx<T> r[E];
+        if (!LES || grp >= 3) {
+            const int f = !LES ? k4_in_field<MODE>(grp) : 2 * grp - 3;
             load_fft(r, f);
-            store(r, f, r, false);
+            store(LES ? f : grp, [&](int e, int) { return r[e]; });
+        } else {
+            cx<T> t[E];
+            load_fft(t, grp == 0 ? 4 : grp + 5);
+            if (grp == 0) store(4, [&](int e, int) { return t[e]; });
+            load_fft(r, grp);
+            store(grp, [&](int e, int m2) { return r[e] + mul_i(T(g.sy * m2) * t[e]); });
         }
     }
 }
@@ -961,6 +971,7 @@ __device__ __forceinline__ void k5_fwd_x_body(Geo g, const cx<T> *__restrict__ i
     const bool ok = kz < g.Kz;
     SmRowMajor<T, P> sm{reinterpret_cast<cx<T> *>(smraw), p};
     const long long col = (long long)iy * g.Mx * g.Kz + kz;
+    constexpr bool LES = MODE == MODE_LES;
     auto load_fft = [&](cx<T>(&r)[E], int f) {
         const cx<T> *src = in + (long long)f * g.S1 + col;
 #pragma unroll
@@ -969,24 +980,18 @@ __device__ __forceinline__ void k5_fwd_x_body(Geo g, const cx<T> *__restrict__ i
     };
 #pragma unroll 1
     for (int f = 0; f < Fields<MODE>::NOUT; f++) {
-        cx<T> r[E];
+        cx<T> r[E], t[LES ? E : 1];
         load_fft(r, f);
-        if constexpr (MODE == MODE_LES) {
-            cx<T> t[E];
-            load_fft(t, 3 + f); // t11, t21=t12, t31=t13
+        if constexpr (LES) load_fft(t, 3 + f);   // t11, t12, t13
+        if (!ok) continue;
+        cx<T> *o = G + (long long)f * g.S0 + (long long)iy * g.Kx * g.Kz + kz;
 #pragma unroll
-            for (int e = 0; e < E; e++) {
-                const int m1 = ffreq(out_row<L, E, false>(q, e), L);
-                r[e] = r[e] + mul_i(T(g.sx * m1) * t[e]);
-            }
-        }
-        if (ok) {
-            cx<T> *o = G + (long long)f * g.S0 + (long long)iy * g.Kx * g.Kz + kz;
-#pragma unroll
-            for (int e = 0; e < E; e++) {
-                const int m1 = ffreq(out_row<L, E, false>(q, e), L);
-                if (m1 <= g.hx && m1 >= -g.hx) o[(long long)(m1 >= 0 ? m1 : m1 + g.Kx) * g.Kz] = r[e];
-            }
+        for (int e = 0; e < E; e++) {
+            const int m1 = ffreq(out_row<L, E, false>(q, e), L);
+            if (m1 > g.hx || m1 < -g.hx) continue;
+            cx<T> val = r[e];
+            if constexpr (LES) val = val + mul_i(T(g.sx * m1) * t[e]);
+            o[(long long)(m1 >= 0 ? m1 : m1 + g.Kx) * g.Kz] = val;
         }
     }
 }
@@ -1591,13 +1596,13 @@ static __global__ void k_dft_axis(const double2 *__restrict__ in, double2 *__res
 // come from a device table (BatchMember).  The arithmetic is the one-box kernel's.
 // ===========================================================================
 template <typename T, int L, int E, int P, int MODE>
-__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 1>::N) k1_inv_x(Geo g, const cx<T> *__restrict__ u, const cx<T> *__restrict__ v,
+__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 1, MODE>::N) k1_inv_x(Geo g, const cx<T> *__restrict__ u, const cx<T> *__restrict__ v,
                                                                            const cx<T> *__restrict__ w, cx<T> *__restrict__ out,
                                                                            const cx<T> *__restrict__ tw) {
     k1_inv_x_body<T, L, E, P, MODE>(g, u, v, w, out, tw);
 }
 template <typename T, int L, int E, int P, int MODE>
-__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 2>::N) k2_inv_y(Geo g, const cx<T> *__restrict__ in, cx<T> *__restrict__ out,
+__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 2, MODE>::N) k2_inv_y(Geo g, const cx<T> *__restrict__ in, cx<T> *__restrict__ out,
                                                                            const cx<T> *__restrict__ tw) {
     k2_inv_y_body<T, L, E, P, MODE>(g, in, out, tw);
 }
@@ -1608,12 +1613,12 @@ __global__ void __launch_bounds__(P *(L / E), K3MinBlocks<T, MODE, P *(L / E)>::
     k3_z_body<T, L, E, P, MODE, STAGE>(g, buf, c, ds, phys, tw);
 }
 template <typename T, int L, int E, int P, int MODE>
-__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 4>::N) k4_fwd_y(Geo g, const cx<T> *__restrict__ in, cx<T> *__restrict__ out,
+__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 4, MODE>::N) k4_fwd_y(Geo g, const cx<T> *__restrict__ in, cx<T> *__restrict__ out,
                                                                            const cx<T> *__restrict__ tw) {
     k4_fwd_y_body<T, L, E, P, MODE>(g, in, out, tw);
 }
 template <typename T, int L, int E, int P, int MODE>
-__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 5>::N) k5_fwd_x(Geo g, const cx<T> *__restrict__ in, cx<T> *__restrict__ G,
+__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 5, MODE>::N) k5_fwd_x(Geo g, const cx<T> *__restrict__ in, cx<T> *__restrict__ G,
                                                                            const cx<T> *__restrict__ tw) {
     k5_fwd_x_body<T, L, E, P, MODE>(g, in, G, tw);
 }
@@ -1633,14 +1638,14 @@ struct BatchMember {
     StepConsts c;
 };
 template <typename T, int L, int E, int P, int MODE>
-__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 1>::N) k1_inv_x_batch(Geo g, const BatchMember *__restrict__ tab,
+__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 1, MODE>::N) k1_inv_x_batch(Geo g, const BatchMember *__restrict__ tab,
                                                                                  const cx<T> *__restrict__ tw) {
     const BatchMember &m = tab[blockIdx.z];
     const cx<T> *U = static_cast<const cx<T> *>(m.U);
     k1_inv_x_body<T, L, E, P, MODE>(g, U, U + g.S0, U + 2 * g.S0, static_cast<cx<T> *>(m.B1), tw);
 }
 template <typename T, int L, int E, int P, int MODE>
-__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 2>::N) k2_inv_y_batch(Geo g, const BatchMember *__restrict__ tab,
+__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 2, MODE>::N) k2_inv_y_batch(Geo g, const BatchMember *__restrict__ tab,
                                                                                  const cx<T> *__restrict__ tw) {
     const BatchMember &m = tab[blockIdx.z];
     k2_inv_y_body<T, L, E, P, MODE>(g, static_cast<const cx<T> *>(m.B1), static_cast<cx<T> *>(m.B2), tw);
@@ -1652,13 +1657,13 @@ __global__ void __launch_bounds__(P *(L / E), K3MinBlocks<T, MODE, P *(L / E)>::
     k3_z_body<T, L, E, P, MODE, STAGE>(g, static_cast<cx<T> *>(m.B2), m.c, m.ds, nullptr, tw);
 }
 template <typename T, int L, int E, int P, int MODE>
-__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 4>::N) k4_fwd_y_batch(Geo g, const BatchMember *__restrict__ tab,
+__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 4, MODE>::N) k4_fwd_y_batch(Geo g, const BatchMember *__restrict__ tab,
                                                                                  const cx<T> *__restrict__ tw) {
     const BatchMember &m = tab[blockIdx.z];
     k4_fwd_y_body<T, L, E, P, MODE>(g, static_cast<const cx<T> *>(m.B2), static_cast<cx<T> *>(m.B1), tw);
 }
 template <typename T, int L, int E, int P, int MODE>
-__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 5>::N) k5_fwd_x_batch(Geo g, const BatchMember *__restrict__ tab,
+__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 5, MODE>::N) k5_fwd_x_batch(Geo g, const BatchMember *__restrict__ tab,
                                                                                  const cx<T> *__restrict__ tw) {
     const BatchMember &m = tab[blockIdx.z];
     k5_fwd_x_body<T, L, E, P, MODE>(g, static_cast<const cx<T> *>(m.B1), static_cast<cx<T> *>(m.B2), tw);
