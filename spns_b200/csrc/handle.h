@@ -147,6 +147,9 @@ template <typename T, int L, int MODE, int ALT> using ShapeK5A =
     typename std::conditional<ALT != 0, ShapeT<T, L, SPNS_ALT_E, ShapeSel<T>::K5_T>,
                               typename std::conditional<MODE != spns::MODE_LES, ShapeK5<T, L>, ShapeT<T, L, SPNS_LES_E, SPNS_LES_T5>>::type>::type;
 
+#ifndef SPNS_SPLIT_WAVES
+#define SPNS_SPLIT_WAVES 4       // x/y passes with fewer than 4 blocks per SM spread their fields over blocks
+#endif
 // Rotational z pass with pair-by-pair bulk-copy staging, persistent
 // (k3_rot_staged, zpass_staged.cuh): used at lengths from SPNS_ZS_MIN_L up to 768.
 // Per precision: E values per thread, PB pencils per block, SLOTS physical slots

@@ -16,13 +16,19 @@ template <typename T> struct LenLaunch {
     static C *U(spns_handle *h, int f = 0) { return (C *)h->U + (long long)f * h->g.S0; }
     static const C *tw(spns_handle *h, int L) { return (const C *)h->tw[L]; }
 
+    // Grid of an x/y pass: kz chunks x lines, and for small boxes the fields (or groups of
+    // fields) of the pass spread over blocks.
+    static dim3 axis_grid(const spns_handle *h, int P, int lines, int fields) {
+        const int chunks = (h->g.Kz + P - 1) / P;
+        return dim3(chunks, lines, (long long)chunks * lines < (long long)SPNS_SPLIT_WAVES * h->sms ? fields : 1);
+    }
     template <int L, int MODE, int ALT = 0> static cudaError_t launch_k1(spns_handle *h) {
         using S = ShapeK1A<T, L, ALT>;
         auto kern = spns::k1_inv_x<T, L, S::E, S::P, MODE>;
         constexpr size_t smem = spns::K1Smem<T, L, S::E, S::P, MODE>::BYTES;
         cudaError_t e = spns_set_smem(kern, smem);
         if (e != cudaSuccess) return e;
-        dim3 grid((h->g.Kz + S::P - 1) / S::P, h->g.Ky);
+        const dim3 grid = axis_grid(h, S::P, h->g.Ky, spns::Fields<MODE>::K1);
         kern<<<grid, S::THREADS, smem, h->st>>>(h->g, U(h, 0), U(h, 1), U(h, 2), (C *)h->B1, tw(h, L));
         return cudaGetLastError();
     }
@@ -129,7 +135,7 @@ template <typename T> struct LenLaunch {
         auto kern = spns::k2_inv_y<T, L, S::E, S::P, MODE>;
         cudaError_t e = spns_set_smem(kern, S::SMEM_ROW);
         if (e != cudaSuccess) return e;
-        dim3 grid((h->g.Kz + S::P - 1) / S::P, h->g.Mx);
+        const dim3 grid = axis_grid(h, S::P, h->g.Mx, spns::Fields<MODE>::K2);
         kern<<<grid, S::THREADS, S::SMEM_ROW, h->st>>>(h->g, (const C *)h->B1, (C *)h->B2, tw(h, L));
         return cudaGetLastError();
     }
@@ -201,7 +207,7 @@ template <typename T> struct LenLaunch {
         auto kern = spns::k4_fwd_y<T, L, S::E, S::P, MODE>;
         cudaError_t e = spns_set_smem(kern, S::SMEM_ROW);
         if (e != cudaSuccess) return e;
-        dim3 grid((h->g.Kz + S::P - 1) / S::P, h->g.Mx);
+        const dim3 grid = axis_grid(h, S::P, h->g.Mx, MODE == spns::MODE_LES ? 5 : spns::Fields<MODE>::NOUT);
         kern<<<grid, S::THREADS, S::SMEM_ROW, h->st>>>(h->g, (const C *)h->B2, (C *)h->B1, tw(h, L));
         return cudaGetLastError();
     }
@@ -212,7 +218,7 @@ template <typename T> struct LenLaunch {
         auto kern = spns::k5_fwd_x<T, L, S::E, S::P, MODE>;
         cudaError_t e = spns_set_smem(kern, S::SMEM_ROW);
         if (e != cudaSuccess) return e;
-        dim3 grid((h->g.Kz + S::P - 1) / S::P, h->g.Ky);
+        const dim3 grid = axis_grid(h, S::P, h->g.Ky, spns::Fields<MODE>::NOUT);
         kern<<<grid, S::THREADS, S::SMEM_ROW, h->st>>>(h->g, (const C *)h->B1, (C *)h->B2, tw(h, L));
         return cudaGetLastError();
     }

@@ -124,7 +124,8 @@ template <typename T, int L, int E, int P, int MODE> struct K1Smem {
 };
 template <typename T, int L, int E, int P, int MODE>
 __device__ __forceinline__ void k1_inv_x_body(Geo g, const cx<T> *__restrict__ u, const cx<T> *__restrict__ v,
-                                              const cx<T> *__restrict__ w, cx<T> *__restrict__ out, const cx<T> *__restrict__ tw) {
+                                              const cx<T> *__restrict__ w, cx<T> *__restrict__ out, const cx<T> *__restrict__ tw,
+                                              int f0, int fs) {
     extern __shared__ __align__(16) unsigned char smraw[];
     constexpr int THREADS = P * (L / E);
     const int tid = threadIdx.x, p = tid % P, q = tid / P;
@@ -153,6 +154,23 @@ __device__ __forceinline__ void k1_inv_x_body(Geo g, const cx<T> *__restrict__ u
     if constexpr (MODE == MODE_ROT) {
         const T kzf = T(g.sz * kz), kyf = T(g.sy * ky_mode(g, iy));
         cx<T> *const slot = reinterpret_cast<cx<T> *>(smraw) + L * P + tid;
+        if (fs > 1) {   // outputs split over blocks: each forms its own input
+#pragma unroll 1
+            for (int f = f0; f < 6; f += fs) {
+                cx<T> r[E];
+                load(r, f == 0 || f == 4 ? u : f == 1 || f == 5 ? v : w, f == 5);
+                if (f >= 3) {
+                    cx<T> b[E];
+                    load(b, f == 5 ? u : f == 4 ? w : v, f == 4);
+                    const T ka = f == 3 ? kyf : f == 4 ? kzf : T(1), kb = f == 3 ? kzf : f == 4 ? T(1) : kyf;
+#pragma unroll
+                    for (int e = 0; e < E; e++) r[e] = mul_i(ka * r[e] - kb * b[e]);
+                }
+                fft<T, L, E, true>(r, sm, q, tw);
+                put(f, [&](int e) { return r[e]; });
+            }
+            return;
+        }
 #pragma unroll 1
         for (int s = 0; s < 5; s++) {
             cx<T> r[E];
@@ -169,7 +187,7 @@ __device__ __forceinline__ void k1_inv_x_body(Geo g, const cx<T> *__restrict__ u
         }
     } else {
 #pragma unroll 1
-        for (int f = 0; f < Fields<MODE>::K1; f++) {
+        for (int f = f0; f < Fields<MODE>::K1; f += fs) {
             cx<T> r[E];
             load(r, f % 3 == 0 ? u : f % 3 == 1 ? v : w, f >= 3);
             fft<T, L, E, true>(r, sm, q, tw);
@@ -186,7 +204,7 @@ __device__ __forceinline__ void k1_inv_x_body(Geo g, const cx<T> *__restrict__ u
 // ===========================================================================
 template <typename T, int L, int E, int P, int MODE>
 __device__ __forceinline__ void k2_inv_y_body(Geo g, const cx<T> *__restrict__ in, cx<T> *__restrict__ out,
-                                              const cx<T> *__restrict__ tw) {
+                                              const cx<T> *__restrict__ tw, int f0, int fs) {
     extern __shared__ __align__(16) unsigned char smraw[];
     const int tid = threadIdx.x, p = tid % P, q0 = tid / P;
     const int x = blockIdx.y, kz = blockIdx.x * P + p;
@@ -196,7 +214,7 @@ __device__ __forceinline__ void k2_inv_y_body(Geo g, const cx<T> *__restrict__ i
     // one register and one multiply-add per address instead of a 64-bit chain
     const unsigned col = (unsigned)x * g.Kz + kz, rs = (unsigned)g.Mx * g.Kz;
 #pragma unroll 1
-    for (int f = 0; f < Fields<MODE>::K2; f++) {
+    for (int f = f0; f < Fields<MODE>::K2; f += fs) {
         const int q = opaque(q0);
         cx<T> r[E];
         const bool deriv = (MODE == MODE_ADV || MODE == MODE_LES || MODE == MODE_INV) && f >= 6;
@@ -912,7 +930,7 @@ template <int MODE> __host__ __device__ constexpr int k4_in_field(int f) { retur
 // ===========================================================================
 template <typename T, int L, int E, int P, int MODE>
 __device__ __forceinline__ void k4_fwd_y_body(Geo g, const cx<T> *__restrict__ in, cx<T> *__restrict__ out,
-                                              const cx<T> *__restrict__ tw) {
+                                              const cx<T> *__restrict__ tw, int f0, int fs) {
     extern __shared__ __align__(16) unsigned char smraw[];
     const int tid = threadIdx.x, p = tid % P, q0 = tid / P;
     const int x = blockIdx.y, kz = blockIdx.x * P + p;
@@ -942,7 +960,7 @@ __device__ __forceinline__ void k4_fwd_y_body(Geo g, const cx<T> *__restrict__ i
         }
     };
 #pragma unroll 1
-    for (int grp = 0; grp < NG; grp++) {
+    for (int grp = f0; grp < NG; grp += fs) {
         cx<T> r[E];
         if (!LES || grp >= 3) {
             const int f = !LES ? k4_in_field<MODE>(grp) : 2 * grp - 3;
@@ -964,7 +982,7 @@ __device__ __forceinline__ void k4_fwd_y_body(Geo g, const cx<T> *__restrict__ i
 // ===========================================================================
 template <typename T, int L, int E, int P, int MODE>
 __device__ __forceinline__ void k5_fwd_x_body(Geo g, const cx<T> *__restrict__ in, cx<T> *__restrict__ G,
-                                              const cx<T> *__restrict__ tw) {
+                                              const cx<T> *__restrict__ tw, int f0, int fs) {
     extern __shared__ __align__(16) unsigned char smraw[];
     const int tid = threadIdx.x, p = tid % P, q = tid / P;
     const int iy = blockIdx.y, kz = blockIdx.x * P + p;
@@ -979,7 +997,7 @@ __device__ __forceinline__ void k5_fwd_x_body(Geo g, const cx<T> *__restrict__ i
         fft<T, L, E, false>(r, sm, q, tw);
     };
 #pragma unroll 1
-    for (int f = 0; f < Fields<MODE>::NOUT; f++) {
+    for (int f = f0; f < Fields<MODE>::NOUT; f += fs) {
         cx<T> r[E], t[LES ? E : 1];
         load_fft(r, f);
         if constexpr (LES) load_fft(t, 3 + f);   // t11, t12, t13
@@ -1599,12 +1617,12 @@ template <typename T, int L, int E, int P, int MODE>
 __global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 1, MODE>::N) k1_inv_x(Geo g, const cx<T> *__restrict__ u, const cx<T> *__restrict__ v,
                                                                            const cx<T> *__restrict__ w, cx<T> *__restrict__ out,
                                                                            const cx<T> *__restrict__ tw) {
-    k1_inv_x_body<T, L, E, P, MODE>(g, u, v, w, out, tw);
+    k1_inv_x_body<T, L, E, P, MODE>(g, u, v, w, out, tw, blockIdx.z, gridDim.z);
 }
 template <typename T, int L, int E, int P, int MODE>
 __global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 2, MODE>::N) k2_inv_y(Geo g, const cx<T> *__restrict__ in, cx<T> *__restrict__ out,
                                                                            const cx<T> *__restrict__ tw) {
-    k2_inv_y_body<T, L, E, P, MODE>(g, in, out, tw);
+    k2_inv_y_body<T, L, E, P, MODE>(g, in, out, tw, blockIdx.z, gridDim.z);
 }
 template <typename T, int L, int E, int P, int MODE, bool STAGE = false>
 __global__ void __launch_bounds__(P *(L / E), K3MinBlocks<T, MODE, P *(L / E)>::N) k3_z(Geo g, cx<T> *__restrict__ buf, StepConsts c,
@@ -1615,12 +1633,12 @@ __global__ void __launch_bounds__(P *(L / E), K3MinBlocks<T, MODE, P *(L / E)>::
 template <typename T, int L, int E, int P, int MODE>
 __global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 4, MODE>::N) k4_fwd_y(Geo g, const cx<T> *__restrict__ in, cx<T> *__restrict__ out,
                                                                            const cx<T> *__restrict__ tw) {
-    k4_fwd_y_body<T, L, E, P, MODE>(g, in, out, tw);
+    k4_fwd_y_body<T, L, E, P, MODE>(g, in, out, tw, blockIdx.z, gridDim.z);
 }
 template <typename T, int L, int E, int P, int MODE>
 __global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 5, MODE>::N) k5_fwd_x(Geo g, const cx<T> *__restrict__ in, cx<T> *__restrict__ G,
                                                                            const cx<T> *__restrict__ tw) {
-    k5_fwd_x_body<T, L, E, P, MODE>(g, in, G, tw);
+    k5_fwd_x_body<T, L, E, P, MODE>(g, in, G, tw, blockIdx.z, gridDim.z);
 }
 template <typename T, bool SELF>
 __global__ void __launch_bounds__(256) k6_sweep(Geo g, const cx<T> *__restrict__ G, const cx<T> *U, const cx<T> *Ulo, cx<T> *R, cx<T> *Uout,
@@ -1642,13 +1660,13 @@ __global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 1, MODE>::N) k1_i
                                                                                  const cx<T> *__restrict__ tw) {
     const BatchMember &m = tab[blockIdx.z];
     const cx<T> *U = static_cast<const cx<T> *>(m.U);
-    k1_inv_x_body<T, L, E, P, MODE>(g, U, U + g.S0, U + 2 * g.S0, static_cast<cx<T> *>(m.B1), tw);
+    k1_inv_x_body<T, L, E, P, MODE>(g, U, U + g.S0, U + 2 * g.S0, static_cast<cx<T> *>(m.B1), tw, 0, 1);
 }
 template <typename T, int L, int E, int P, int MODE>
 __global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 2, MODE>::N) k2_inv_y_batch(Geo g, const BatchMember *__restrict__ tab,
                                                                                  const cx<T> *__restrict__ tw) {
     const BatchMember &m = tab[blockIdx.z];
-    k2_inv_y_body<T, L, E, P, MODE>(g, static_cast<const cx<T> *>(m.B1), static_cast<cx<T> *>(m.B2), tw);
+    k2_inv_y_body<T, L, E, P, MODE>(g, static_cast<const cx<T> *>(m.B1), static_cast<cx<T> *>(m.B2), tw, 0, 1);
 }
 template <typename T, int L, int E, int P, int MODE, bool STAGE = false>
 __global__ void __launch_bounds__(P *(L / E), K3MinBlocks<T, MODE, P *(L / E)>::N) k3_z_batch(Geo g, const BatchMember *__restrict__ tab,
@@ -1660,13 +1678,13 @@ template <typename T, int L, int E, int P, int MODE>
 __global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 4, MODE>::N) k4_fwd_y_batch(Geo g, const BatchMember *__restrict__ tab,
                                                                                  const cx<T> *__restrict__ tw) {
     const BatchMember &m = tab[blockIdx.z];
-    k4_fwd_y_body<T, L, E, P, MODE>(g, static_cast<const cx<T> *>(m.B2), static_cast<cx<T> *>(m.B1), tw);
+    k4_fwd_y_body<T, L, E, P, MODE>(g, static_cast<const cx<T> *>(m.B2), static_cast<cx<T> *>(m.B1), tw, 0, 1);
 }
 template <typename T, int L, int E, int P, int MODE>
 __global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 5, MODE>::N) k5_fwd_x_batch(Geo g, const BatchMember *__restrict__ tab,
                                                                                  const cx<T> *__restrict__ tw) {
     const BatchMember &m = tab[blockIdx.z];
-    k5_fwd_x_body<T, L, E, P, MODE>(g, static_cast<const cx<T> *>(m.B1), static_cast<cx<T> *>(m.B2), tw);
+    k5_fwd_x_body<T, L, E, P, MODE>(g, static_cast<const cx<T> *>(m.B1), static_cast<cx<T> *>(m.B2), tw, 0, 1);
 }
 // Adams-Bashforth members only (the kappa scheme swaps state buffers every step).
 template <typename T>
