@@ -273,7 +273,7 @@ template <typename T> struct Passes {
                                  int unpack) {
         const long long n = (long long)nf * n1 * n2 * h->g.Kz;
         const int blocks = (int)std::min<long long>((n + 255) / 256, 16LL * h->sms);
-        spns::k_slab_pack<T><<<blocks, 256, 0, h->st>>>((C *)full, (C *)stage, nf, n1, n2, h->g.Kz, r, axis, unpack);
+        spns::k_slab_pack<T><<<blocks, 256, 0, h->st>>>((C *)full, (C *)stage, nf, n1, n2, h->g.Kz, h->g.Kp, r, axis, unpack);
         return cudaGetLastError();
     }
     // Offsets of the staging blocks: block s holds nf * (axis 1: count_s * n2, axis 2: n1 * count_s) * Kz.

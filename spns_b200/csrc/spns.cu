@@ -276,8 +276,9 @@ static int box_geometry(const spns_hit_args &a, Geo &g, int &last_rad, int &last
     g.Mx = actual_n(a.Mx, a.Lx_factor); g.My = actual_n(a.My, a.Ly_factor); g.Mz = actual_n(a.Mz, a.Lz_factor);
     g.sx = a.Lx_factor; g.sy = a.Ly_factor; g.sz = a.Lz_factor;
     g.S0 = (long long)g.Ky * g.Kx * g.Kz;
-    g.S1 = (long long)g.Ky * g.Mx * g.Kz;
-    g.S2 = (long long)g.My * g.Mx * g.Kz;
+    g.Kp = row_pitch(g.Kz, a.precision == SPNS_FP64 ? sizeof(double2) : sizeof(float2));
+    g.S1 = (long long)g.Ky * g.Mx * g.Kp;
+    g.S2 = (long long)g.My * g.Mx * g.Kp;
     g.y0 = 0;
     g.Kyg = g.Ky;
     if (!spns_length_supported(g.Mx) || !spns_length_supported(g.My) || !spns_length_supported(g.Mz))
@@ -1080,13 +1081,13 @@ extern "C" int spns_slab_create(const spns_hit_args *args, int nranks, int rank,
     g.y0 = yr.start[rank];
     g.Kyg = gf.Ky;
     g.S0 = (long long)g.Ky * g.Kx * g.Kz;
-    g.S1 = (long long)g.Ky * g.Mx * g.Kz;
+    g.S1 = (long long)g.Ky * g.Mx * g.Kp;
     g.S2 = 0;
     Geo gx = gf;
     gx.Mx = xr.count[rank];
     gx.S0 = 0;
-    gx.S1 = (long long)gf.Ky * gx.Mx * gf.Kz;
-    gx.S2 = (long long)gf.My * gx.Mx * gf.Kz;
+    gx.S1 = (long long)gf.Ky * gx.Mx * gf.Kp;
+    gx.S2 = (long long)gf.My * gx.Mx * gf.Kp;
     h->g = g;
     h->gx = gx;
     step_consts(h, gf);
@@ -1105,7 +1106,7 @@ extern "C" int spns_slab_create(const spns_hit_args *args, int nranks, int rank,
     const size_t state = cs * 3 * (size_t)g.S0;
     h->nB1 = 6;
     h->nB2 = 9;
-    h->xelems = 6 * (size_t)std::max(g.S1, gx.S1);
+    h->xelems = 6 * (size_t)std::max((long long)g.Ky * g.Mx, (long long)gx.Ky * gx.Mx) * g.Kz;
     auto amalloc = [&](void **p, size_t n) { return n == 0 || cudaMallocAsync(p, n, h->st) == cudaSuccess; };
     const bool okm = amalloc((void **)&h->ds, sizeof(DevScalars)) && amalloc(&h->U, state) && amalloc(&h->Ulo, hilo ? state : 0) &&
                      amalloc(&h->R, state) && amalloc(&h->Up, a.isSelfAdaptive ? state : 0) &&

@@ -188,7 +188,7 @@ __device__ __forceinline__ void k3_field_body(Geo g, cx<T> *__restrict__ buf, co
             const int item = team + r * NT, pl = item / NPAIR;
             const ZPair pr = zfield_pair<MODE>(item - pl * NPAIR);
             const bool ok = pl < np;
-            const cx<T> *base = buf + (p0 + (ok ? pl : 0)) * Kz;
+            const cx<T> *base = buf + (p0 + (ok ? pl : 0)) * g.Kp;
             SmPencil<T, L, E> sm{smc + item * PITCH};
             k3_load_pair<T, L, E>(A, base + pr.a * g.S2, pr.da, pr.b < 0 ? nullptr : base + pr.b * g.S2, pr.db, Kz, sz, q, ok);
             fft<T, L, E, true, SmPencil<T, L, E>, WARP>(A, sm, q, tw);
@@ -217,7 +217,7 @@ __device__ __forceinline__ void k3_field_body(Geo g, cx<T> *__restrict__ buf, co
             const ZJob jb = zfield_job<MODE>(idle < 0 ? j : 0);
             const bool ok = idle < 0 && pl < np;
             SmPencil<T, L, E> sm{smc + (pl * NPAIR + j) * PITCH};
-            cx<T> *base = buf + (p0 + (ok ? pl : 0)) * Kz;
+            cx<T> *base = buf + (p0 + (ok ? pl : 0)) * g.Kp;
             cx<T> *oa = base + jb.a * g.S2, *ob = jb.b < 0 ? nullptr : base + jb.b * g.S2;
 #pragma unroll
             for (int e = 0; e < E; e++) A[e] = sm.at(in_row<L, E, false>(q, e));

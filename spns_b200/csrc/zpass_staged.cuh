@@ -80,13 +80,13 @@ template <typename T, int L, int E, int PB, int SLOTS_SM> struct ZStagedLayout {
     static constexpr int Q = L / E;
     static constexpr int PITCH = pencil_pitch<T, L, E>();
     static constexpr long long SLOT_ELEMS = ((long long)SLOTS_SM * PB * L * (long long)sizeof(T) + (long long)sizeof(cx<T>) - 1) / (long long)sizeof(cx<T>);
-    // staging stride of one field: PB*Kz rounded up to 16 bytes
-    __host__ __device__ static int stage_stride(int Kz) {
+    // staging stride of one field: PB rows of pitch Kp, the last without its padding (Kp is whole 16-byte units)
+    __host__ __device__ static int stage_stride(int Kz, int Kp) {
         const int per16 = 16 / (int)sizeof(cx<T>);
-        return (PB * Kz + per16 - 1) / per16 * per16;
+        return (PB - 1) * Kp + (Kz + per16 - 1) / per16 * per16;
     }
-    __host__ __device__ static long long elems(int Kz) { return (long long)PB * PITCH + 2LL * stage_stride(Kz) + SLOT_ELEMS; }
-    __host__ __device__ static size_t smem_bytes(int Kz) { return (size_t)elems(Kz) * sizeof(cx<T>) + 16; }
+    __host__ __device__ static long long elems(int Kz, int Kp) { return (long long)PB * PITCH + 2LL * stage_stride(Kz, Kp) + SLOT_ELEMS; }
+    __host__ __device__ static size_t smem_bytes(int Kz, int Kp) { return (size_t)elems(Kz, Kp) * sizeof(cx<T>) + 16; }
 };
 
 // Physical slot S (0 u, 1 v, 2 w_x, 3 w_y) of register slot e (grid row `row`):
@@ -108,13 +108,13 @@ __global__ void __launch_bounds__(PB *(L / E), MINB) k3_rot_staged(Geo g, cx<T> 
     extern __shared__ __align__(128) unsigned char smraw_zs[];
     const int tid = threadIdx.x, sub = tid / Q, q0 = tid % Q;
     const int Kz = g.Kz;
-    const int KS = LY::stage_stride(Kz);
+    const int Kp = g.Kp, KS = LY::stage_stride(Kz, Kp);
     cx<T> *const smc = reinterpret_cast<cx<T> *>(smraw_zs);
     SmPencil<T, L, E> sm{smc + sub * LY::PITCH};
     cx<T> *const stA = smc + PB * LY::PITCH;                  // staging: field a of the pair
     cx<T> *const stB = stA + KS;                              // field b
     T *const slot_sm = reinterpret_cast<T *>(stB + KS) + sub * L;   // slot j of this pencil at slot_sm[j*PB*L + row]
-    unsigned long long *const bar = reinterpret_cast<unsigned long long *>(smc + LY::elems(Kz));
+    unsigned long long *const bar = reinterpret_cast<unsigned long long *>(smc + LY::elems(Kz, Kp));
     if (tid == 0) {
         mbar_init(bar, 1);
         fence_mbar_init();
@@ -132,17 +132,17 @@ __global__ void __launch_bounds__(PB *(L / E), MINB) k3_rot_staged(Geo g, cx<T> 
     auto issue = [&](long long grp, int fa, int fb) {
         const long long p0 = grp * PB;
         const int np = (int)(npen - p0 < PB ? npen - p0 : PB);
-        const cx<T> *A = buf + (long long)fa * g.S2 + p0 * Kz, *B = buf + (long long)fb * g.S2 + p0 * Kz;
+        const cx<T> *A = buf + (long long)fa * g.S2 + p0 * Kp, *B = buf + (long long)fb * g.S2 + p0 * Kp;
         if constexpr (BULK) {
             if (tid == 0) {
-                const unsigned bytes = (unsigned)(np * Kz * sizeof(cx<T>));
+                const unsigned bytes = (unsigned)((KS - (PB - np) * Kp) * sizeof(cx<T>));
                 fence_proxy_async_smem();
                 mbar_arrive_expect_tx(bar, 2 * bytes);
                 bulk_copy_g2s(stA, A, bytes, bar);
                 bulk_copy_g2s(stB, B, bytes, bar);
             }
         } else {
-            for (int k = tid; k < np * Kz; k += THREADS) {
+            for (int k = tid; k < KS - (PB - np) * Kp; k += THREADS) {
                 cp_async_elem<T>(stA + k, A + k);
                 cp_async_elem<T>(stB + k, B + k);
             }
@@ -167,9 +167,9 @@ __global__ void __launch_bounds__(PB *(L / E), MINB) k3_rot_staged(Geo g, cx<T> 
         const int q = opaque(q0);
         const long long pen = grp * PB + sub;
         const bool ok = pen < npen;
-        cx<T> *const B0 = buf + (ok ? pen : 0) * Kz;
+        cx<T> *const B0 = buf + (ok ? pen : 0) * Kp;
 #define FZ(i) (B0 + (long long)(i) * g.S2)
-        const cx<T> *sa = stA + sub * Kz, *sb = stB + sub * Kz;
+        const cx<T> *sa = stA + sub * Kp, *sb = stB + sub * Kp;
         cx<T> A[E];
         constexpr int NREG = 4 - SLOTS_SM;
         T r_sl[NREG > 0 ? NREG : 1][E];
