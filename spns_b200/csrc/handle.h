@@ -36,7 +36,9 @@ template <typename T, int L, int E_, int THR> struct ShapeT {
     static constexpr int E = E_;             // complex values per thread
     static constexpr int Q = L / E;          // threads per pencil
     static constexpr int P0 = THR / Q;
-    static constexpr int P = P0 >= 32 ? 32 : P0 >= 16 ? 16 : P0 >= 8 ? 8 : 4; // pencils per block
+    static constexpr int P1 = P0 >= 32 ? 32 : P0 >= 16 ? 16 : P0 >= 8 ? 8 : 4;
+    static constexpr int PM = 128 / (int)sizeof(spns::cx<T>);   // one 128-byte line of a row
+    static constexpr int P = P1 > PM ? PM : P1;               // pencils per block
     static constexpr int THREADS = P * Q;
     static constexpr size_t SMEM_ROW = (size_t)L * P * sizeof(spns::cx<T>);
     static constexpr size_t SMEM_PEN = (size_t)spns::SmPencil<T, L, E_>::PITCH * P * sizeof(spns::cx<T>);
@@ -133,10 +135,10 @@ template <int L, int MODE> constexpr bool shape_alt_ok() {
 #define SPNS_LES_E 12
 #endif
 #ifndef SPNS_LES_T4
-#define SPNS_LES_T4 256
+#define SPNS_LES_T4 128
 #endif
 #ifndef SPNS_LES_T5
-#define SPNS_LES_T5 256
+#define SPNS_LES_T5 128
 #endif
 template <typename T, int L, int ALT> using ShapeK1A = typename std::conditional<ALT != 0, ShapeT<T, L, SPNS_ALT_E, ShapeSel<T>::K1_T>, ShapeK1<T, L>>::type;
 template <typename T, int L, int ALT> using ShapeK2A = typename std::conditional<ALT != 0, ShapeT<T, L, SPNS_ALT_E, ShapeSel<T>::K2_T>, ShapeK2<T, L>>::type;
@@ -219,7 +221,7 @@ template <typename T, int L, int MODE, int ALT = 0> struct Shape3 {
 #define SPNS_ZF_R24 168
 #endif
 #ifndef SPNS_ZF_R12
-#define SPNS_ZF_R12 112
+#define SPNS_ZF_R12 84
 #endif
 #ifndef SPNS_ZF_R6
 #define SPNS_ZF_R6 80

@@ -107,7 +107,7 @@ __device__ __forceinline__ int ffreq(int a, int M) { return a <= M / 2 ? a : a -
 #define SPNS_F32_AX_MINB 2
 #endif
 #ifndef SPNS_LES_MINB
-#define SPNS_LES_MINB 2
+#define SPNS_LES_MINB 3
 #endif
 template <typename T, int PASS, int MODE> struct AxisMinBlocks {
     static constexpr int N = MODE == 3 /* LES */ && PASS >= 4 ? SPNS_LES_MINB : sizeof(T) == 8 ? ((PASS == 2 || PASS == 4) ? SPNS_K2_MINB : PASS == 1 ? SPNS_K1_MINB : SPNS_K5_MINB)
