@@ -37,12 +37,45 @@
 
 namespace spns {
 
+// Two single-precision values operated on by the packed instructions of sm_100a
+// (add/sub/mul/fma.rn.f32x2): lane 0 belongs to one transform, lane 1 to another, so a
+// thread runs two single-precision transforms with the instructions of one.  Each lane is
+// rounded as the scalar instruction rounds it.  One packed instruction takes the issue
+// slot of one scalar one and does the work of two (measured: 130 lanes per clock and SM
+// packed, 115-123 scalar, at half the issue slots).
+struct f2 {
+    unsigned long long v;
+    f2() = default;
+    __device__ __forceinline__ f2(float a, float b) { asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b)); }
+    __device__ __forceinline__ explicit f2(float a) : f2(a, a) {}
+    __device__ __forceinline__ explicit f2(double a) : f2((float)a) {}
+    __device__ __forceinline__ explicit f2(int a) : f2((float)a) {}
+    __device__ __forceinline__ float lo() const { float a; asm("mov.b64 {%0, _}, %1;" : "=f"(a) : "l"(v)); return a; }
+    __device__ __forceinline__ float hi() const { float b; asm("mov.b64 {_, %0}, %1;" : "=f"(b) : "l"(v)); return b; }
+};
+__device__ __forceinline__ f2 operator+(f2 a, f2 b) { f2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ f2 operator-(f2 a, f2 b) { f2 r; asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ f2 operator*(f2 a, f2 b) { f2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ f2 operator-(f2 a) { f2 r; r.v = a.v ^ 0x8000000080000000ull; return r; }
+// a * b + c; the scalar forms leave the contraction to the compiler
+__device__ __forceinline__ f2 mad(f2 a, f2 b, f2 c) { f2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v)); return r; }
+__device__ __forceinline__ float mad(float a, float b, float c) { return a * b + c; }
+__device__ __forceinline__ double mad(double a, double b, double c) { return a * b + c; }
+
+// Precision and storage of an arithmetic type: the element type of the arrays in memory,
+// and how many of them (columns or pencils) a thread transforms at once.
+template <typename T> struct Arith { using S = T; static constexpr int W = 1; static constexpr bool SINGLE = sizeof(T) == 4; };
+template <> struct Arith<f2> { using S = float; static constexpr int W = 2; static constexpr bool SINGLE = true; };
+
 template <typename T> struct alignas(2 * sizeof(T)) cx { T x, y; };
 
 template <typename T> __device__ __forceinline__ cx<T> mk(T a, T b) { cx<T> r; r.x = a; r.y = b; return r; }
 template <typename T> __device__ __forceinline__ cx<T> operator+(cx<T> a, cx<T> b) { return mk<T>(a.x + b.x, a.y + b.y); }
 template <typename T> __device__ __forceinline__ cx<T> operator-(cx<T> a, cx<T> b) { return mk<T>(a.x - b.x, a.y - b.y); }
 template <typename T> __device__ __forceinline__ cx<T> operator*(T s, cx<T> a) { return mk<T>(s * a.x, s * a.y); }
+// products of packed values: the same two roundings per part as the contracted scalar forms
+__device__ __forceinline__ cx<f2> cmul(cx<f2> a, cx<f2> b) { cx<f2> r; r.x = mad(a.x, b.x, a.y * -b.y); r.y = mad(a.x, b.y, a.y * b.x); return r; }
+__device__ __forceinline__ cx<f2> cmulc(cx<f2> a, cx<f2> b) { cx<f2> r; r.x = mad(a.x, b.x, a.y * b.y); r.y = mad(a.y, b.x, a.x * -b.y); return r; }
 template <typename T> __device__ __forceinline__ cx<T> cmul(cx<T> a, cx<T> b) { return mk<T>(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
 template <typename T> __device__ __forceinline__ cx<T> cmulc(cx<T> a, cx<T> b) { return mk<T>(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y); }
 template <typename T> __device__ __forceinline__ cx<T> conj(cx<T> a) { return mk<T>(a.x, -a.y); }
@@ -95,28 +128,33 @@ template <typename T, bool INV> __device__ __forceinline__ void dft2(cx<T> *x) {
 template <typename T, bool INV> __device__ __forceinline__ void dft3(cx<T> *x) {
     const T c3 = T(-0.5);
     const T s3 = INV ? T(0.86602540378443864676372317075294) : T(-0.86602540378443864676372317075294);
+    const T n3 = INV ? T(-0.86602540378443864676372317075294) : T(0.86602540378443864676372317075294);
     cx<T> s = x[1] + x[2], d = x[1] - x[2];
     cx<T> y0 = x[0] + s;
-    cx<T> m = mk<T>(x[0].x + c3 * s.x, x[0].y + c3 * s.y);
-    cx<T> e = mk<T>(-s3 * d.y, s3 * d.x);
-    x[0] = y0; x[1] = m + e; x[2] = m - e;
+    cx<T> m = mk<T>(mad(c3, s.x, x[0].x), mad(c3, s.y, x[0].y));
+    x[0] = y0;
+    x[1] = mk<T>(mad(n3, d.y, m.x), mad(s3, d.x, m.y));
+    x[2] = mk<T>(mad(s3, d.y, m.x), mad(n3, d.x, m.y));
 }
 template <typename T, bool INV> __device__ __forceinline__ void dft4(cx<T> *x) {
     cx<T> t0 = x[0] + x[2], t1 = x[0] - x[2], t2 = x[1] + x[3], t3 = x[1] - x[3];
-    cx<T> u = INV ? mk<T>(-t3.y, t3.x) : mk<T>(t3.y, -t3.x); // (+/-i)*t3
-    x[0] = t0 + t2; x[2] = t0 - t2; x[1] = t1 + u; x[3] = t1 - u;
+    // x1, x3 = t1 +- (+/-i) t3
+    const cx<T> a = mk<T>(t1.x - t3.y, t1.y + t3.x), b = mk<T>(t1.x + t3.y, t1.y - t3.x);
+    x[0] = t0 + t2; x[2] = t0 - t2; x[1] = INV ? a : b; x[3] = INV ? b : a;
 }
 template <typename T, bool INV> __device__ __forceinline__ void dft8(cx<T> *x) {
     const T h = T(0.70710678118654752440084436210485);
     cx<T> e[4] = {x[0], x[2], x[4], x[6]}, o[4] = {x[1], x[3], x[5], x[7]};
     dft4<T, INV>(e); dft4<T, INV>(o);
     // w8^k for k=1..3: forward exp(-i*pi*k/4)
+    const T n = T(-0.70710678118654752440084436210485);
     cx<T> o1 = INV ? mk<T>(h * (o[1].x - o[1].y), h * (o[1].x + o[1].y)) : mk<T>(h * (o[1].x + o[1].y), h * (o[1].y - o[1].x));
-    cx<T> o2 = INV ? mk<T>(-o[2].y, o[2].x) : mk<T>(o[2].y, -o[2].x);
-    cx<T> o3 = INV ? mk<T>(-h * (o[3].x + o[3].y), h * (o[3].x - o[3].y)) : mk<T>(h * (o[3].y - o[3].x), -h * (o[3].x + o[3].y));
+    cx<T> o3 = INV ? mk<T>(n * (o[3].x + o[3].y), h * (o[3].x - o[3].y)) : mk<T>(h * (o[3].y - o[3].x), n * (o[3].x + o[3].y));
+    // x2, x6 = e2 +- (+/-i) o2
+    const cx<T> a = mk<T>(e[2].x - o[2].y, e[2].y + o[2].x), b = mk<T>(e[2].x + o[2].y, e[2].y - o[2].x);
     x[0] = e[0] + o[0]; x[4] = e[0] - o[0];
     x[1] = e[1] + o1;   x[5] = e[1] - o1;
-    x[2] = e[2] + o2;   x[6] = e[2] - o2;
+    x[2] = INV ? a : b; x[6] = INV ? b : a;
     x[3] = e[3] + o3;   x[7] = e[3] - o3;
 }
 // Good-Thomas split of R = A*B (gcd 1): input n = (B a + A b) mod R, output
@@ -252,7 +290,7 @@ __device__ __forceinline__ void fft_run(cx<T> (&v)[E], SM sm, int q, const cx<T>
             const int k = j % Ns;                  // w^r = w_n^{r k}, n = Ns R, r k < n
             constexpr int TWO = tw_sub_offset(L, Ns * R);
             const cx<T> *__restrict__ twn = tw + TWO;
-            if constexpr (sizeof(T) == 4) {
+            if constexpr (Arith<T>::SINGLE) {
                 cx<T> wp[R];
                 if constexpr (SPNS_F32_TW_POW) {
                     constexpr int P2 = tw_pow_offset(L, Ns * R, 2), P4 = tw_pow_offset(L, Ns * R, 4),

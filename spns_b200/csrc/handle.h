@@ -30,6 +30,12 @@ inline bool spns_length_supported(int L) {
     return false;
 }
 
+// Single-precision x/y passes that transform packed pairs of columns (f2): the forward y
+// pass (N=512 1.59 -> 1.37 ms, LES N=256 0.72 -> 0.59) and the forward x pass from length
+// 288 (N=512 1.30 -> 1.22 ms, N=256 0.168 -> 0.134; LES at 192 0.041 -> 0.055).  The inverse
+// passes wait on their loads, not on issue, and were slower in pairs (y, N=512: 3.65 against
+// 4.13 ms; x 2.78 against 3.15).
+constexpr bool spns_pair_pass(int pass, int L) { return pass == 4 || (pass == 5 && L >= 288); }
 // Tile shapes per pass (complex values per thread E, threads per block),
 // chosen by timing the N=512 step on B200.
 template <typename T, int L, int E_, int THR> struct ShapeT {
@@ -156,7 +162,7 @@ template <typename T, int L, int MODE, int ALT> using ShapeK5A =
 // Per precision: E values per thread, PB pencils per block, SLOTS physical slots
 // in shared memory (of four), MINB resident blocks per SM for the register budget.
 #ifndef SPNS_ZS_MIN_L
-#define SPNS_ZS_MIN_L 768         // double: measured 14.65 against 14.93 ms at 768, slower at 384
+#define SPNS_ZS_MIN_L 384         // double: measured 14.65 against 14.93 ms at 768, slower at 384
 #endif
 #ifndef SPNS_F32_ZS_MIN_L
 #define SPNS_F32_ZS_MIN_L 100000  // single: off (12.29 against 11.61 ms at 768)
@@ -296,6 +302,7 @@ struct spns_handle {
     double nut_stats[3] = {0.0, 0.0, 0.0};           // mean, rms, max of nu_t at the last invariant pass
     bool edge_axis[3] = {false, false, false};       // axes whose +-N/2 planes alias (M = 3h)
     std::map<int, void *> tw;                        // twiddle tables per length (precision of the handle)
+    std::map<int, void *> tw2;                       // single precision: the same tables as packed pairs (f2)
     int sms = 0;                                     // SM count of the handle's device
     // slab decomposition (spns_slab_create): this rank holds the compact ky rows
     // [g.y0, g.y0 + g.Ky) of the state and, in the y and z passes, the x planes
@@ -353,7 +360,7 @@ int spns_fail(spns_handle *h, int code, const char *fmt, ...);
 // divisor n < L of L, in increasing n (spns::tw_sub_offset), and the power tables
 // w_n^{r k} for r = 2, 4, 8 (spns::tw_pow_offset); allocated in stream
 // order on `st` (no device-wide synchronisation).
-template <typename T> inline void *spns_make_twiddles(int L, cudaStream_t st) {
+template <typename T> inline void *spns_make_twiddles(int L, cudaStream_t st, bool pairs = false) {
     const int total = spns::tw_full_size(L);
     std::vector<spns::cx<T>> t(total);
     for (int m = 0; m < L; m++) {
@@ -372,9 +379,15 @@ template <typename T> inline void *spns_make_twiddles(int L, cudaStream_t st) {
             const int off = spns::tw_pow_offset(L, n, r);
             for (int k = 0; k < n; k++) t[off + k] = t[(long long)((r * k) % n) * (L / n)];
         }
+    // pairs: every value twice (the two lanes of cx<f2>)
+    if (pairs) {
+        const std::vector<spns::cx<T>> s = t;
+        t.resize(2 * (size_t)total);
+        for (int i = 0; i < total; i++) { t[2 * i] = {s[i].x, s[i].x}; t[2 * i + 1] = {s[i].y, s[i].y}; }
+    }
     void *d = nullptr;
-    if (cudaMallocAsync(&d, sizeof(spns::cx<T>) * total, st) != cudaSuccess) return nullptr;
-    if (cudaMemcpyAsync(d, t.data(), sizeof(spns::cx<T>) * total, cudaMemcpyHostToDevice, st) != cudaSuccess ||
+    if (cudaMallocAsync(&d, sizeof(spns::cx<T>) * t.size(), st) != cudaSuccess) return nullptr;
+    if (cudaMemcpyAsync(d, t.data(), sizeof(spns::cx<T>) * t.size(), cudaMemcpyHostToDevice, st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess) {
         cudaFreeAsync(d, st);
         return nullptr;

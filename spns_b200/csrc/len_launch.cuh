@@ -13,38 +13,48 @@ template <typename T> struct LenLaunch {
 
     static C *U(spns_handle *h, int f = 0) { return (C *)h->U + (long long)f * h->g.S0; }
     static const C *tw(spns_handle *h, int L) { return (const C *)h->tw[L]; }
+    // arithmetic of the z passes: single precision runs two pencils per thread in packed pairs
+    using A = typename std::conditional<sizeof(T) == 4, spns::f2, T>::type;
+    // arithmetic of the x/y passes
+    template <int PASS, int L> using AX = typename std::conditional<sizeof(T) == 4 && spns_pair_pass(PASS, L), spns::f2, T>::type;
+    template <int PASS, int L> static const spns::cx<AX<PASS, L>> *twx(spns_handle *h) {
+        return (const spns::cx<AX<PASS, L>> *)(sizeof(AX<PASS, L>) != sizeof(T) ? h->tw2[L] : h->tw[L]);
+    }
+    static const spns::cx<A> *twa(spns_handle *h, int L) { return (const spns::cx<A> *)(sizeof(T) == 4 ? h->tw2[L] : h->tw[L]); }
 
+    // kz chunks of an x/y pass with P threads along kz
+    template <typename X> static int axis_chunks(const spns_handle *h, int P) { const int w = P * spns::Arith<X>::W; return (h->g.Kz + w - 1) / w; }
     // Grid of an x/y pass: kz chunks x lines, and for small boxes the fields (or groups of
     // fields) of the pass spread over blocks.
-    static dim3 axis_grid(const spns_handle *h, int P, int lines, int fields) {
-        const int chunks = (h->g.Kz + P - 1) / P;
+    template <typename X> static dim3 axis_grid(const spns_handle *h, int P, int lines, int fields) {
+        const int chunks = axis_chunks<X>(h, P);
         return dim3(chunks, lines, (long long)chunks * lines < (long long)SPNS_SPLIT_WAVES * h->sms ? fields : 1);
     }
     template <int L, int MODE, int ALT = 0> static cudaError_t launch_k1(spns_handle *h) {
-        using S = ShapeK1A<T, L, ALT>;
-        auto kern = spns::k1_inv_x<T, L, S::E, S::P, MODE>;
-        constexpr size_t smem = spns::K1Smem<T, L, S::E, S::P, MODE>::BYTES;
+        using S = ShapeK1A<AX<1, L>, L, ALT>;
+        auto kern = spns::k1_inv_x<AX<1, L>, L, S::E, S::P, MODE>;
+        constexpr size_t smem = spns::K1Smem<AX<1, L>, L, S::E, S::P, MODE>::BYTES;
         cudaError_t e = spns_set_smem(kern, smem);
         if (e != cudaSuccess) return e;
-        const dim3 grid = axis_grid(h, S::P, h->g.Ky, spns::Fields<MODE>::K1);
-        kern<<<grid, S::THREADS, smem, h->st>>>(h->g, U(h, 0), U(h, 1), U(h, 2), (C *)h->B1, tw(h, L));
+        const dim3 grid = axis_grid<AX<1, L>>(h, S::P, h->g.Ky, spns::Fields<MODE>::K1);
+        kern<<<grid, S::THREADS, smem, h->st>>>(h->g, U(h, 0), U(h, 1), U(h, 2), (C *)h->B1, twx<1, L>(h));
         return cudaGetLastError();
     }
     template <int L, int MODE, int ALT = 0> static cudaError_t launch_k2(spns_handle *h) {
-        using S = ShapeK2A<T, L, ALT>;
-        auto kern = spns::k2_inv_y<T, L, S::E, S::P, MODE>;
+        using S = ShapeK2A<AX<2, L>, L, ALT>;
+        auto kern = spns::k2_inv_y<AX<2, L>, L, S::E, S::P, MODE>;
         cudaError_t e = spns_set_smem(kern, S::SMEM_ROW);
         if (e != cudaSuccess) return e;
-        const dim3 grid = axis_grid(h, S::P, h->g.Mx, spns::Fields<MODE>::K2);
-        kern<<<grid, S::THREADS, S::SMEM_ROW, h->st>>>(h->g, (const C *)h->B1, (C *)h->B2, tw(h, L));
+        const dim3 grid = axis_grid<AX<2, L>>(h, S::P, h->g.Mx, spns::Fields<MODE>::K2);
+        kern<<<grid, S::THREADS, S::SMEM_ROW, h->st>>>(h->g, (const C *)h->B1, (C *)h->B2, twx<2, L>(h));
         return cudaGetLastError();
     }
     // Rotational z pass staged pair by pair with bulk copies (zpass_staged.cuh),
     // persistent: one wave of blocks over the SMs.
     template <int L> static cudaError_t launch_k3_staged(spns_handle *h) {
-        using ZS = ZStagedShape<T, L>;
-        using LY = spns::ZStagedLayout<T, L, ZS::E, ZS::PB, ZS::SLOTS>;
-        auto kern = spns::k3_rot_staged<T, L, ZS::E, ZS::PB, ZS::SLOTS, ZS::MINB>;
+        using ZS = ZStagedShape<A, L>;
+        using LY = spns::ZStagedLayout<A, L, ZS::E, ZS::PB, ZS::SLOTS>;
+        auto kern = spns::k3_rot_staged<A, L, ZS::E, ZS::PB, ZS::SLOTS, ZS::MINB>;
         const size_t smem = LY::smem_bytes(h->g.Kz, h->g.Kp);
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
@@ -54,20 +64,20 @@ template <typename T> struct LenLaunch {
         if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
         if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, THREADS, smem)) != cudaSuccess) return e;
         if (per_sm < 1) return cudaErrorInvalidConfiguration;
-        const long long groups = ((long long)h->g.Mx * h->g.My + ZS::PB - 1) / ZS::PB;
+        const long long groups = ((long long)h->g.Mx * h->g.My / LY::W + ZS::PB - 1) / ZS::PB;
         long long blocks = (long long)sms * per_sm;
         if (blocks > groups) blocks = groups;
-        kern<<<(unsigned)blocks, THREADS, smem, h->st>>>(h->g, (C *)h->B2, h->c, h->ds, tw(h, L));
+        kern<<<(unsigned)blocks, THREADS, smem, h->st>>>(h->g, (C *)h->B2, h->c, h->ds, twa(h, L));
         return cudaGetLastError();
     }
     // Persistent launch of k3_field: one wave of blocks.
     template <int L, int MODE, int ALT> static cudaError_t launch_k3_field(spns_handle *h, double *nut) {
-        using S = ZFieldShape<T, L, MODE, ALT>;
-        auto kern = spns::k3_field<T, L, S::E, S::PB, S::NT, MODE, S::MINB>;
+        using S = ZFieldShape<A, L, MODE, ALT>;
+        auto kern = spns::k3_field<A, L, S::E, S::PB, S::NT, MODE, S::MINB>;
         unsigned blocks = 0;
-        cudaError_t e = wave_of_blocks(h, kern, S::THREADS, S::LY::SMEM, ((long long)h->g.Mx * h->g.My + S::PB - 1) / S::PB, &blocks);
+        cudaError_t e = wave_of_blocks(h, kern, S::THREADS, S::LY::SMEM, ((long long)h->g.Mx * h->g.My / spns::Arith<A>::W + S::PB - 1) / S::PB, &blocks);
         if (e != cudaSuccess) return e;
-        kern<<<blocks, S::THREADS, S::LY::SMEM, h->st>>>(h->g, (C *)h->B2, h->c, h->ds, nut, tw(h, L));
+        kern<<<blocks, S::THREADS, S::LY::SMEM, h->st>>>(h->g, (C *)h->B2, h->c, h->ds, nut, twa(h, L));
         return cudaGetLastError();
     }
     // Shared-memory opt-in and grid of a persistent kernel over n work items.
@@ -82,7 +92,7 @@ template <typename T> struct LenLaunch {
     }
     template <int L, int MODE, int ALT = 0> static cudaError_t launch_k3(spns_handle *h, double *phys) {
         if constexpr (MODE != spns::MODE_VEL && (MODE != spns::MODE_ROT || SPNS_ZF_ROT)) return launch_k3_field<L, MODE, ALT>(h, phys);
-        if constexpr (MODE == spns::MODE_ROT && ALT == 0 && ZStagedShape<T, L>::ON) return launch_k3_staged<L>(h);
+        if constexpr (MODE == spns::MODE_ROT && ALT == 0 && ZStagedShape<A, L>::ON) return launch_k3_staged<L>(h);
         using S3 = Shape3<T, L, MODE, ALT>;
         constexpr bool STAGE_ROT = MODE == spns::MODE_ROT && ShapeSel<T>::Z_STAGE;
         constexpr bool STAGE_LES = MODE == spns::MODE_LES && sizeof(T) == 4 && SPNS_F32_Z_STAGE_LES;
@@ -101,21 +111,21 @@ template <typename T> struct LenLaunch {
         return cudaGetLastError();
     }
     template <int L, int MODE, int ALT = 0> static cudaError_t launch_k4(spns_handle *h) {
-        using S = ShapeK4A<T, L, MODE, ALT>;
-        auto kern = spns::k4_fwd_y<T, L, S::E, S::P, MODE>;
+        using S = ShapeK4A<AX<4, L>, L, MODE, ALT>;
+        auto kern = spns::k4_fwd_y<AX<4, L>, L, S::E, S::P, MODE>;
         cudaError_t e = spns_set_smem(kern, S::SMEM_ROW);
         if (e != cudaSuccess) return e;
-        const dim3 grid = axis_grid(h, S::P, h->g.Mx, MODE == spns::MODE_LES ? 5 : spns::Fields<MODE>::NOUT);
-        kern<<<grid, S::THREADS, S::SMEM_ROW, h->st>>>(h->g, (const C *)h->B2, (C *)h->B1, tw(h, L));
+        const dim3 grid = axis_grid<AX<4, L>>(h, S::P, h->g.Mx, MODE == spns::MODE_LES ? 5 : spns::Fields<MODE>::NOUT);
+        kern<<<grid, S::THREADS, S::SMEM_ROW, h->st>>>(h->g, (const C *)h->B2, (C *)h->B1, twx<4, L>(h));
         return cudaGetLastError();
     }
     template <int L, int MODE, int ALT = 0> static cudaError_t launch_k5(spns_handle *h) {
-        using S = ShapeK5A<T, L, MODE, ALT>;
-        auto kern = spns::k5_fwd_x<T, L, S::E, S::P, MODE>;
+        using S = ShapeK5A<AX<5, L>, L, MODE, ALT>;
+        auto kern = spns::k5_fwd_x<AX<5, L>, L, S::E, S::P, MODE>;
         cudaError_t e = spns_set_smem(kern, S::SMEM_ROW);
         if (e != cudaSuccess) return e;
-        const dim3 grid = axis_grid(h, S::P, h->g.Ky, spns::Fields<MODE>::NOUT);
-        kern<<<grid, S::THREADS, S::SMEM_ROW, h->st>>>(h->g, (const C *)h->B1, (C *)h->B2, tw(h, L));
+        const dim3 grid = axis_grid<AX<5, L>>(h, S::P, h->g.Ky, spns::Fields<MODE>::NOUT);
+        kern<<<grid, S::THREADS, S::SMEM_ROW, h->st>>>(h->g, (const C *)h->B1, (C *)h->B2, twx<5, L>(h));
         return cudaGetLastError();
     }
     // Launch of pass K1..K5 in the shape the handle selected (shape_alt).
@@ -152,44 +162,44 @@ template <typename T> struct LenLaunch {
     }
     // ---- batched launches: one per pass for the members of a table, all of h0's class ----
     template <int L, int MODE, int ALT> static cudaError_t launch_k1b(spns_handle *h, const spns::BatchMember *tab, int n, cudaStream_t st) {
-        using S = ShapeK1A<T, L, ALT>;
-        auto kern = spns::k1_inv_x_batch<T, L, S::E, S::P, MODE>;
+        using S = ShapeK1A<AX<1, L>, L, ALT>;
+        auto kern = spns::k1_inv_x_batch<AX<1, L>, L, S::E, S::P, MODE>;
         cudaError_t e = spns_set_smem(kern, S::SMEM_ROW);
         if (e != cudaSuccess) return e;
-        kern<<<dim3((h->g.Kz + S::P - 1) / S::P, h->g.Ky, n), S::THREADS, S::SMEM_ROW, st>>>(h->g, tab, tw(h, L));
+        kern<<<dim3(axis_chunks<AX<1, L>>(h, S::P), h->g.Ky, n), S::THREADS, S::SMEM_ROW, st>>>(h->g, tab, twx<1, L>(h));
         return cudaGetLastError();
     }
     template <int L, int MODE, int ALT> static cudaError_t launch_k2b(spns_handle *h, const spns::BatchMember *tab, int n, cudaStream_t st) {
-        using S = ShapeK2A<T, L, ALT>;
-        auto kern = spns::k2_inv_y_batch<T, L, S::E, S::P, MODE>;
+        using S = ShapeK2A<AX<2, L>, L, ALT>;
+        auto kern = spns::k2_inv_y_batch<AX<2, L>, L, S::E, S::P, MODE>;
         cudaError_t e = spns_set_smem(kern, S::SMEM_ROW);
         if (e != cudaSuccess) return e;
-        kern<<<dim3((h->g.Kz + S::P - 1) / S::P, h->g.Mx, n), S::THREADS, S::SMEM_ROW, st>>>(h->g, tab, tw(h, L));
+        kern<<<dim3(axis_chunks<AX<2, L>>(h, S::P), h->g.Mx, n), S::THREADS, S::SMEM_ROW, st>>>(h->g, tab, twx<2, L>(h));
         return cudaGetLastError();
     }
     template <int L, int MODE, int ALT> static cudaError_t launch_k3b(spns_handle *h, const spns::BatchMember *tab, int n, cudaStream_t st) {
-        using S = ZFieldShape<T, L, MODE, ALT>;
-        auto kern = spns::k3_field_batch<T, L, S::E, S::PB, S::NT, MODE, S::MINB>;
+        using S = ZFieldShape<A, L, MODE, ALT>;
+        auto kern = spns::k3_field_batch<A, L, S::E, S::PB, S::NT, MODE, S::MINB>;
         unsigned blocks = 0;
-        cudaError_t e = wave_of_blocks(h, kern, S::THREADS, S::LY::SMEM, ((long long)h->g.Mx * h->g.My + S::PB - 1) / S::PB, &blocks);
+        cudaError_t e = wave_of_blocks(h, kern, S::THREADS, S::LY::SMEM, ((long long)h->g.Mx * h->g.My / spns::Arith<A>::W + S::PB - 1) / S::PB, &blocks);
         if (e != cudaSuccess) return e;
-        kern<<<dim3(blocks, n), S::THREADS, S::LY::SMEM, st>>>(h->g, tab, tw(h, L));
+        kern<<<dim3(blocks, n), S::THREADS, S::LY::SMEM, st>>>(h->g, tab, twa(h, L));
         return cudaGetLastError();
     }
     template <int L, int MODE, int ALT> static cudaError_t launch_k4b(spns_handle *h, const spns::BatchMember *tab, int n, cudaStream_t st) {
-        using S = ShapeK4A<T, L, MODE, ALT>;
-        auto kern = spns::k4_fwd_y_batch<T, L, S::E, S::P, MODE>;
+        using S = ShapeK4A<AX<4, L>, L, MODE, ALT>;
+        auto kern = spns::k4_fwd_y_batch<AX<4, L>, L, S::E, S::P, MODE>;
         cudaError_t e = spns_set_smem(kern, S::SMEM_ROW);
         if (e != cudaSuccess) return e;
-        kern<<<dim3((h->g.Kz + S::P - 1) / S::P, h->g.Mx, n), S::THREADS, S::SMEM_ROW, st>>>(h->g, tab, tw(h, L));
+        kern<<<dim3(axis_chunks<AX<4, L>>(h, S::P), h->g.Mx, n), S::THREADS, S::SMEM_ROW, st>>>(h->g, tab, twx<4, L>(h));
         return cudaGetLastError();
     }
     template <int L, int MODE, int ALT> static cudaError_t launch_k5b(spns_handle *h, const spns::BatchMember *tab, int n, cudaStream_t st) {
-        using S = ShapeK5A<T, L, MODE, ALT>;
-        auto kern = spns::k5_fwd_x_batch<T, L, S::E, S::P, MODE>;
+        using S = ShapeK5A<AX<5, L>, L, MODE, ALT>;
+        auto kern = spns::k5_fwd_x_batch<AX<5, L>, L, S::E, S::P, MODE>;
         cudaError_t e = spns_set_smem(kern, S::SMEM_ROW);
         if (e != cudaSuccess) return e;
-        kern<<<dim3((h->g.Kz + S::P - 1) / S::P, h->g.Ky, n), S::THREADS, S::SMEM_ROW, st>>>(h->g, tab, tw(h, L));
+        kern<<<dim3(axis_chunks<AX<5, L>>(h, S::P), h->g.Ky, n), S::THREADS, S::SMEM_ROW, st>>>(h->g, tab, twx<5, L>(h));
         return cudaGetLastError();
     }
 #define SPNS_SELECT_B(name, idx)                                                                                       \

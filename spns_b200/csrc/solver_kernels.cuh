@@ -123,6 +123,42 @@ template <int MODE> struct Fields {
 };
 
 // ===========================================================================
+// Elements of the x/y passes.  A thread transforms one kz column, or in single precision
+// (T = f2) two adjacent ones, which are 16 bytes of a row: the same tiles, shared-memory
+// layouts and launch shapes as in double precision.
+// ===========================================================================
+template <typename T> using SCx = cx<typename Arith<T>::S>;   // element of the arrays in memory
+// Work buffers (S1, S2): rows start on 16 bytes and are padded, so both columns are always there.
+__device__ __forceinline__ cx<double> ld_work(const cx<double> *p, cx<double> *) { return *p; }
+__device__ __forceinline__ cx<float> ld_work(const cx<float> *p, cx<float> *) { return *p; }
+__device__ __forceinline__ cx<f2> ld_work(const cx<float> *p, cx<f2> *) {
+    const float4 a = *reinterpret_cast<const float4 *>(p);
+    return mk<f2>(f2(a.x, a.z), f2(a.y, a.w));
+}
+__device__ __forceinline__ void st_work(cx<double> *p, cx<double> v) { *p = v; }
+__device__ __forceinline__ void st_work(cx<float> *p, cx<float> v) { *p = v; }
+__device__ __forceinline__ void st_work(cx<float> *p, cx<f2> v) {
+    *reinterpret_cast<float4 *>(p) = make_float4(v.x.lo(), v.y.lo(), v.x.hi(), v.y.hi());
+}
+// Compact arrays (S0): rows of Kz elements, so a pair may straddle 16 bytes and the last row end (two: it is whole).
+__device__ __forceinline__ cx<double> ld_compact(const cx<double> *p, bool, cx<double> *) { return *p; }
+__device__ __forceinline__ cx<float> ld_compact(const cx<float> *p, bool, cx<float> *) { return *p; }
+__device__ __forceinline__ cx<f2> ld_compact(const cx<float> *p, bool two, cx<f2> *) {
+    const cx<float> a = p[0], b = two ? p[1] : zero<float>();
+    return mk<f2>(f2(a.x, b.x), f2(a.y, b.y));
+}
+__device__ __forceinline__ void st_compact(cx<double> *p, cx<double> v, bool) { *p = v; }
+__device__ __forceinline__ void st_compact(cx<float> *p, cx<float> v, bool) { *p = v; }
+__device__ __forceinline__ void st_compact(cx<float> *p, cx<f2> v, bool two) {
+    p[0] = mk<float>(v.x.lo(), v.y.lo());
+    if (two) p[1] = mk<float>(v.x.hi(), v.y.hi());
+}
+// s kz of the thread's columns
+__device__ __forceinline__ double col_k(int s, int kz, double *) { return (double)(s * kz); }
+__device__ __forceinline__ float col_k(int s, int kz, float *) { return (float)(s * kz); }
+__device__ __forceinline__ f2 col_k(int s, int kz, f2 *) { return f2((float)(s * kz), (float)(s * kz + s)); }
+
+// ===========================================================================
 // K1: inverse transform along x.  Block = (kz chunk, iy).
 //   VEL: u,v,w   ROT: u,v,w and the vorticity   ADV/LES: u,v,w, du/dx, dv/dx, dw/dx
 // ky and kz are constant along a line, so of the vorticity w_x = i(ky w - kz v),
@@ -135,22 +171,23 @@ template <typename T, int L, int E, int P, int MODE> struct K1Smem {
     static constexpr size_t BYTES = (size_t)L * P * sizeof(cx<T>) * (MODE == MODE_ROT ? 2 : 1);
 };
 template <typename T, int L, int E, int P, int MODE>
-__device__ __forceinline__ void k1_inv_x_body(Geo g, const cx<T> *__restrict__ u, const cx<T> *__restrict__ v,
-                                              const cx<T> *__restrict__ w, cx<T> *__restrict__ out, const cx<T> *__restrict__ tw,
+__device__ __forceinline__ void k1_inv_x_body(Geo g, const SCx<T> *__restrict__ u, const SCx<T> *__restrict__ v,
+                                              const SCx<T> *__restrict__ w, SCx<T> *__restrict__ out, const cx<T> *__restrict__ tw,
                                               int f0, int fs) {
     extern __shared__ __align__(16) unsigned char smraw[];
     constexpr int THREADS = P * (L / E);
     const int tid = threadIdx.x, p = tid % P, q = tid / P;
-    const int iy = blockIdx.y, kz = blockIdx.x * P + p;
-    const bool ok = kz < g.Kz;
+    const int iy = blockIdx.y, kz = (blockIdx.x * P + p) * Arith<T>::W;
+    const bool ok = kz < g.Kz, two = kz + 1 < g.Kz;
     SmRowMajor<T, P> sm{reinterpret_cast<cx<T> *>(smraw), p};
     const long long rb = (long long)iy * g.Kx * g.Kz + kz, ob = (long long)iy * g.Mx * g.Kp + kz;
     // loads the field into the input rows, times kx where `deriv` (all loads before the first use)
-    auto load = [&](cx<T>(&r)[E], const cx<T> *src, bool deriv) {
+    auto load = [&](cx<T>(&r)[E], const SCx<T> *src, bool deriv) {
 #pragma unroll
         for (int e = 0; e < E; e++) {
             const int m1 = ffreq(in_row<L, E, true>(q, e), L);
-            r[e] = (ok && m1 <= g.hx && m1 >= -g.hx) ? src[rb + (long long)(m1 >= 0 ? m1 : m1 + g.Kx) * g.Kz] : zero<T>();
+            r[e] = (ok && m1 <= g.hx && m1 >= -g.hx) ? ld_compact(src + rb + (long long)(m1 >= 0 ? m1 : m1 + g.Kx) * g.Kz, two, (cx<T> *)nullptr)
+                                                           : zero<T>();
         }
         if (deriv) {
 #pragma unroll
@@ -159,12 +196,12 @@ __device__ __forceinline__ void k1_inv_x_body(Geo g, const cx<T> *__restrict__ u
     };
     auto put = [&](int f, auto value) {
         if (!ok) return;
-        cx<T> *o = out + (long long)f * g.S1 + ob;
+        SCx<T> *o = out + (long long)f * g.S1 + ob;
 #pragma unroll
-        for (int e = 0; e < E; e++) o[(long long)out_row<L, E, true>(q, e) * g.Kp] = value(e);
+        for (int e = 0; e < E; e++) st_work(o + (long long)out_row<L, E, true>(q, e) * g.Kp, value(e));
     };
     if constexpr (MODE == MODE_ROT) {
-        const T kzf = T(g.sz * kz), kyf = T(g.sy * ky_mode(g, iy));
+        const T kzf = col_k(g.sz, kz, (T *)nullptr), kyf = T(g.sy * ky_mode(g, iy));
         cx<T> *const slot = reinterpret_cast<cx<T> *>(smraw) + L * P + tid;
         if (fs > 1) {   // outputs split over blocks: each forms its own input
 #pragma unroll 1
@@ -215,11 +252,11 @@ __device__ __forceinline__ void k1_inv_x_body(Geo g, const cx<T> *__restrict__ u
 //   ADV/LES: u,v,w, du/dx,dv/dx,dw/dx, du/dy,dv/dy,dw/dy
 // ===========================================================================
 template <typename T, int L, int E, int P, int MODE>
-__device__ __forceinline__ void k2_inv_y_body(Geo g, const cx<T> *__restrict__ in, cx<T> *__restrict__ out,
+__device__ __forceinline__ void k2_inv_y_body(Geo g, const SCx<T> *__restrict__ in, SCx<T> *__restrict__ out,
                                               const cx<T> *__restrict__ tw, int f0, int fs) {
     extern __shared__ __align__(16) unsigned char smraw[];
     const int tid = threadIdx.x, p = tid % P, q0 = tid / P;
-    const int x = blockIdx.y, kz = blockIdx.x * P + p;
+    const int x = blockIdx.y, kz = (blockIdx.x * P + p) * Arith<T>::W;
     const bool ok = kz < g.Kz;
     SmRowMajor<T, P> sm{reinterpret_cast<cx<T> *>(smraw), p};
     // row offsets in 32 bits (a field has fewer than 2^31 elements at every compiled length):
@@ -230,11 +267,11 @@ __device__ __forceinline__ void k2_inv_y_body(Geo g, const cx<T> *__restrict__ i
         const int q = opaque(q0);
         cx<T> r[E];
         const bool deriv = (MODE == MODE_ADV || MODE == MODE_LES || MODE == MODE_INV) && f >= 6;
-        const cx<T> *F = in + (long long)(deriv ? f - 6 : f) * g.S1;
+        const SCx<T> *F = in + (long long)(deriv ? f - 6 : f) * g.S1;
 #pragma unroll
         for (int e = 0; e < E; e++) {
             const int m2 = ffreq(in_row<L, E, true>(q, e), L);
-            r[e] = (ok && m2 <= g.hy && m2 >= -g.hy) ? F[col + (unsigned)(m2 >= 0 ? m2 : m2 + g.Ky) * rs] : zero<T>();
+            r[e] = (ok && m2 <= g.hy && m2 >= -g.hy) ? ld_work(F + (col + (unsigned)(m2 >= 0 ? m2 : m2 + g.Ky) * rs), (cx<T> *)nullptr) : zero<T>();
         }
         if (deriv) {
 #pragma unroll
@@ -242,9 +279,9 @@ __device__ __forceinline__ void k2_inv_y_body(Geo g, const cx<T> *__restrict__ i
         }
         fft<T, L, E, true>(r, sm, q, tw);
         if (ok) {
-            cx<T> *o = out + (long long)f * g.S2;
+            SCx<T> *o = out + (long long)f * g.S2;
 #pragma unroll
-            for (int e = 0; e < E; e++) o[col + (unsigned)out_row<L, E, true>(q, e) * rs] = r[e];
+            for (int e = 0; e < E; e++) st_work(o + (col + (unsigned)out_row<L, E, true>(q, e) * rs), r[e]);
         }
     }
 }
@@ -257,11 +294,25 @@ __device__ __forceinline__ void k2_inv_y_body(Geo g, const cx<T> *__restrict__ i
 // pencils; each thread keeps the values of its own grid rows in registers, so
 // the inverse/forward hand-off needs no shared-memory round trip.
 // ===========================================================================
+// Element k of the pencil(s) a thread transforms: one pencil, or two (T = f2) that lie
+// `step` elements apart.
+__device__ __forceinline__ cx<double> ld_pencil(const cx<double> *p, int k, int, cx<double> *) { return p[k]; }
+__device__ __forceinline__ cx<float> ld_pencil(const cx<float> *p, int k, int, cx<float> *) { return p[k]; }
+__device__ __forceinline__ cx<f2> ld_pencil(const cx<float> *p, int k, int step, cx<f2> *) {
+    const cx<float> a = p[k], b = p[k + step];
+    return mk<f2>(f2(a.x, b.x), f2(a.y, b.y));
+}
+__device__ __forceinline__ void st_pencil(cx<double> *p, int k, int, cx<double> v) { p[k] = v; }
+__device__ __forceinline__ void st_pencil(cx<float> *p, int k, int, cx<float> v) { p[k] = v; }
+__device__ __forceinline__ void st_pencil(cx<float> *p, int k, int step, cx<f2> v) {
+    p[k] = mk<float>(v.x.lo(), v.y.lo());
+    p[k + step] = mk<float>(v.x.hi(), v.y.hi());
+}
 // Loads the 2-for-1 spectrum Z = Xa + i Xb at the thread's input rows.
 // ma/mb: multiply the field by i*kz (z derivative) first.
 template <typename T, int L, int E>
-__device__ __forceinline__ void k3_load_pair(cx<T> (&r)[E], const cx<T> *__restrict__ A, bool ma, const cx<T> *__restrict__ B,
-                                             bool mb, int Kz, T sz, int q, bool ok) {
+__device__ __forceinline__ void k3_load_pair(cx<T> (&r)[E], const SCx<T> *__restrict__ A, bool ma, const SCx<T> *__restrict__ B,
+                                             bool mb, int Kz, T sz, int q, bool ok, int step = 0) {
 #pragma unroll
     for (int e = 0; e < E; e++) {
         const int row = in_row<L, E, true>(q, e);
@@ -270,7 +321,7 @@ __device__ __forceinline__ void k3_load_pair(cx<T> (&r)[E], const cx<T> *__restr
             const bool lo = row < Kz, hi = row > L - Kz;
             if (lo || hi) {
                 const int kk = lo ? row : L - row;
-                cx<T> a = A[kk], b = B ? B[kk] : zero<T>();
+                cx<T> a = ld_pencil(A, kk, step, (cx<T> *)nullptr), b = B ? ld_pencil(B, kk, step, (cx<T> *)nullptr) : zero<T>();
                 if (ma) a = mul_i(T(kk) * sz * a);
                 if (mb) b = mul_i(T(kk) * sz * b);
                 if (row == 0) z = mk<T>(a.x, b.x);
@@ -427,6 +478,13 @@ __device__ __forceinline__ void cfl_update(double (&mx)[4], double uu, double vv
     if (!(s <= 1.7976931348623157e308)) { mx[0] = mx[1] = mx[2] = mx[3] = __longlong_as_double(0x7ff0000000000000LL); return; }
     mx[0] = fmax(mx[0], au); mx[1] = fmax(mx[1], av); mx[2] = fmax(mx[2], aw);
     mx[3] = fmax(mx[3], s);
+}
+
+__device__ __forceinline__ void cfl_rows(double (&mx)[4], double u, double v, double w, const StepConsts &c) { cfl_update<double>(mx, u, v, w, c); }
+__device__ __forceinline__ void cfl_rows(double (&mx)[4], float u, float v, float w, const StepConsts &c) { cfl_update<float>(mx, u, v, w, c); }
+__device__ __forceinline__ void cfl_rows(double (&mx)[4], f2 u, f2 v, f2 w, const StepConsts &c) {
+    cfl_update<float>(mx, u.lo(), v.lo(), w.lo(), c);
+    cfl_update<float>(mx, u.hi(), v.hi(), w.hi(), c);
 }
 
 // Asynchronous global->shared copy of one complex element (LDGSTS; 16 B for
@@ -941,11 +999,11 @@ template <int MODE> __host__ __device__ constexpr int k4_in_field(int f) { retur
 // LES: G_i += i ky t_i2 (SGS divergence, y part).
 // ===========================================================================
 template <typename T, int L, int E, int P, int MODE>
-__device__ __forceinline__ void k4_fwd_y_body(Geo g, const cx<T> *__restrict__ in, cx<T> *__restrict__ out,
+__device__ __forceinline__ void k4_fwd_y_body(Geo g, const SCx<T> *__restrict__ in, SCx<T> *__restrict__ out,
                                               const cx<T> *__restrict__ tw, int f0, int fs) {
     extern __shared__ __align__(16) unsigned char smraw[];
     const int tid = threadIdx.x, p = tid % P, q0 = tid / P;
-    const int x = blockIdx.y, kz = blockIdx.x * P + p;
+    const int x = blockIdx.y, kz = (blockIdx.x * P + p) * Arith<T>::W;
     const bool ok = kz < g.Kz;
     SmRowMajor<T, P> sm{reinterpret_cast<cx<T> *>(smraw), p};
     const unsigned col = (unsigned)x * g.Kp + kz, rs = (unsigned)g.Mx * g.Kp;
@@ -956,19 +1014,19 @@ __device__ __forceinline__ void k4_fwd_y_body(Geo g, const cx<T> *__restrict__ i
     constexpr int NG = LES ? 5 : Fields<MODE>::NOUT;
     auto load_fft = [&](cx<T>(&r)[E], int f) {
         const int q = opaque(q0);
-        const cx<T> *src = in + (long long)f * g.S2;
+        const SCx<T> *src = in + (long long)f * g.S2;
 #pragma unroll
-        for (int e = 0; e < E; e++) r[e] = ok ? src[col + (unsigned)in_row<L, E, false>(q, e) * rs] : zero<T>();
+        for (int e = 0; e < E; e++) r[e] = ok ? ld_work(src + (col + (unsigned)in_row<L, E, false>(q, e) * rs), (cx<T> *)nullptr) : zero<T>();
         fft<T, L, E, false>(r, sm, q, tw);
     };
     auto store = [&](int f, auto value) {
         if (!ok) return;
         const int q = opaque(q0);
-        cx<T> *o = out + (long long)f * g.S1;
+        SCx<T> *o = out + (long long)f * g.S1;
 #pragma unroll
         for (int e = 0; e < E; e++) {
             const int m2 = ffreq(out_row<L, E, false>(q, e), L);
-            if (m2 <= g.hy && m2 >= -g.hy) o[col + (unsigned)(m2 >= 0 ? m2 : m2 + g.Ky) * rs] = value(e, m2);
+            if (m2 <= g.hy && m2 >= -g.hy) st_work(o + (col + (unsigned)(m2 >= 0 ? m2 : m2 + g.Ky) * rs), value(e, m2));
         }
     };
 #pragma unroll 1
@@ -993,19 +1051,19 @@ __device__ __forceinline__ void k4_fwd_y_body(Geo g, const cx<T> *__restrict__ i
 // (S0).  Block = (kz chunk, iy).  LES: G_i += i kx t_i1 (SGS divergence, x part).
 // ===========================================================================
 template <typename T, int L, int E, int P, int MODE>
-__device__ __forceinline__ void k5_fwd_x_body(Geo g, const cx<T> *__restrict__ in, cx<T> *__restrict__ G,
+__device__ __forceinline__ void k5_fwd_x_body(Geo g, const SCx<T> *__restrict__ in, SCx<T> *__restrict__ G,
                                               const cx<T> *__restrict__ tw, int f0, int fs) {
     extern __shared__ __align__(16) unsigned char smraw[];
     const int tid = threadIdx.x, p = tid % P, q = tid / P;
-    const int iy = blockIdx.y, kz = blockIdx.x * P + p;
-    const bool ok = kz < g.Kz;
+    const int iy = blockIdx.y, kz = (blockIdx.x * P + p) * Arith<T>::W;
+    const bool ok = kz < g.Kz, two = kz + 1 < g.Kz;
     SmRowMajor<T, P> sm{reinterpret_cast<cx<T> *>(smraw), p};
     const long long col = (long long)iy * g.Mx * g.Kp + kz;
     constexpr bool LES = MODE == MODE_LES;
     auto load_fft = [&](cx<T>(&r)[E], int f) {
-        const cx<T> *src = in + (long long)f * g.S1 + col;
+        const SCx<T> *src = in + (long long)f * g.S1 + col;
 #pragma unroll
-        for (int e = 0; e < E; e++) r[e] = ok ? src[(long long)in_row<L, E, false>(q, e) * g.Kp] : zero<T>();
+        for (int e = 0; e < E; e++) r[e] = ok ? ld_work(src + (long long)in_row<L, E, false>(q, e) * g.Kp, (cx<T> *)nullptr) : zero<T>();
         fft<T, L, E, false>(r, sm, q, tw);
     };
 #pragma unroll 1
@@ -1014,14 +1072,14 @@ __device__ __forceinline__ void k5_fwd_x_body(Geo g, const cx<T> *__restrict__ i
         load_fft(r, f);
         if constexpr (LES) load_fft(t, 3 + f);   // t11, t12, t13
         if (!ok) continue;
-        cx<T> *o = G + (long long)f * g.S0 + (long long)iy * g.Kx * g.Kz + kz;
+        SCx<T> *o = G + (long long)f * g.S0 + (long long)iy * g.Kx * g.Kz + kz;
 #pragma unroll
         for (int e = 0; e < E; e++) {
             const int m1 = ffreq(out_row<L, E, false>(q, e), L);
             if (m1 > g.hx || m1 < -g.hx) continue;
             cx<T> val = r[e];
             if constexpr (LES) val = val + mul_i(T(g.sx * m1) * t[e]);
-            o[(long long)(m1 >= 0 ? m1 : m1 + g.Kx) * g.Kz] = val;
+            st_compact(o + (long long)(m1 >= 0 ? m1 : m1 + g.Kx) * g.Kz, val, two);
         }
     }
 }
@@ -1627,13 +1685,13 @@ static __global__ void k_dft_axis(const double2 *__restrict__ in, double2 *__res
 // come from a device table (BatchMember).  The arithmetic is the one-box kernel's.
 // ===========================================================================
 template <typename T, int L, int E, int P, int MODE>
-__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 1, MODE>::N) k1_inv_x(Geo g, const cx<T> *__restrict__ u, const cx<T> *__restrict__ v,
-                                                                           const cx<T> *__restrict__ w, cx<T> *__restrict__ out,
+__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 1, MODE>::N) k1_inv_x(Geo g, const SCx<T> *__restrict__ u, const SCx<T> *__restrict__ v,
+                                                                           const SCx<T> *__restrict__ w, SCx<T> *__restrict__ out,
                                                                            const cx<T> *__restrict__ tw) {
     k1_inv_x_body<T, L, E, P, MODE>(g, u, v, w, out, tw, blockIdx.z, gridDim.z);
 }
 template <typename T, int L, int E, int P, int MODE>
-__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 2, MODE>::N) k2_inv_y(Geo g, const cx<T> *__restrict__ in, cx<T> *__restrict__ out,
+__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 2, MODE>::N) k2_inv_y(Geo g, const SCx<T> *__restrict__ in, SCx<T> *__restrict__ out,
                                                                            const cx<T> *__restrict__ tw) {
     k2_inv_y_body<T, L, E, P, MODE>(g, in, out, tw, blockIdx.z, gridDim.z);
 }
@@ -1644,12 +1702,12 @@ __global__ void __launch_bounds__(P *(L / E), K3MinBlocks<T, MODE, P *(L / E)>::
     k3_z_body<T, L, E, P, MODE, STAGE>(g, buf, c, ds, phys, tw);
 }
 template <typename T, int L, int E, int P, int MODE>
-__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 4, MODE>::N) k4_fwd_y(Geo g, const cx<T> *__restrict__ in, cx<T> *__restrict__ out,
+__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 4, MODE>::N) k4_fwd_y(Geo g, const SCx<T> *__restrict__ in, SCx<T> *__restrict__ out,
                                                                            const cx<T> *__restrict__ tw) {
     k4_fwd_y_body<T, L, E, P, MODE>(g, in, out, tw, blockIdx.z, gridDim.z);
 }
 template <typename T, int L, int E, int P, int MODE>
-__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 5, MODE>::N) k5_fwd_x(Geo g, const cx<T> *__restrict__ in, cx<T> *__restrict__ G,
+__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 5, MODE>::N) k5_fwd_x(Geo g, const SCx<T> *__restrict__ in, SCx<T> *__restrict__ G,
                                                                            const cx<T> *__restrict__ tw) {
     k5_fwd_x_body<T, L, E, P, MODE>(g, in, G, tw, blockIdx.z, gridDim.z);
 }
@@ -1672,14 +1730,14 @@ template <typename T, int L, int E, int P, int MODE>
 __global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 1, MODE>::N) k1_inv_x_batch(Geo g, const BatchMember *__restrict__ tab,
                                                                                  const cx<T> *__restrict__ tw) {
     const BatchMember &m = tab[blockIdx.z];
-    const cx<T> *U = static_cast<const cx<T> *>(m.U);
-    k1_inv_x_body<T, L, E, P, MODE>(g, U, U + g.S0, U + 2 * g.S0, static_cast<cx<T> *>(m.B1), tw, 0, 1);
+    const SCx<T> *U = static_cast<const SCx<T> *>(m.U);
+    k1_inv_x_body<T, L, E, P, MODE>(g, U, U + g.S0, U + 2 * g.S0, static_cast<SCx<T> *>(m.B1), tw, 0, 1);
 }
 template <typename T, int L, int E, int P, int MODE>
 __global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 2, MODE>::N) k2_inv_y_batch(Geo g, const BatchMember *__restrict__ tab,
                                                                                  const cx<T> *__restrict__ tw) {
     const BatchMember &m = tab[blockIdx.z];
-    k2_inv_y_body<T, L, E, P, MODE>(g, static_cast<const cx<T> *>(m.B1), static_cast<cx<T> *>(m.B2), tw, 0, 1);
+    k2_inv_y_body<T, L, E, P, MODE>(g, static_cast<const SCx<T> *>(m.B1), static_cast<SCx<T> *>(m.B2), tw, 0, 1);
 }
 template <typename T, int L, int E, int P, int MODE, bool STAGE = false>
 __global__ void __launch_bounds__(P *(L / E), K3MinBlocks<T, MODE, P *(L / E)>::N) k3_z_batch(Geo g, const BatchMember *__restrict__ tab,
@@ -1691,13 +1749,13 @@ template <typename T, int L, int E, int P, int MODE>
 __global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 4, MODE>::N) k4_fwd_y_batch(Geo g, const BatchMember *__restrict__ tab,
                                                                                  const cx<T> *__restrict__ tw) {
     const BatchMember &m = tab[blockIdx.z];
-    k4_fwd_y_body<T, L, E, P, MODE>(g, static_cast<const cx<T> *>(m.B2), static_cast<cx<T> *>(m.B1), tw, 0, 1);
+    k4_fwd_y_body<T, L, E, P, MODE>(g, static_cast<const SCx<T> *>(m.B2), static_cast<SCx<T> *>(m.B1), tw, 0, 1);
 }
 template <typename T, int L, int E, int P, int MODE>
 __global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 5, MODE>::N) k5_fwd_x_batch(Geo g, const BatchMember *__restrict__ tab,
                                                                                  const cx<T> *__restrict__ tw) {
     const BatchMember &m = tab[blockIdx.z];
-    k5_fwd_x_body<T, L, E, P, MODE>(g, static_cast<const cx<T> *>(m.B1), static_cast<cx<T> *>(m.B2), tw, 0, 1);
+    k5_fwd_x_body<T, L, E, P, MODE>(g, static_cast<const SCx<T> *>(m.B1), static_cast<SCx<T> *>(m.B2), tw, 0, 1);
 }
 // Adams-Bashforth members only (the kappa scheme swaps state buffers every step).
 template <typename T>

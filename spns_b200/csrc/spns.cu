@@ -364,6 +364,7 @@ static void free_handle(spns_handle *h) {
     for (void *b : bufs)
         if (b) cudaFreeAsync(b, h->st);
     for (auto &kv : h->tw) cudaFreeAsync(kv.second, h->st);
+    for (auto &kv : h->tw2) if (kv.second) cudaFreeAsync(kv.second, h->st);
     for (auto ev : h->prof_ev) cudaEventDestroy(ev);
     for (auto &gx : h->graph) if (gx) cudaGraphExecDestroy(gx);
     if (h->edge_fork) cudaEventDestroy(h->edge_fork);
@@ -458,6 +459,8 @@ int spns_create(const spns_hit_args *args, const double *file_uvw, spns_handle *
             void *t = hilo ? spns_make_twiddles<float>(L, h->st) : spns_make_twiddles<double>(L, h->st);
             if (!t) return cleanup(spns_fail(nullptr, SPNS_ERR_OUT_OF_MEMORY, "twiddle allocation failed"));
             h->tw[L] = t;
+            if (hilo && !(h->tw2[L] = spns_make_twiddles<float>(L, h->st, true)))
+                return cleanup(spns_fail(nullptr, SPNS_ERR_OUT_OF_MEMORY, "twiddle allocation failed"));
         }
     DevScalars s0v;
     memset(&s0v, 0, sizeof(s0v));
@@ -1121,6 +1124,8 @@ extern "C" int spns_slab_create(const spns_hit_args *args, int nranks, int rank,
             void *t = hilo ? spns_make_twiddles<float>(L, h->st) : spns_make_twiddles<double>(L, h->st);
             if (!t) return cleanup(spns_fail(nullptr, SPNS_ERR_OUT_OF_MEMORY, "twiddle allocation failed"));
             h->tw[L] = t;
+            if (hilo && !(h->tw2[L] = spns_make_twiddles<float>(L, h->st, true)))
+                return cleanup(spns_fail(nullptr, SPNS_ERR_OUT_OF_MEMORY, "twiddle allocation failed"));
         }
     DevScalars s0v;
     memset(&s0v, 0, sizeof(s0v));

@@ -146,6 +146,23 @@ __device__ __forceinline__ void zfield_row(cx<T> (&v)[ZFieldForm<MODE>::NPAIR], 
     }
 }
 
+// The row of a thread: one pencil's, or one of each pencil of a pair.
+template <int MODE, typename T>
+__device__ __forceinline__ void zfield_rows(cx<T> (&v)[ZFieldForm<MODE>::NPAIR], const StepConsts &c, double (&mx)[4], double (&nut)[3]) {
+    if constexpr (Arith<T>::W == 1) {
+        zfield_row<T, MODE>(v, c, mx, nut);
+    } else {
+        constexpr int N = ZFieldForm<MODE>::NPAIR;
+        cx<float> a[N], b[N];
+#pragma unroll
+        for (int p = 0; p < N; p++) { a[p] = mk<float>(v[p].x.lo(), v[p].y.lo()); b[p] = mk<float>(v[p].x.hi(), v[p].y.hi()); }
+        zfield_row<float, MODE>(a, c, mx, nut);
+        zfield_row<float, MODE>(b, c, mx, nut);
+#pragma unroll
+        for (int p = 0; p < ZFieldForm<MODE>::NJOB; p++) v[p] = mk<f2>(f2(a[p].x, b[p].x), f2(a[p].y, b[p].y));
+    }
+}
+
 template <typename T, int L, int E, int PB, int NT, int MODE> struct ZFieldLayout {
     static constexpr int Q = L / E;
     // teams of a warp; where Q does not divide 32 the last lanes of a warp have no team
@@ -163,7 +180,7 @@ template <typename T, int L, int E, int PB, int NT, int MODE> struct ZFieldLayou
 };
 
 template <typename T, int L, int E, int PB, int NT, int MODE>
-__device__ __forceinline__ void k3_field_body(Geo g, cx<T> *__restrict__ buf, const StepConsts &c, DevScalars *ds,
+__device__ __forceinline__ void k3_field_body(Geo g, SCx<T> *__restrict__ buf, const StepConsts &c, DevScalars *ds,
                                               double *__restrict__ nut_out, const cx<T> *__restrict__ tw) {
     using LY = ZFieldLayout<T, L, E, PB, NT, MODE>;
     constexpr int Q = LY::Q, NPAIR = LY::NPAIR, NJOB = LY::NJOB, PITCH = LY::PITCH;
@@ -173,7 +190,9 @@ __device__ __forceinline__ void k3_field_body(Geo g, cx<T> *__restrict__ buf, co
     const int tid = threadIdx.x, lane = tid & 31;
     const int team = Q <= 32 ? (tid >> 5) * LY::TPW + lane / Q : tid / Q, q = Q <= 32 ? lane % Q : tid % Q;
     const bool has_team = Q > 32 || lane < LY::TPW * Q;
-    const long long npen = (long long)g.Mx * g.My, ngrp = (npen + PB - 1) / PB;
+    // pencils, or pairs of neighbouring pencils (npen is even: every compiled length is)
+    constexpr int W = Arith<T>::W;
+    const long long npen = (long long)g.Mx * g.My / W, ngrp = (npen + PB - 1) / PB;
     const T sz = T(g.sz);
     const int Kz = g.Kz;
     double mx[4] = {0.0, 0.0, 0.0, 0.0}, nut[3] = {0.0, 0.0, 0.0};
@@ -188,9 +207,9 @@ __device__ __forceinline__ void k3_field_body(Geo g, cx<T> *__restrict__ buf, co
             const int item = team + r * NT, pl = item / NPAIR;
             const ZPair pr = zfield_pair<MODE>(item - pl * NPAIR);
             const bool ok = pl < np;
-            const cx<T> *base = buf + (p0 + (ok ? pl : 0)) * g.Kp;
+            const SCx<T> *base = buf + (p0 + (ok ? pl : 0)) * W * g.Kp;
             SmPencil<T, L, E> sm{smc + item * PITCH};
-            k3_load_pair<T, L, E>(A, base + pr.a * g.S2, pr.da, pr.b < 0 ? nullptr : base + pr.b * g.S2, pr.db, Kz, sz, q, ok);
+            k3_load_pair<T, L, E>(A, base + pr.a * g.S2, pr.da, pr.b < 0 ? nullptr : base + pr.b * g.S2, pr.db, Kz, sz, q, ok, g.Kp);
             fft<T, L, E, true, SmPencil<T, L, E>, WARP>(A, sm, q, tw);
 #pragma unroll
             for (int e = 0; e < E; e++) sm.at(out_row<L, E, true>(q, e)) = A[e];
@@ -203,7 +222,7 @@ __device__ __forceinline__ void k3_field_body(Geo g, cx<T> *__restrict__ buf, co
             cx<T> v[NPAIR];
 #pragma unroll
             for (int p = 0; p < NPAIR; p++) v[p] = b[p * PITCH];
-            zfield_row<T, MODE>(v, c, mx, nut);
+            zfield_rows<MODE>(v, c, mx, nut);
 #pragma unroll
             for (int j = 0; j < NJOB; j++) b[j * PITCH] = v[j];
         }
@@ -217,8 +236,8 @@ __device__ __forceinline__ void k3_field_body(Geo g, cx<T> *__restrict__ buf, co
             const ZJob jb = zfield_job<MODE>(idle < 0 ? j : 0);
             const bool ok = idle < 0 && pl < np;
             SmPencil<T, L, E> sm{smc + (pl * NPAIR + j) * PITCH};
-            cx<T> *base = buf + (p0 + (ok ? pl : 0)) * g.Kp;
-            cx<T> *oa = base + jb.a * g.S2, *ob = jb.b < 0 ? nullptr : base + jb.b * g.S2;
+            SCx<T> *base = buf + (p0 + (ok ? pl : 0)) * W * g.Kp;
+            SCx<T> *oa = base + jb.a * g.S2, *ob = jb.b < 0 ? nullptr : base + jb.b * g.S2;
 #pragma unroll
             for (int e = 0; e < E; e++) A[e] = sm.at(in_row<L, E, false>(q, e));
             stage_barrier<WARP>();
@@ -231,13 +250,13 @@ __device__ __forceinline__ void k3_field_body(Geo g, cx<T> *__restrict__ buf, co
                 for (int k = q; k < Kz; k += Q) {
                     const cx<T> zk = sm.at(k), zm = sm.at(k == 0 ? 0 : L - k);
                     if (jb.single) {
-                        oa[k] = zk;
+                        st_pencil(oa, k, g.Kp, zk);
                     } else {
                         cx<T> xa = mk<T>(h * (zk.x + zm.x), h * (zk.y - zm.y));
                         const cx<T> xb = mk<T>(h * (zk.y + zm.y), h * (zm.x - zk.x));
                         if (jb.fold) xa = xa + mul_i(T(k) * sz * xb);
-                        oa[k] = xa;
-                        if (ob) ob[k] = xb;
+                        st_pencil(oa, k, g.Kp, xa);
+                        if (ob) st_pencil(ob, k, g.Kp, xb);
                     }
                 }
             }
@@ -256,7 +275,7 @@ __device__ __forceinline__ void k3_field_body(Geo g, cx<T> *__restrict__ buf, co
 }
 
 template <typename T, int L, int E, int PB, int NT, int MODE, int MINB>
-__global__ void __launch_bounds__(ZFieldLayout<T, L, E, PB, NT, MODE>::THREADS, MINB) k3_field(Geo g, cx<T> *__restrict__ buf, StepConsts c, DevScalars *ds,
+__global__ void __launch_bounds__(ZFieldLayout<T, L, E, PB, NT, MODE>::THREADS, MINB) k3_field(Geo g, SCx<T> *__restrict__ buf, StepConsts c, DevScalars *ds,
                                                               double *__restrict__ nut_out, const cx<T> *__restrict__ tw) {
     k3_field_body<T, L, E, PB, NT, MODE>(g, buf, c, ds, nut_out, tw);
 }
@@ -264,7 +283,7 @@ __global__ void __launch_bounds__(ZFieldLayout<T, L, E, PB, NT, MODE>::THREADS, 
 template <typename T, int L, int E, int PB, int NT, int MODE, int MINB>
 __global__ void __launch_bounds__(ZFieldLayout<T, L, E, PB, NT, MODE>::THREADS, MINB) k3_field_batch(Geo g, const BatchMember *__restrict__ tab, const cx<T> *__restrict__ tw) {
     const BatchMember &m = tab[blockIdx.y];
-    k3_field_body<T, L, E, PB, NT, MODE>(g, static_cast<cx<T> *>(m.B2), m.c, m.ds, nullptr, tw);
+    k3_field_body<T, L, E, PB, NT, MODE>(g, static_cast<SCx<T> *>(m.B2), m.c, m.ds, nullptr, tw);
 }
 
 } // namespace spns

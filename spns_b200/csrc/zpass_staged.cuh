@@ -13,8 +13,8 @@
 //     bytes on an mbarrier), while the current pair is transformed; the first
 //     pair of the next group is fetched during the two forward transforms.  The
 //     staging takes 2*PB*Kz complex values instead of 6*PB*Kz, so more blocks fit
-//     an SM.  In single precision a group of pencils need not start on 16 bytes
-//     (Kz is odd), so there the staging uses per-lane cp.async instead.
+//     an SM.  In single precision (T = f2) a thread transforms two neighbouring pencils
+//     with packed arithmetic, so a block is the double-precision block of 2 PB pencils.
 //   * Working set per thread: four physical slots (u, v, w_x, w_y; the last
 //     SLOTS_SM of them in shared memory, own rows only) and one complex register
 //     array.  c_z
@@ -73,20 +73,21 @@ __device__ __forceinline__ bool mbar_wait_bounded(unsigned long long *bar, unsig
 
 constexpr int ZS_WAIT_LIMIT = 1 << 22;
 
-// Shared memory of one block: PB exchange buffers, 2 staging fields of PB pencils
-// (stride KS complex values per field), SLOTS_SM physical slots of L reals per
-// pencil, then the block's mbarrier.
+// Shared memory of one block: PB exchange buffers, 2 staging fields of PB * W pencils (rows
+// of the work buffers' pitch Kp, the last without its padding; W = Arith<T>::W pencils to a
+// thread), SLOTS_SM physical slots of L reals per exchange buffer, then the block's mbarrier.
 template <typename T, int L, int E, int PB, int SLOTS_SM> struct ZStagedLayout {
-    static constexpr int Q = L / E;
+    static constexpr int Q = L / E, W = Arith<T>::W;
     static constexpr int PITCH = pencil_pitch<T, L, E>();
-    static constexpr long long SLOT_ELEMS = ((long long)SLOTS_SM * PB * L * (long long)sizeof(T) + (long long)sizeof(cx<T>) - 1) / (long long)sizeof(cx<T>);
-    // staging stride of one field: PB rows of pitch Kp, the last without its padding (Kp is whole 16-byte units)
-    __host__ __device__ static int stage_stride(int Kz, int Kp) {
-        const int per16 = 16 / (int)sizeof(cx<T>);
-        return (PB - 1) * Kp + (Kz + per16 - 1) / per16 * per16;
+    // staged elements of np pencils of one field (whole 16-byte units, as Kp is)
+    __host__ __device__ static int stage_elems(int np, int Kz, int Kp) {
+        constexpr int U = 16 / (int)sizeof(SCx<T>);
+        return (np - 1) * Kp + (Kz + U - 1) / U * U;
     }
-    __host__ __device__ static long long elems(int Kz, int Kp) { return (long long)PB * PITCH + 2LL * stage_stride(Kz, Kp) + SLOT_ELEMS; }
-    __host__ __device__ static size_t smem_bytes(int Kz, int Kp) { return (size_t)elems(Kz, Kp) * sizeof(cx<T>) + 16; }
+    __host__ __device__ static size_t stage_bytes(int Kz, int Kp) { return (size_t)stage_elems(PB * W, Kz, Kp) * sizeof(SCx<T>); }
+    static constexpr size_t EXCH = (size_t)PB * PITCH * sizeof(cx<T>), SLOTS = (size_t)SLOTS_SM * PB * L * sizeof(T);
+    __host__ __device__ static size_t bar_offset(int Kz, int Kp) { return EXCH + 2 * stage_bytes(Kz, Kp) + SLOTS; }
+    __host__ __device__ static size_t smem_bytes(int Kz, int Kp) { return bar_offset(Kz, Kp) + 16; }
 };
 
 // Physical slot S (0 u, 1 v, 2 w_x, 3 w_y) of register slot e (grid row `row`):
@@ -98,66 +99,53 @@ __device__ __forceinline__ T &zs_slot(T (&rg)[NREG > 0 ? NREG : 1][E], T *sm_slo
 }
 
 template <typename T, int L, int E, int PB, int SLOTS_SM, int MINB>
-__global__ void __launch_bounds__(PB *(L / E), MINB) k3_rot_staged(Geo g, cx<T> *__restrict__ buf, StepConsts c, DevScalars *ds,
+__global__ void __launch_bounds__(PB *(L / E), MINB) k3_rot_staged(Geo g, SCx<T> *__restrict__ buf, StepConsts c, DevScalars *ds,
                                                                    const cx<T> *__restrict__ tw) {
     using LY = ZStagedLayout<T, L, E, PB, SLOTS_SM>;
     constexpr int Q = LY::Q, THREADS = PB * Q;
     static_assert(SLOTS_SM >= 0 && SLOTS_SM <= 4, "zero to four slots in shared memory");
     constexpr bool WARP = (32 % Q == 0);                      // a pencil never leaves its warp
-    constexpr bool BULK = sizeof(cx<T>) == 16;                // double: 16-byte elements, bulk copies
+    constexpr int W = LY::W;
     extern __shared__ __align__(128) unsigned char smraw_zs[];
     const int tid = threadIdx.x, sub = tid / Q, q0 = tid % Q;
     const int Kz = g.Kz;
-    const int Kp = g.Kp, KS = LY::stage_stride(Kz, Kp);
+    const int Kp = g.Kp;
     cx<T> *const smc = reinterpret_cast<cx<T> *>(smraw_zs);
     SmPencil<T, L, E> sm{smc + sub * LY::PITCH};
-    cx<T> *const stA = smc + PB * LY::PITCH;                  // staging: field a of the pair
-    cx<T> *const stB = stA + KS;                              // field b
-    T *const slot_sm = reinterpret_cast<T *>(stB + KS) + sub * L;   // slot j of this pencil at slot_sm[j*PB*L + row]
-    unsigned long long *const bar = reinterpret_cast<unsigned long long *>(smc + LY::elems(Kz, Kp));
+    SCx<T> *const stA = reinterpret_cast<SCx<T> *>(smraw_zs + LY::EXCH);                              // staging: field a of the pair
+    SCx<T> *const stB = reinterpret_cast<SCx<T> *>(smraw_zs + LY::EXCH + LY::stage_bytes(Kz, Kp));    // field b
+    T *const slot_sm = reinterpret_cast<T *>(smraw_zs + LY::EXCH + 2 * LY::stage_bytes(Kz, Kp)) + sub * L;   // slot j of this pencil at slot_sm[j*PB*L + row]
+    unsigned long long *const bar = reinterpret_cast<unsigned long long *>(smraw_zs + LY::bar_offset(Kz, Kp));
     if (tid == 0) {
         mbar_init(bar, 1);
         fence_mbar_init();
     }
     __syncthreads();
 
-    const long long npen = (long long)g.Mx * g.My;
+    // npen is even (every compiled length is), so W = 2 leaves no single pencil
+    const long long npen = (long long)g.Mx * g.My / W;
     const long long ngrp = (npen + PB - 1) / PB;
     const T sz = T(g.sz);
     unsigned parity = 0;
     bool bad = false;
     double mx[4] = {0.0, 0.0, 0.0, 0.0};
 
-    // stage fields fa, fb of pencil group grp (its valid pencils are contiguous in each field)
+    // stage fields fa, fb of group grp (its pencils' rows are contiguous in each field)
     auto issue = [&](long long grp, int fa, int fb) {
+        if (tid != 0) return;
         const long long p0 = grp * PB;
-        const int np = (int)(npen - p0 < PB ? npen - p0 : PB);
-        const cx<T> *A = buf + (long long)fa * g.S2 + p0 * Kp, *B = buf + (long long)fb * g.S2 + p0 * Kp;
-        if constexpr (BULK) {
-            if (tid == 0) {
-                const unsigned bytes = (unsigned)((KS - (PB - np) * Kp) * sizeof(cx<T>));
-                fence_proxy_async_smem();
-                mbar_arrive_expect_tx(bar, 2 * bytes);
-                bulk_copy_g2s(stA, A, bytes, bar);
-                bulk_copy_g2s(stB, B, bytes, bar);
-            }
-        } else {
-            for (int k = tid; k < KS - (PB - np) * Kp; k += THREADS) {
-                cp_async_elem<T>(stA + k, A + k);
-                cp_async_elem<T>(stB + k, B + k);
-            }
-            cp_async_commit();
-        }
+        const int np = (int)(npen - p0 < PB ? npen - p0 : PB) * W;
+        const SCx<T> *A = buf + (long long)fa * g.S2 + p0 * W * Kp, *B = buf + (long long)fb * g.S2 + p0 * W * Kp;
+        const unsigned bytes = (unsigned)(LY::stage_elems(np, Kz, Kp) * sizeof(SCx<T>));
+        fence_proxy_async_smem();
+        mbar_arrive_expect_tx(bar, 2 * bytes);
+        bulk_copy_g2s(stA, A, bytes, bar);
+        bulk_copy_g2s(stB, B, bytes, bar);
     };
     // the staged pair is complete and visible to every thread of the block
     auto wait_stage = [&]() -> bool {
-        bool ok = true;
-        if constexpr (BULK) {
-            ok = mbar_wait_bounded(bar, parity, ZS_WAIT_LIMIT);
-            parity ^= 1u;
-        } else {
-            cp_async_wait<0>();
-        }
+        const bool ok = mbar_wait_bounded(bar, parity, ZS_WAIT_LIMIT);
+        parity ^= 1u;
         return __syncthreads_and(ok ? 1 : 0) != 0;
     };
 
@@ -167,9 +155,9 @@ __global__ void __launch_bounds__(PB *(L / E), MINB) k3_rot_staged(Geo g, cx<T> 
         const int q = opaque(q0);
         const long long pen = grp * PB + sub;
         const bool ok = pen < npen;
-        cx<T> *const B0 = buf + (ok ? pen : 0) * Kp;
+        SCx<T> *const B0 = buf + (ok ? pen : 0) * W * Kp;
 #define FZ(i) (B0 + (long long)(i) * g.S2)
-        const cx<T> *sa = stA + sub * Kp, *sb = stB + sub * Kp;
+        const SCx<T> *sa = stA + sub * W * Kp, *sb = stB + sub * W * Kp;
         cx<T> A[E];
         constexpr int NREG = 4 - SLOTS_SM;
         T r_sl[NREG > 0 ? NREG : 1][E];
@@ -177,7 +165,7 @@ __global__ void __launch_bounds__(PB *(L / E), MINB) k3_rot_staged(Geo g, cx<T> 
 #define SL(j, e) zs_slot<(j), NREG, T, E>(r_sl, slot_sm, PB * L, (e), out_row<L, E, true>(q, (e)))
         // pair 0: u + i w_x
         if (!wait_stage()) { bad = true; break; }
-        k3_load_pair<T, L, E>(A, sa, false, sb, false, Kz, sz, q, ok);
+        k3_load_pair<T, L, E>(A, sa, false, sb, false, Kz, sz, q, ok, Kp);
         __syncthreads();
         issue(grp, 1, 4);
         pencil_fft<T, L, E, true, WARP>(A, sm, q, tw);
@@ -185,7 +173,7 @@ __global__ void __launch_bounds__(PB *(L / E), MINB) k3_rot_staged(Geo g, cx<T> 
         for (int e = 0; e < E; e++) { SL(0, e) = A[e].x; SL(2, e) = A[e].y; }
         // pair 1: v + i w_y; then c_z = w_x v - w_y u, transformed and written over w_x (field 3)
         if (!wait_stage()) { bad = true; break; }
-        k3_load_pair<T, L, E>(A, sa, false, sb, false, Kz, sz, q, ok);
+        k3_load_pair<T, L, E>(A, sa, false, sb, false, Kz, sz, q, ok, Kp);
         __syncthreads();
         issue(grp, 2, 5);
         pencil_fft<T, L, E, true, WARP>(A, sm, q, tw);
@@ -197,23 +185,23 @@ __global__ void __launch_bounds__(PB *(L / E), MINB) k3_rot_staged(Geo g, cx<T> 
         }
         pencil_fft<T, L, E, false, WARP>(A, sm, q, tw);
         if (ok) {
-            cx<T> *o = FZ(3);
+            SCx<T> *o = FZ(3);
 #pragma unroll
             for (int e = 0; e < E; e++) {
                 const int row = out_row<L, E, false>(q, e);
-                if (row < Kz) o[row] = A[e];
+                if (row < Kz) st_pencil(o, row, Kp, A[e]);
             }
         }
         // pair 2: w + i w_z; then (c_x, c_y) and the CFL maxima
         if (!wait_stage()) { bad = true; break; }
-        k3_load_pair<T, L, E>(A, sa, false, sb, false, Kz, sz, q, ok);
+        k3_load_pair<T, L, E>(A, sa, false, sb, false, Kz, sz, q, ok, Kp);
         __syncthreads();
         if (grp + gridDim.x < ngrp) issue(grp + gridDim.x, 0, 3);
         pencil_fft<T, L, E, true, WARP>(A, sm, q, tw);
 #pragma unroll
         for (int e = 0; e < E; e++) {
             const T ww = A[e].x, oz = A[e].y, uu = SL(0, e), vv = SL(1, e);
-            if (ok) cfl_update<T>(mx, uu, vv, ww, c);
+            if (ok) cfl_rows(mx, uu, vv, ww, c);
             A[e] = mk<T>(SL(3, e) * ww - oz * vv, oz * uu - SL(2, e) * ww);
         }
         // forward transform of c_x + i c_y and extraction of both half spectra, kz < Kz
@@ -223,11 +211,11 @@ __global__ void __launch_bounds__(PB *(L / E), MINB) k3_rot_staged(Geo g, cx<T> 
         stage_barrier<WARP>();
         if (ok) {
             const T h = T(0.5);
-            cx<T> *oa = FZ(0), *ob = FZ(1);
+            SCx<T> *oa = FZ(0), *ob = FZ(1);
             for (int k = q; k < Kz; k += Q) {
                 const cx<T> zk = sm.at(k), zm = sm.at(k == 0 ? 0 : L - k);
-                oa[k] = mk<T>(h * (zk.x + zm.x), h * (zk.y - zm.y));
-                ob[k] = mk<T>(h * (zk.y + zm.y), h * (zm.x - zk.x));
+                st_pencil(oa, k, Kp, mk<T>(h * (zk.x + zm.x), h * (zk.y - zm.y)));
+                st_pencil(ob, k, Kp, mk<T>(h * (zk.y + zm.y), h * (zm.x - zk.x)));
             }
         }
         stage_barrier<WARP>();
