@@ -105,12 +105,6 @@ template <typename T, int L, int E_, int THR> struct ShapeT {
 #ifndef SPNS_F32_Z_STAGE
 #define SPNS_F32_Z_STAGE 1
 #endif
-#ifndef SPNS_Z_E_ROT
-#define SPNS_Z_E_ROT SPNS_Z_E
-#endif
-#ifndef SPNS_F32_Z_E_ROT
-#define SPNS_F32_Z_E_ROT 12
-#endif
 template <typename T> struct ShapeSel {
     static constexpr bool D = sizeof(T) == 8;
     static constexpr int K1_E = D ? SPNS_K1_E : SPNS_F32_K1_E, K1_T = D ? SPNS_K1_T : SPNS_F32_K1_T;
@@ -118,7 +112,6 @@ template <typename T> struct ShapeSel {
     static constexpr int K5_E = D ? SPNS_K5_E : SPNS_F32_K5_E, K5_T = D ? SPNS_K5_T : SPNS_F32_K5_T;
     static constexpr int Z_E = D ? SPNS_Z_E : SPNS_F32_Z_E, Z_T = D ? SPNS_Z_THREADS : SPNS_F32_Z_T;
     static constexpr bool Z_STAGE = D ? SPNS_Z_STAGE : SPNS_F32_Z_STAGE;
-    static constexpr int Z_E_ROT = D ? SPNS_Z_E_ROT : SPNS_F32_Z_E_ROT;   // rotational/velocity z pass
 };
 template <typename T, int L> using ShapeK1 = ShapeT<T, L, ShapeSel<T>::K1_E, ShapeSel<T>::K1_T>;   // inverse x
 template <typename T, int L> using ShapeK2 = ShapeT<T, L, ShapeSel<T>::K2_E, ShapeSel<T>::K2_T>;   // inverse y (and forward y)
@@ -203,14 +196,14 @@ template <typename T, int L> struct ZStagedShape {
     static constexpr bool ON = L >= (D ? SPNS_ZS_MIN_L : SPNS_F32_ZS_MIN_L) && L <= 768 && L % E == 0 && spns::n_stages(L, E) > 0;
 };
 
-// z pass: pencils per block limited by the shared memory of the exchange
-// buffer plus the physical fields kept per pencil.
-template <typename T, int L, int MODE, int ALT = 0> struct Shape3 {
-    static constexpr int E = ALT ? SPNS_ALT_E : (MODE == spns::MODE_ROT || MODE == spns::MODE_VEL) ? ShapeSel<T>::Z_E_ROT : ShapeSel<T>::Z_E;
+// Velocity and short-length rotational z pass (k3_z): pencils per block limited by the
+// shared memory of the exchange buffers.
+template <typename T, int L, int ALT = 0> struct Shape3 {
+    static constexpr int E = ALT ? SPNS_ALT_E : ShapeSel<T>::Z_E;
     static constexpr int Q = L / E;
     static constexpr int ZT = ShapeSel<T>::Z_T / Q;
     static constexpr int P0 = ZT >= 32 ? 32 : ZT >= 16 ? 16 : ZT >= 8 ? 8 : ZT >= 4 ? 4 : ZT >= 2 ? 2 : 1;
-    static constexpr size_t PER_PEN = (size_t)spns::pencil_pitch<T, L, E>() * sizeof(spns::cx<T>) + (size_t)spns::K3Reg<T, MODE, E>::NSM * L * sizeof(T);
+    static constexpr size_t PER_PEN = (size_t)spns::pencil_pitch<T, L, E>() * sizeof(spns::cx<T>);
     static constexpr int PMAX = (int)((200 * 1024) / PER_PEN);
     static constexpr int P = P0 <= PMAX ? P0 : PMAX >= 16 ? 16 : PMAX >= 8 ? 8 : PMAX >= 4 ? 4 : PMAX >= 2 ? 2 : 1;
     static constexpr int THREADS = P * Q;

@@ -91,17 +91,17 @@ template <typename T> struct LenLaunch {
         return cudaSuccess;
     }
     template <int L, int MODE, int ALT = 0> static cudaError_t launch_k3(spns_handle *h, double *phys) {
-        if constexpr (MODE != spns::MODE_VEL && (MODE != spns::MODE_ROT || SPNS_ZF_ROT)) return launch_k3_field<L, MODE, ALT>(h, phys);
+        if constexpr (MODE != spns::MODE_VEL && MODE != spns::MODE_ROT) {
+            return launch_k3_field<L, MODE, ALT>(h, phys);
+        } else {
         if constexpr (MODE == spns::MODE_ROT && ALT == 0 && ZStagedShape<A, L>::ON) return launch_k3_staged<L>(h);
-        using S3 = Shape3<T, L, MODE, ALT>;
-        constexpr bool STAGE_ROT = MODE == spns::MODE_ROT && ShapeSel<T>::Z_STAGE;
-        constexpr bool STAGE_LES = MODE == spns::MODE_LES && sizeof(T) == 4 && SPNS_F32_Z_STAGE_LES;
-        constexpr bool STAGE = STAGE_ROT || STAGE_LES;
+        using S3 = Shape3<T, L, ALT>;
+        constexpr bool STAGE = MODE == spns::MODE_ROT && ShapeSel<T>::Z_STAGE;
         auto kern = spns::k3_z<T, L, S3::E, S3::P, MODE, STAGE>;
-        constexpr size_t stage_fields = STAGE_ROT ? 2 * spns::K3StagePairs<T>::N : STAGE_LES ? 9 : 0;
+        constexpr size_t stage_fields = STAGE ? 2 * spns::K3StagePairs<T>::N : 0;
         // the staging is sized by Kz at run time: at most L/2+1 values per field and pencil
         static_assert(S3::SMEM + (size_t)S3::P * stage_fields * (L / 2 + 1) * sizeof(C) <= 227 * 1024,
-                      "z-pass shared memory (exchange, physical slots and staging) exceeds 227 KB for this shape");
+                      "z-pass shared memory (exchange and staging) exceeds 227 KB for this shape");
         const size_t smem = S3::SMEM + (size_t)S3::P * stage_fields * h->g.Kz * sizeof(C);
         cudaError_t e = spns_set_smem(kern, smem);
         if (e != cudaSuccess) return e;
@@ -109,6 +109,7 @@ template <typename T> struct LenLaunch {
         dim3 grid((unsigned)((npen + S3::P - 1) / S3::P));
         kern<<<grid, S3::THREADS, smem, h->st>>>(h->g, (C *)h->B2, h->c, h->ds, phys, tw(h, L));
         return cudaGetLastError();
+        }
     }
     template <int L, int MODE, int ALT = 0> static cudaError_t launch_k4(spns_handle *h) {
         using S = ShapeK4A<AX<4, L>, L, MODE, ALT>;

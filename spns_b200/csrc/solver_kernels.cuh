@@ -396,50 +396,12 @@ __device__ __forceinline__ void block_max_bits(double v, unsigned long long *dst
     __syncthreads();
 }
 
-// Forward transform of the register pair z = a + i b and extraction of both
-// half spectra for kz < Kz:  Xa = (Z_k + conj Z_{L-k})/2, Xb = (Z_k - conj Z_{L-k})/(2i).
-// With jz: Xa += i kz Xb (the z-derivative of b folded into a; SGS divergence).
+// Forward transform of the register pair z = a + i b and extraction of both half spectra
+// for kz < Kz:  Xa = (Z_k + conj Z_{L-k})/2, Xb = (Z_k - conj Z_{L-k})/(2i); with `single`
+// one real field (b = 0), stored from the registers.  One copy of the transform code.
 template <typename T, int L, int E>
-__device__ __forceinline__ void k3_store_pair(cx<T> (&r)[E], SmPencil<T, L, E> sm, int q, int Kz, cx<T> *A, cx<T> *B,
-                                              bool fold_dz_b_into_a, T sz, bool ok, const cx<T> *__restrict__ tw) {
-    constexpr int Q = L / E;
-    pencil_fft<T, L, E, false, (32 % (L / E) == 0)>(r, sm, q, tw);
-#pragma unroll
-    for (int e = 0; e < E; e++) sm.at(out_row<L, E, false>(q, e)) = r[e];
-    __syncthreads();
-    if (ok) {
-        const T h = T(0.5);
-        for (int k = q; k < Kz; k += Q) {
-            cx<T> zk = sm.at(k), zm = sm.at(k == 0 ? 0 : L - k);
-            cx<T> xa = mk<T>(h * (zk.x + zm.x), h * (zk.y - zm.y));
-            cx<T> xb = mk<T>(h * (zk.y + zm.y), h * (zm.x - zk.x));
-            if (fold_dz_b_into_a) xa = xa + mul_i(T(k) * sz * xb);
-            A[k] = xa;
-            if (B) B[k] = xb;
-        }
-    }
-    __syncthreads();
-}
-
-// Single real field: forward transform of (a + 0i), kz < Kz written directly.
-template <typename T, int L, int E>
-__device__ __forceinline__ void k3_store_single(cx<T> (&r)[E], SmPencil<T, L, E> sm, int q, int Kz, cx<T> *A, bool ok,
-                                                const cx<T> *__restrict__ tw) {
-    pencil_fft<T, L, E, false, (32 % (L / E) == 0)>(r, sm, q, tw);
-    if (ok) {
-#pragma unroll
-        for (int e = 0; e < E; e++) {
-            const int row = out_row<L, E, false>(q, e);
-            if (row < Kz) A[row] = r[e];
-        }
-    }
-}
-
-// One forward job of the z pass: a pair (k3_store_pair) or, with `single`, a
-// single real field (k3_store_single), behind one copy of the transform code.
-template <typename T, int L, int E>
-__device__ __forceinline__ void k3_store_job(cx<T> (&r)[E], SmPencil<T, L, E> sm, int q, int Kz, cx<T> *A, cx<T> *B, bool fold,
-                                             bool single, T sz, bool ok, const cx<T> *__restrict__ tw) {
+__device__ __forceinline__ void k3_store_job(cx<T> (&r)[E], SmPencil<T, L, E> sm, int q, int Kz, cx<T> *A, cx<T> *B,
+                                             bool single, bool ok, const cx<T> *__restrict__ tw) {
     constexpr int Q = L / E;
     pencil_fft<T, L, E, false, (32 % (L / E) == 0)>(r, sm, q, tw);
     if (single) {
@@ -459,11 +421,8 @@ __device__ __forceinline__ void k3_store_job(cx<T> (&r)[E], SmPencil<T, L, E> sm
         const T h = T(0.5);
         for (int k = q; k < Kz; k += Q) {
             cx<T> zk = sm.at(k), zm = sm.at(k == 0 ? 0 : L - k);
-            cx<T> xa = mk<T>(h * (zk.x + zm.x), h * (zk.y - zm.y));
-            cx<T> xb = mk<T>(h * (zk.y + zm.y), h * (zm.x - zk.x));
-            if (fold) xa = xa + mul_i(T(k) * sz * xb);
-            A[k] = xa;
-            if (B) B[k] = xb;
+            A[k] = mk<T>(h * (zk.x + zm.x), h * (zk.y - zm.y));
+            B[k] = mk<T>(h * (zk.y + zm.y), h * (zm.x - zk.x));
         }
     }
     __syncthreads();
@@ -497,18 +456,6 @@ template <typename T> __device__ __forceinline__ void cp_async_elem(cx<T> *smem_
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
-// Shared-memory slots of physical fields kept per pencil (rows of this thread only).
-// slots: 0 u, 1 v, 2 w, 3..5 conv_x,y,z, LES 6..11 a11, a12, a22, a13, a23, a33 (then t_ij)
-template <int MODE> struct K3Phys { static constexpr int N = MODE == MODE_ADV ? 6 : MODE == MODE_LES ? 12 : MODE == MODE_INV ? 9 : 0; };
-// The first slots live in registers (indexed by the thread's register slot e, not
-// by row), the rest in shared memory: the twelve LES slots of a 384-pencil take
-// 37 KB of shared memory in FP64, which alone would allow 4 pencils per SM.
-#ifndef SPNS_K3_REG_SLOTS
-#define SPNS_K3_REG_SLOTS 6
-#endif
-#ifndef SPNS_F32_K3_REG_SLOTS
-#define SPNS_F32_K3_REG_SLOTS 9
-#endif
 #ifndef SPNS_Z_STAGE_PAIRS
 #define SPNS_Z_STAGE_PAIRS 3      // double rotational z pass: input pairs staged in shared memory
 #endif
@@ -516,49 +463,22 @@ template <int MODE> struct K3Phys { static constexpr int N = MODE == MODE_ADV ? 
 #define SPNS_F32_Z_STAGE_PAIRS 3
 #endif
 template <typename T> struct K3StagePairs { static constexpr int N = sizeof(T) == 8 ? SPNS_Z_STAGE_PAIRS : SPNS_F32_Z_STAGE_PAIRS; };
-#ifndef SPNS_F32_Z_STAGE_LES
-#define SPNS_F32_Z_STAGE_LES 1    // single-precision LES z pass: stage the nine input fields in shared memory
-#endif
-// Staging slot of S2 input field f (0 u, 1 v, 2 w, 3-5 d/dx, 6-8 d/dy) in the LES z pass:
-// the order of first use by the pairs, 0 1 2 3 6 4 7 5 8.
-__host__ __device__ constexpr int k3_stage_slot(int f) { return f <= 3 ? f : f == 6 ? 4 : f == 4 ? 5 : f == 7 ? 6 : f == 5 ? 7 : 8; }
-template <typename T, int MODE, int E = 12> struct K3Reg {
-    // with few values per thread (E <= 6) more slots fit in registers
-    static constexpr int R = E <= 6 ? (sizeof(T) == 8 ? 8 : 12) : sizeof(T) == 8 ? SPNS_K3_REG_SLOTS : SPNS_F32_K3_REG_SLOTS;
-    static constexpr int N = K3Phys<MODE>::N < R ? K3Phys<MODE>::N : R;   // slots in registers
-    static constexpr int NSM = K3Phys<MODE>::N - N;                       // slots in shared memory
-};
-template <int S, int NREG, int L, typename T, int E>
-__device__ __forceinline__ T &k3_slot(T (&rg)[NREG > 0 ? NREG : 1][E], T *ph, int e, int row) {
-    if constexpr (S < NREG) return rg[S][e];
-    else return ph[(S - NREG) * L + row];
-}
-
 // STAGE (rotational form): the six input fields of the block's pencils are
 // copied into shared memory asynchronously at the start, in the order the
 // three pairs use them, so the loads of the second and third pairs overlap the
 // transforms of the first.  Dynamic shared memory then holds P*6*Kz extra
 // complex values after the exchange buffers.
-// Register budget of the z pass, as registers per thread (0: none), turned into
-// the minimum resident blocks per SM of __launch_bounds__ for the block size
-// at hand: single precision 128 for the velocity and rotational forms (16 warps
-// per SM), 168 for the advective and LES forms (12 warps); double precision none.
+// Register budget of the z pass, as registers per thread (0: none), turned into the
+// minimum resident blocks per SM of __launch_bounds__ for the block size at hand: single
+// precision 128 (16 warps per SM), double precision none.
 #ifndef SPNS_K3_REGS_ROT
 #define SPNS_K3_REGS_ROT 0
-#endif
-#ifndef SPNS_K3_REGS_ADV
-#define SPNS_K3_REGS_ADV 0
 #endif
 #ifndef SPNS_F32_K3_REGS_ROT
 #define SPNS_F32_K3_REGS_ROT 128
 #endif
-#ifndef SPNS_F32_K3_REGS_ADV
-#define SPNS_F32_K3_REGS_ADV 168
-#endif
-template <typename T, int MODE, int THREADS> struct K3MinBlocks {
-    static constexpr bool D = sizeof(T) == 8;
-    static constexpr int REGS = (MODE == MODE_LES || MODE == MODE_ADV) ? (D ? SPNS_K3_REGS_ADV : SPNS_F32_K3_REGS_ADV)
-                              : (MODE == MODE_ROT || MODE == MODE_VEL) ? (D ? SPNS_K3_REGS_ROT : SPNS_F32_K3_REGS_ROT) : 0;
+template <typename T, int THREADS> struct K3MinBlocks {
+    static constexpr int REGS = sizeof(T) == 8 ? SPNS_K3_REGS_ROT : SPNS_F32_K3_REGS_ROT;
     static constexpr int B = REGS > 0 ? 65536 / (REGS * THREADS) : 1;
     static constexpr int N = B < 1 ? 1 : B;
 };
@@ -575,8 +495,6 @@ __device__ __forceinline__ void k3_z_body(Geo g, cx<T> *__restrict__ buf, const 
     cx<T> *smc = reinterpret_cast<cx<T> *>(smraw);
     constexpr int PITCH = pencil_pitch<T, L, E>();
     SmPencil<T, L, E> sm{smc + p * PITCH};
-    constexpr int NREG = K3Reg<T, MODE, E>::N;
-    T *ph = reinterpret_cast<T *>(smc + P * PITCH) + (long long)p * K3Reg<T, MODE, E>::NSM * L;
     const T sz = T(g.sz);
     cx<T> *const B0 = buf + base;
 #define F(i) (B0 + (long long)(i) * g.S2)
@@ -608,7 +526,8 @@ __device__ __forceinline__ void k3_z_body(Geo g, cx<T> *__restrict__ buf, const 
         }
         block_max4<T>(mx, ds);
         block_sum(ss, &ds->sumsq_phys);
-    } else if constexpr (MODE == MODE_ROT) {
+    } else {
+        static_assert(MODE == MODE_ROT, "the other forms run in k3_field");
         // pairs (u, w_x), (v, w_y), (w, w_z);  c = w x u  (= u.grad u + gradient)
         // STAGE: the input fields of the last NSP pairs are copied into shared memory
         // asynchronously at the start, in the order the pairs use them, so their loads
@@ -677,315 +596,8 @@ __device__ __forceinline__ void k3_z_body(Geo g, cx<T> *__restrict__ buf, const 
             }
             // c_z goes over w_x (field 3, consumed by the first pair): the forward y pass
             // reads the rotational nonlinear term from fields 0, 1 and 3 (k4_in_field)
-            k3_store_job<T, L, E>(A, sm, q, g.Kz, j == 0 ? F(0) : F(3), j == 0 ? F(1) : nullptr, false, j == 1, sz, ok, tw);
+            k3_store_job<T, L, E>(A, sm, q, g.Kz, j == 0 ? F(0) : F(3), j == 0 ? F(1) : nullptr, j == 1, ok, tw);
         }
-    } else if constexpr (MODE == MODE_INV) {
-        // Velocity-gradient invariants (src/HIT_LES.cpp:1297-1319, definitions
-        // src/tensor_algebra.cpp:165-306, 356-358) of G_ij = d_j u_i, and the
-        // eddy-viscosity statistics of the grid: `phys` holds 3 accumulators here
-        // (sum of nu_t, sum of nu_t^2, bits of the maximum nu_t).
-        // S2 inputs as in the advective form: 0 u, 1 v, 2 w, 3 du/dx, 4 dv/dx, 5 dw/dx,
-        // 6 du/dy, 7 dv/dy, 8 dw/dy; z-derivatives formed here.  Slots s = 3 i + j hold G_ij.
-        // Outputs (S2 fields 0..4): Q_G, Q_S, R_G, R_S, V^2 forward-transformed, kz <= hz.
-        double nut_sum = 0.0, nut_sq = 0.0, nut_max = 0.0;
-        cx<T> A[E];
-        T rg[NREG > 0 ? NREG : 1][E];
-#pragma unroll
-        for (int i = 0; i < (NREG > 0 ? NREG : 1); i++)
-#pragma unroll
-            for (int e = 0; e < E; e++) rg[i][e] = T(0);
-#define PH(slot, row) k3_slot<(slot), NREG, L, T, E>(rg, ph, e, row)
-        // pairs: (du/dx, du/dy), (dv/dx, dv/dy), (dw/dx, dw/dy), (du/dz, dv/dz), (dw/dz, -)
-#pragma unroll 1
-        for (int pi = 0; pi < 5; pi++) {
-            const cx<T> *fa = pi < 3 ? F(3 + pi) : pi == 3 ? F(0) : F(2);
-            const cx<T> *fb = pi < 3 ? F(6 + pi) : pi == 3 ? F(1) : nullptr;
-            k3_load_pair<T, L, E>(A, fa, pi >= 3, fb, pi == 3, g.Kz, sz, q, ok);
-            pencil_fft<T, L, E, true, (32 % (L / E) == 0)>(A, sm, q, tw);
-            switch (pi) {
-            case 0:
-#pragma unroll
-                for (int e = 0; e < E; e++) { const int row = out_row<L, E, true>(q, e); PH(0, row) = A[e].x; PH(1, row) = A[e].y; }
-                break;
-            case 1:
-#pragma unroll
-                for (int e = 0; e < E; e++) { const int row = out_row<L, E, true>(q, e); PH(3, row) = A[e].x; PH(4, row) = A[e].y; }
-                break;
-            case 2:
-#pragma unroll
-                for (int e = 0; e < E; e++) { const int row = out_row<L, E, true>(q, e); PH(6, row) = A[e].x; PH(7, row) = A[e].y; }
-                break;
-            case 3:
-#pragma unroll
-                for (int e = 0; e < E; e++) { const int row = out_row<L, E, true>(q, e); PH(2, row) = A[e].x; PH(5, row) = A[e].y; }
-                break;
-            default:
-#pragma unroll
-                for (int e = 0; e < E; e++) { const int row = out_row<L, E, true>(q, e); PH(8, row) = A[e].x; }
-                break;
-            }
-        }
-        // invariants per grid row, written over slots 0..4
-#pragma unroll
-        for (int e = 0; e < E; e++) {
-            const int row = out_row<L, E, true>(q, e);
-            double G[3][3], S[3][3], O[3][3], S2[3][3], O2[3][3];
-            G[0][0] = PH(0, row); G[0][1] = PH(1, row); G[0][2] = PH(2, row);
-            G[1][0] = PH(3, row); G[1][1] = PH(4, row); G[1][2] = PH(5, row);
-            G[2][0] = PH(6, row); G[2][1] = PH(7, row); G[2][2] = PH(8, row);
-#pragma unroll
-            for (int i = 0; i < 3; i++)
-#pragma unroll
-                for (int j = 0; j < 3; j++) { S[i][j] = 0.5 * G[i][j] + 0.5 * G[j][i]; O[i][j] = G[i][j] - S[i][j]; }
-            double trG = G[0][0] + G[1][1] + G[2][2], trS = S[0][0] + S[1][1] + S[2][2], trGG = 0.0, trSS = 0.0, trS2O2 = 0.0;
-#pragma unroll
-            for (int i = 0; i < 3; i++)
-#pragma unroll
-                for (int j = 0; j < 3; j++) {
-                    trGG += G[i][j] * G[j][i];
-                    trSS += S[i][j] * S[j][i];
-                    double s2 = 0.0, o2 = 0.0;
-#pragma unroll
-                    for (int k = 0; k < 3; k++) { s2 += S[i][k] * S[k][j]; o2 += O[i][k] * O[k][j]; }
-                    S2[i][j] = s2; O2[i][j] = o2;
-                }
-#pragma unroll
-            for (int i = 0; i < 3; i++)
-#pragma unroll
-                for (int k = 0; k < 3; k++) trS2O2 += S2[i][k] * O2[k][i];
-            auto det3 = [](const double (&t)[3][3]) {
-                double d = 0.0;
-                d += t[0][0] * t[1][1] * t[2][2];
-                d += t[0][1] * t[1][2] * t[2][0];
-                d += t[0][2] * t[1][0] * t[2][1];
-                d -= t[0][2] * t[1][1] * t[2][0];
-                d -= t[0][1] * t[1][0] * t[2][2];
-                d -= t[0][0] * t[1][2] * t[2][1];
-                return d;
-            };
-            const double QG = 0.5 * (trG * trG - trGG), QS = 0.5 * (trS * trS - trSS);
-            // eddy viscosity of this grid point (src/HIT_LES.cpp:130-142, same expression order)
-            {
-                double ne = 2.0 * G[0][0] * G[0][0];
-                ne += 2.0 * G[1][1] * G[1][1];
-                ne += 2.0 * G[2][2] * G[2][2];
-                ne += (G[0][1] + G[1][0]) * (G[0][1] + G[1][0]);
-                ne += (G[0][2] + G[2][0]) * (G[0][2] + G[2][0]);
-                ne += (G[1][2] + G[2][1]) * (G[1][2] + G[2][1]);
-                const double nt = ok ? c.les_ct * sqrt(ne) : 0.0;
-                nut_sum += nt; nut_sq += nt * nt; nut_max = fmax(nut_max, nt);
-            }
-            PH(0, row) = T(QG);
-            PH(1, row) = T(QS);
-            PH(2, row) = T(det3(G));
-            PH(3, row) = T(det3(S));
-            PH(4, row) = T(4.0 * (trS2O2 - 2.0 * QS * (QG - QS)));
-        }
-        if (phys) {
-            block_sum(nut_sum, phys);
-            block_sum(nut_sq, phys + 1);
-            block_max_bits(nut_max, reinterpret_cast<unsigned long long *>(phys + 2));
-        }
-#pragma unroll 1
-        for (int j = 0; j < 3; j++) {
-            if (j == 0) {
-#pragma unroll
-                for (int e = 0; e < E; e++) { const int row = out_row<L, E, true>(q, e); A[e] = mk<T>(PH(0, row), PH(1, row)); }
-            } else if (j == 1) {
-#pragma unroll
-                for (int e = 0; e < E; e++) { const int row = out_row<L, E, true>(q, e); A[e] = mk<T>(PH(2, row), PH(3, row)); }
-            } else {
-#pragma unroll
-                for (int e = 0; e < E; e++) { const int row = out_row<L, E, true>(q, e); A[e] = mk<T>(PH(4, row), T(0)); }
-            }
-            k3_store_job<T, L, E>(A, sm, q, g.Kz, F(2 * j), j < 2 ? F(2 * j + 1) : nullptr, false, j == 2, sz, ok, tw);
-        }
-        (void)mx;
-#undef PH
-    } else {
-        // Advective form of the reference (src/HIT_LES.cpp:74-125): conv_i = u_j d_j u_i.
-        // S2 inputs: 0 u, 1 v, 2 w, 3 du/dx, 4 dv/dx, 5 dw/dx, 6 du/dy, 7 dv/dy, 8 dw/dy;
-        // z-derivatives are formed here from u, v, w.  Physical values of the
-        // thread's own rows are kept in per-thread slots, the first K3Reg::N in
-        // registers and the rest in shared memory (own rows only: no barrier needed).
-        // LES (src/HIT_LES.cpp:130-171): strain combinations a_ij accumulate in further slots.
-        // The transforms run in two loops (inverse pairs, forward jobs) around one
-        // copy of the transform code each: unrolled one after another, the eleven
-        // LES transforms overflow the instruction cache.
-        cx<T> A[E];
-        T rg[NREG > 0 ? NREG : 1][E];
-        // slots are written in one iteration of the pair loop and read in later ones:
-        // define them on entry (a rolled loop over partly defined registers miscompiled)
-#pragma unroll
-        for (int i = 0; i < (NREG > 0 ? NREG : 1); i++)
-#pragma unroll
-            for (int e = 0; e < E; e++) rg[i][e] = T(0);
-#define PH(slot, row) k3_slot<(slot), NREG, L, T, E>(rg, ph, e, row)
-        // inverse pairs: (u, v), (w, du/dz), (du/dx, du/dy), (dv/dx, dv/dy), (dw/dx, dw/dy), (dv/dz, dw/dz)
-        // STAGE (single-precision LES): the nine input fields of the block's pencils are
-        // copied into shared memory asynchronously at the start, in five groups in the
-        // order the pairs first use them ({u, v}, {w}, {du/dx, du/dy}, {dv/dx, dv/dy},
-        // {dw/dx, dw/dy}), so later pairs' loads overlap the earlier transforms.
-        // Field f sits in staging slot K3StageSlot(f) of its pencil.
-        cx<T> *const st = reinterpret_cast<cx<T> *>(reinterpret_cast<T *>(smc + P * PITCH) +
-                                                    (long long)P * K3Reg<T, MODE, E>::NSM * L) + (long long)p * 9 * g.Kz;
-        if constexpr (STAGE) {
-#pragma unroll
-            for (int grp = 0; grp < 5; grp++) {
-#pragma unroll
-                for (int h2 = 0; h2 < 2; h2++) {
-                    const int f = grp == 0 ? h2 : grp == 1 ? (h2 == 0 ? 2 : -1) : (h2 == 0 ? grp + 1 : grp + 4);
-                    if (f >= 0 && ok)
-                        for (int k = q; k < g.Kz; k += Q) cp_async_elem<T>(st + k3_stage_slot(f) * g.Kz + k, F(f) + k);
-                }
-                cp_async_commit();
-            }
-        }
-#pragma unroll 1
-        for (int pi = 0; pi < 6; pi++) {
-            const int fa = pi == 0 ? 0 : pi == 1 ? 2 : pi == 5 ? 1 : pi + 1;
-            const int fb = pi == 0 ? 1 : pi == 1 ? 0 : pi == 5 ? 2 : pi + 4;
-            if constexpr (STAGE) {
-                switch (pi) {
-                case 0: cp_async_wait<4>(); break;
-                case 1: cp_async_wait<3>(); break;
-                case 2: cp_async_wait<2>(); break;
-                case 3: cp_async_wait<1>(); break;
-                default: cp_async_wait<0>(); break;
-                }
-                __syncthreads();
-                k3_load_pair<T, L, E>(A, st + k3_stage_slot(fa) * g.Kz, pi == 5, st + k3_stage_slot(fb) * g.Kz, pi == 1 || pi == 5,
-                                      g.Kz, sz, q, ok);
-            } else {
-                k3_load_pair<T, L, E>(A, F(fa), pi == 5, F(fb), pi == 1 || pi == 5, g.Kz, sz, q, ok);
-            }
-            pencil_fft<T, L, E, true, (32 % (L / E) == 0)>(A, sm, q, tw);
-            switch (pi) {
-            case 0:
-#pragma unroll
-                for (int e = 0; e < E; e++) { const int row = out_row<L, E, true>(q, e); PH(0, row) = A[e].x; PH(1, row) = A[e].y; }
-                break;
-            case 1:
-#pragma unroll
-                for (int e = 0; e < E; e++) {
-                    const int row = out_row<L, E, true>(q, e);
-                    const T ww = A[e].x;
-                    PH(2, row) = ww;
-                    cfl_update<T>(mx, PH(0, row), PH(1, row), ww, c);
-                    PH(3, row) = ww * A[e].y;
-                    if (MODE == MODE_LES) PH(9, row) = A[e].y; // a13 = du/dz (+ dw/dx below)
-                }
-                break;
-            case 2:
-#pragma unroll
-                for (int e = 0; e < E; e++) {
-                    const int row = out_row<L, E, true>(q, e);
-                    PH(3, row) = PH(0, row) * A[e].x + PH(1, row) * A[e].y + PH(3, row);
-                    if (MODE == MODE_LES) { PH(6, row) = A[e].x; PH(7, row) = A[e].y; } // a11, a12 (partial)
-                }
-                break;
-            case 3:
-#pragma unroll
-                for (int e = 0; e < E; e++) {
-                    const int row = out_row<L, E, true>(q, e);
-                    PH(4, row) = PH(0, row) * A[e].x + PH(1, row) * A[e].y;
-                    if (MODE == MODE_LES) { PH(7, row) = PH(7, row) + A[e].x; PH(8, row) = A[e].y; } // a12, a22
-                }
-                break;
-            case 4:
-#pragma unroll
-                for (int e = 0; e < E; e++) {
-                    const int row = out_row<L, E, true>(q, e);
-                    PH(5, row) = PH(0, row) * A[e].x + PH(1, row) * A[e].y;
-                    if (MODE == MODE_LES) { PH(9, row) = PH(9, row) + A[e].x; PH(10, row) = A[e].y; } // a13, a23 (partial)
-                }
-                break;
-            default:
-#pragma unroll
-                for (int e = 0; e < E; e++) {
-                    const int row = out_row<L, E, true>(q, e);
-                    const T ww = PH(2, row);
-                    PH(4, row) = PH(4, row) + ww * A[e].x;
-                    PH(5, row) = PH(5, row) + ww * A[e].y;
-                    if (MODE == MODE_LES) { PH(10, row) = PH(10, row) + A[e].x; PH(11, row) = A[e].y; } // a23, a33
-                }
-                break;
-            }
-        }
-        if (!ok) { mx[0] = mx[1] = mx[2] = mx[3] = 0.0; }
-        block_max4<T>(mx, ds);
-        if constexpr (MODE == MODE_LES) {
-            // eddy viscosity and SGS stress (src/HIT_LES.cpp:130-154), written over the a_ij slots:
-            // slot 6 t11, 7 t12, 8 t22, 9 t13, 10 t23, 11 t33
-            const T ct = T(c.les_ct);
-#pragma unroll
-            for (int e = 0; e < E; e++) {
-                const int row = out_row<L, E, true>(q, e);
-                const T a11 = PH(6, row), a12 = PH(7, row), a22 = PH(8, row), a13 = PH(9, row), a23 = PH(10, row), a33 = PH(11, row);
-                T ne = T(2.0) * a11 * a11;
-                ne += T(2.0) * a22 * a22;
-                ne += T(2.0) * a33 * a33;
-                ne += a12 * a12;
-                ne += a13 * a13;
-                ne += a23 * a23;
-                ne = ct * sqrt(ne);
-                PH(6, row) = T(-2.0) * ne * a11;
-                PH(7, row) = T(-1.0) * ne * a12;
-                PH(8, row) = T(-2.0) * ne * a22;
-                PH(9, row) = T(-1.0) * ne * a13;
-                PH(10, row) = T(-1.0) * ne * a23;
-                PH(11, row) = T(-2.0) * ne * a33;
-            }
-        }
-        // forward jobs.  ADV: (conv_x, conv_y) -> 0, 1; conv_z -> 2.
-        // LES outputs: 0 G_x = conv_x + i kz t13, 1 G_y, 2 G_z, 3 t11, 4 t12, 5 t13, 6 t22, 7 t23
-        constexpr int NJOB = MODE == MODE_LES ? 5 : 2;
-#pragma unroll 1
-        for (int j = 0; j < NJOB; j++) {
-            cx<T> *oa, *ob = nullptr;
-            bool fold = false, single = false;
-            if (MODE == MODE_ADV) {
-                if (j == 0) {
-#pragma unroll
-                    for (int e = 0; e < E; e++) { const int row = out_row<L, E, true>(q, e); A[e] = mk<T>(PH(3, row), PH(4, row)); }
-                    oa = F(0); ob = F(1);
-                } else {
-#pragma unroll
-                    for (int e = 0; e < E; e++) { const int row = out_row<L, E, true>(q, e); A[e] = mk<T>(PH(5, row), T(0)); }
-                    oa = F(2); single = true;
-                }
-            } else {
-                switch (j) {
-                case 0:
-#pragma unroll
-                    for (int e = 0; e < E; e++) { const int row = out_row<L, E, true>(q, e); A[e] = mk<T>(PH(3, row), PH(9, row)); }
-                    oa = F(0); ob = F(5); fold = true;
-                    break;
-                case 1:
-#pragma unroll
-                    for (int e = 0; e < E; e++) { const int row = out_row<L, E, true>(q, e); A[e] = mk<T>(PH(4, row), PH(10, row)); }
-                    oa = F(1); ob = F(7); fold = true;
-                    break;
-                case 2:
-#pragma unroll
-                    for (int e = 0; e < E; e++) { const int row = out_row<L, E, true>(q, e); A[e] = mk<T>(PH(5, row), PH(11, row)); }
-                    oa = F(2); fold = true;
-                    break;
-                case 3:
-#pragma unroll
-                    for (int e = 0; e < E; e++) { const int row = out_row<L, E, true>(q, e); A[e] = mk<T>(PH(6, row), PH(7, row)); }
-                    oa = F(3); ob = F(4);
-                    break;
-                default:
-#pragma unroll
-                    for (int e = 0; e < E; e++) { const int row = out_row<L, E, true>(q, e); A[e] = mk<T>(PH(8, row), T(0)); }
-                    oa = F(6); single = true;
-                    break;
-                }
-            }
-            k3_store_job<T, L, E>(A, sm, q, g.Kz, oa, ob, fold, single, sz, ok, tw);
-        }
-#undef PH
     }
 #undef F
 }
@@ -1696,7 +1308,7 @@ __global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 2, MODE>::N) k2_i
     k2_inv_y_body<T, L, E, P, MODE>(g, in, out, tw, blockIdx.z, gridDim.z);
 }
 template <typename T, int L, int E, int P, int MODE, bool STAGE = false>
-__global__ void __launch_bounds__(P *(L / E), K3MinBlocks<T, MODE, P *(L / E)>::N) k3_z(Geo g, cx<T> *__restrict__ buf, StepConsts c,
+__global__ void __launch_bounds__(P *(L / E), K3MinBlocks<T, P *(L / E)>::N) k3_z(Geo g, cx<T> *__restrict__ buf, StepConsts c,
                                                                                         DevScalars *ds, double *__restrict__ phys,
                                                                                         const cx<T> *__restrict__ tw) {
     k3_z_body<T, L, E, P, MODE, STAGE>(g, buf, c, ds, phys, tw);
@@ -1738,12 +1350,6 @@ __global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 2, MODE>::N) k2_i
                                                                                  const cx<T> *__restrict__ tw) {
     const BatchMember &m = tab[blockIdx.z];
     k2_inv_y_body<T, L, E, P, MODE>(g, static_cast<const SCx<T> *>(m.B1), static_cast<SCx<T> *>(m.B2), tw, 0, 1);
-}
-template <typename T, int L, int E, int P, int MODE, bool STAGE = false>
-__global__ void __launch_bounds__(P *(L / E), K3MinBlocks<T, MODE, P *(L / E)>::N) k3_z_batch(Geo g, const BatchMember *__restrict__ tab,
-                                                                                              const cx<T> *__restrict__ tw) {
-    const BatchMember &m = tab[blockIdx.z];
-    k3_z_body<T, L, E, P, MODE, STAGE>(g, static_cast<cx<T> *>(m.B2), m.c, m.ds, nullptr, tw);
 }
 template <typename T, int L, int E, int P, int MODE>
 __global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 4, MODE>::N) k4_fwd_y_batch(Geo g, const BatchMember *__restrict__ tab,
