@@ -1231,7 +1231,15 @@ struct spns_ensemble {
     bool grouped = false;
     std::vector<EnsembleClass> classes;             // batched classes (two members or more)
     std::vector<int> single;                        // members stepped on their own branch
+    // status of the members after a call, gathered by one kernel and read by one copy
+    DevScalars **ds_list = nullptr;
+    int *status = nullptr;
 };
+// One status word per member: nonzero where check_flags has something to report.
+static __global__ void k_gather_status(DevScalars *const *list, int n, int *status) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) status[i] = list[i]->nonfinite | list[i]->domain_err | list[i]->wait_timeout;
+}
 
 static bool batchable(const spns_handle *h) {
     return h->slab_ranks == 0 && !h->a.isSelfAdaptive && !(h->a.eps_forcing > 0.0) && (h->a.isLES || h->a.nonlinear_form == 2) &&
@@ -1284,6 +1292,8 @@ static void ensemble_free(spns_ensemble *e) {
     for (auto &kv : e->graphs) cudaGraphExecDestroy(kv.second);
     for (auto ev : e->join) if (ev) cudaEventDestroy(ev);
     if (e->fork) cudaEventDestroy(e->fork);
+    if (e->ds_list) cudaFreeAsync(e->ds_list, e->st);
+    if (e->status) cudaFreeAsync(e->status, e->st);
     if (e->st) cudaStreamDestroy(e->st);
     delete e;
 }
@@ -1316,6 +1326,14 @@ extern "C" int spns_ensemble_create(spns_handle *const *members, int n, spns_ens
     bool ok = cudaSetDevice(dev) == cudaSuccess && cudaStreamCreateWithFlags(&e->st, cudaStreamNonBlocking) == cudaSuccess &&
               cudaEventCreateWithFlags(&e->fork, cudaEventDisableTiming) == cudaSuccess;
     for (int i = 0; ok && i < n; i++) ok = cudaEventCreateWithFlags(&e->join[i], cudaEventDisableTiming) == cudaSuccess;
+    if (ok) {
+        std::vector<DevScalars *> list(n);
+        for (int i = 0; i < n; i++) list[i] = members[i]->ds;
+        ok = cudaMallocAsync((void **)&e->ds_list, sizeof(DevScalars *) * n, e->st) == cudaSuccess &&
+             cudaMallocAsync((void **)&e->status, sizeof(int) * n, e->st) == cudaSuccess &&
+             cudaMemcpyAsync(e->ds_list, list.data(), sizeof(DevScalars *) * n, cudaMemcpyHostToDevice, e->st) == cudaSuccess &&
+             cudaStreamSynchronize(e->st) == cudaSuccess;
+    }
     if (!ok) { ensemble_free(e); return spns_fail(nullptr, SPNS_ERR_CUDA, "ensemble stream/event creation failed"); }
     *out = e;
     return SPNS_OK;
@@ -1354,8 +1372,10 @@ extern "C" int spns_ensemble_step(spns_ensemble *e, int nsteps) {
     if (!e || nsteps < 0) return SPNS_ERR_INVALID_ARGUMENT;
     ECK(cudaSetDevice(e->device));
     const int n = (int)e->m.size();
-    // order the ensemble's stream after the members' earlier work
+    // order the ensemble's stream after the members' earlier work, where there is any
     for (int i = 0; i < n; i++) {
+        if (cudaStreamQuery(e->m[i]->st) == cudaSuccess) continue;
+        cudaGetLastError();   // not ready is no error
         ECK(cudaEventRecord(e->join[i], e->m[i]->st));
         ECK(cudaStreamWaitEvent(e->st, e->join[i], 0));
     }
@@ -1427,11 +1447,16 @@ extern "C" int spns_ensemble_step(spns_ensemble *e, int nsteps) {
         for (auto *h : e->m)
             if (h->a.isSelfAdaptive) { std::swap(h->U, h->Up); std::swap(h->Ulo, h->Uplo); }
     }
-    // order the members' later work after the ensemble's, then check every member
-    ECK(cudaEventRecord(e->fork, e->st));
-    for (auto *h : e->m) ECK(cudaStreamWaitEvent(h->st, e->fork, 0));
+    // Every member's status by one kernel and one copy (a copy and a synchronisation for each
+    // of 64 members took 0.7 ms of an 8 ms step).  The synchronisation also orders the
+    // members' later work after the ensemble's.
+    k_gather_status<<<(n + 127) / 128, 128, 0, e->st>>>(e->ds_list, n, e->status);
+    ECK(cudaGetLastError());
+    std::vector<int> status(n);
+    ECK(cudaMemcpyAsync(status.data(), e->status, sizeof(int) * n, cudaMemcpyDeviceToHost, e->st));
     ECK(cudaStreamSynchronize(e->st));
     for (int i = 0; i < n; i++) {
+        if (!status[i]) continue;
         int r = check_flags(e->m[i]);
         if (r) { e->err = "member " + std::to_string(i) + ": " + e->m[i]->err; return r; }
     }
