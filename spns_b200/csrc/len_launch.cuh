@@ -37,7 +37,8 @@ template <typename T> struct LenLaunch {
         cudaError_t e = spns_set_smem(kern, smem);
         if (e != cudaSuccess) return e;
         const dim3 grid = axis_grid<AX<1, L>>(h, S::P, h->g.Ky, spns::Fields<MODE>::K1);
-        kern<<<grid, S::THREADS, smem, h->st>>>(h->g, U(h, 0), U(h, 1), U(h, 2), (C *)h->B1, twx<1, L>(h));
+        kern<<<grid, S::THREADS, smem, h->st>>>(h->g, U(h, 0), U(h, 1), U(h, 2), (C *)h->B1, twx<1, L>(h),
+             MODE == spns::MODE_INV ? nullptr : h->ds);
         return cudaGetLastError();
     }
     template <int L, int MODE, int ALT = 0> static cudaError_t launch_k2(spns_handle *h) {

@@ -45,8 +45,6 @@ template <typename T> struct Passes {
     // Inverse transform of the velocity only (Recalculate_Velocity_Antitransform):
     // refreshes the CFL maxima and, if phys != NULL, writes u,v,w on the grid.
     static int run_velocity(spns_handle *h, double *phys) {
-        spns::k_reset_max<<<1, 1, 0, h->st>>>(h->ds);
-        CKL();
         for (int k = 1; k <= 3; k++) LAUNCH(pass(h, k, spns::MODE_VEL, false, phys));
         return SPNS_OK;
     }
@@ -239,9 +237,6 @@ template <typename T> struct Passes {
         LAUNCH(pass(h, 1, mode, true));
         MARK("k2_inv_y");
         LAUNCH(pass(h, 2, mode, true));
-        MARK("reset_max");
-        spns::k_reset_max<<<1, 1, 0, h->st>>>(h->ds);
-        CKL();
         MARK("k3_z");
         LAUNCH(pass(h, 3, mode, true));
         MARK("k4_fwd_y");
@@ -262,7 +257,7 @@ template <typename T> struct Passes {
         MARK(nullptr);
         if (prof) { if (h->prof_steps == 0) h->prof_nk = slot - 1; h->prof_steps++; }
         if (edge) nk += h->edge_launches;             // build, 2+2 line FFTs, square, apply per group
-        h->kernels_per_step = nk + 8;
+        h->kernels_per_step = nk + 7;
         return SPNS_OK;
 #undef MARK
     }
@@ -324,8 +319,6 @@ template <typename T> struct Passes {
         case SPNS_SLAB_VEL_B:
             LAUNCH(slab_pack(h, h->B1x, h->XR, 3, Ky, nx, fwd_unpack3, 1, 1));
             r = xpasses([&]() -> int {
-                spns::k_reset_max<<<1, 1, 0, h->st>>>(h->ds);
-                CKL();
                 LAUNCH(pass(h, 2, spns::MODE_VEL, false));
                 LAUNCH(pass(h, 3, spns::MODE_VEL, false));
                 return SPNS_OK;
@@ -352,8 +345,6 @@ template <typename T> struct Passes {
             }
             r = xpasses([&]() -> int {
                 LAUNCH(pass(h, 2, mode, false));
-                spns::k_reset_max<<<1, 1, 0, h->st>>>(h->ds);
-                CKL();
                 LAUNCH(pass(h, 3, mode, false));
                 LAUNCH(pass(h, 4, mode, false));
                 return SPNS_OK;
@@ -378,8 +369,6 @@ template <typename T> struct Passes {
     // Adams-Bashforth scheme without constant-power forcing or edge correction.
     static int batch_step(spns_handle *h, const spns::BatchMember *tab, int n, cudaStream_t st) {
         const int mode = h->a.isLES ? spns::MODE_LES : spns::MODE_ADV;
-        spns::k_reset_max_batch<<<n, 1, 0, st>>>(tab);
-        CKL();
         for (int k = 1; k <= 5; k++) LAUNCH(spns_len_table<T>(pass_length(h, k))->batch(h, tab, n, st, k, mode));
         {
             const int nk = h->g.Kx * h->g.Kz;

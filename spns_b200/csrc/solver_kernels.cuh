@@ -122,6 +122,16 @@ template <int MODE> struct Fields {
     static constexpr int NOUT = MODE == MODE_INV ? 5 : 3;                       // compact outputs of the forward x pass
 };
 
+// Start of a step: the maxima of the grid velocity and its squared sum begin at zero (they
+// are gathered by the z pass; the first kernel of a step resets them, after the last step's
+// end has used them and long before this step's z pass).
+__device__ __forceinline__ void reset_maxima(DevScalars *ds) {
+    if (ds && (blockIdx.x | blockIdx.y) == 0 && threadIdx.x == 0) {
+        for (int i = 0; i < 4; i++) ds->max_bits[i] = 0ull;
+        ds->sumsq_phys = 0.0;
+    }
+}
+
 // ===========================================================================
 // Elements of the x/y passes.  A thread transforms one kz column, or in single precision
 // (T = f2) two adjacent ones, which are 16 bytes of a row: the same tiles, shared-memory
@@ -866,11 +876,6 @@ static __global__ void k_finish_step(StepConsts c, DevScalars *ds) {
     ds->iter += 1;
 }
 
-static __global__ void k_reset_max(DevScalars *ds) {
-    for (int i = 0; i < 4; i++) ds->max_bits[i] = 0ull;
-    ds->sumsq_phys = 0.0;
-}
-
 // Shell sums of the spectral state (src/HIT_LES.cpp:1137-1214 with the
 // KineticEnergy and Enstrophy integrands of :991-1003).  Modes with kz>0 carry
 // their conjugate (weight 2).  Ek[K], Om[K] for K=round(|k|) <= Kmax.
@@ -1299,7 +1304,8 @@ static __global__ void k_dft_axis(const double2 *__restrict__ in, double2 *__res
 template <typename T, int L, int E, int P, int MODE>
 __global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 1, MODE>::N) k1_inv_x(Geo g, const SCx<T> *__restrict__ u, const SCx<T> *__restrict__ v,
                                                                            const SCx<T> *__restrict__ w, SCx<T> *__restrict__ out,
-                                                                           const cx<T> *__restrict__ tw) {
+                                                                           const cx<T> *__restrict__ tw, DevScalars *reset) {
+    if (blockIdx.z == 0) reset_maxima(reset);
     k1_inv_x_body<T, L, E, P, MODE>(g, u, v, w, out, tw, blockIdx.z, gridDim.z);
 }
 template <typename T, int L, int E, int P, int MODE>
@@ -1342,6 +1348,7 @@ template <typename T, int L, int E, int P, int MODE>
 __global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 1, MODE>::N) k1_inv_x_batch(Geo g, const BatchMember *__restrict__ tab,
                                                                                  const cx<T> *__restrict__ tw) {
     const BatchMember &m = tab[blockIdx.z];
+    reset_maxima(m.ds);
     const SCx<T> *U = static_cast<const SCx<T> *>(m.U);
     k1_inv_x_body<T, L, E, P, MODE>(g, U, U + g.S0, U + 2 * g.S0, static_cast<SCx<T> *>(m.B1), tw, 0, 1);
 }
@@ -1369,11 +1376,6 @@ __global__ void __launch_bounds__(256) k6_sweep_batch(Geo g, const BatchMember *
     const BatchMember &m = tab[blockIdx.z];
     cx<T> *U = static_cast<cx<T> *>(m.U), *Ulo = static_cast<cx<T> *>(m.Ulo);
     k6_sweep_body<T, false>(g, static_cast<const cx<T> *>(m.B2), U, Ulo, static_cast<cx<T> *>(m.R), U, Ulo, nullptr, nullptr, m.c, m.ds);
-}
-static __global__ void k_reset_max_batch(const BatchMember *__restrict__ tab) {
-    DevScalars *ds = tab[blockIdx.x].ds;
-    for (int i = 0; i < 4; i++) ds->max_bits[i] = 0ull;
-    ds->sumsq_phys = 0.0;
 }
 static __global__ void k_finish_step_batch(const BatchMember *__restrict__ tab) {
     const BatchMember &m = tab[blockIdx.x];
