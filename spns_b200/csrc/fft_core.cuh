@@ -3,7 +3,9 @@
 // One pencil of length L is processed by Q = L/E threads, each holding E
 // complex values in registers.  A stage of radix R performs E/R butterflies
 // per thread; between stages the values are exchanged through shared memory
-// (one buffer, two barriers per stage; warp barriers when a pencil lives in
+// (one buffer, two barriers per stage: before the writes, so that the threads of
+// a pencil may drift over a stage's arithmetic, and between writes and reads; the
+// last reads of a transform are not followed by one; warp barriers when a pencil lives in
 // one warp).  The first stage reads its inputs from registers filled by the
 // caller at rows  j + r*(L/R_first)  and the last stage leaves its outputs in
 // registers at rows  j + r*(L/R_last)  (j = q + Q*m), so callers load pencils
@@ -327,6 +329,9 @@ __device__ __forceinline__ void fft_run(cx<T> (&v)[E], SM sm, int q, const cx<T>
     if constexpr (S + 1 < PL::NST) {
         constexpr int R2 = PL::radix(S + 1);
         constexpr int MB2 = E / R2;
+        // every reader of the buffer's last contents is done (waited for here, after this
+        // stage's arithmetic, rather than right after the reads)
+        stage_barrier<WARP>();
         if constexpr (ex_pad<SM, INV, S>() < 0) {
             // XOR-swizzled layout (fewer bank conflicts for this exchange)
 #pragma unroll
@@ -343,7 +348,6 @@ __device__ __forceinline__ void fft_run(cx<T> (&v)[E], SM sm, int q, const cx<T>
 #pragma unroll
                 for (int r = 0; r < R2; r++) v[m * R2 + r] = sm.xr(j + r * (L / R2));
             }
-            stage_barrier<WARP>();
         } else if constexpr (SmPadded<SM>::value) {
             // padded layout: one base address per butterfly group, offsets in the instructions
             constexpr int X = Ns * R, PAD = SM::template Ex<INV, S>::PAD, XP = X + PAD;
@@ -375,7 +379,6 @@ __device__ __forceinline__ void fft_run(cx<T> (&v)[E], SM sm, int q, const cx<T>
 #pragma unroll
                 for (int r = 0; r < R2; r++) v[m * R2 + r] = rd[r * PSTEP];
             }
-            stage_barrier<WARP>();
         } else {
 #pragma unroll
             for (int m = 0; m < MB; m++) {
@@ -391,7 +394,6 @@ __device__ __forceinline__ void fft_run(cx<T> (&v)[E], SM sm, int q, const cx<T>
 #pragma unroll
                 for (int r = 0; r < R2; r++) v[m * R2 + r] = sm.at(j + r * (L / R2));
             }
-            stage_barrier<WARP>();
         }
         fft_run<T, L, E, INV, WARP, S + 1, SM>(v, sm, q, tw);
     }

@@ -26,7 +26,7 @@
 // divergence is folded into the forward passes (i kz t_i3 in K3, i ky t_i2 in
 // K4, i kx t_i1 in K5).
 #pragma once
-#include "fft768.cuh"
+#include "fft_core.cuh"
 
 namespace spns {
 
@@ -413,7 +413,7 @@ template <typename T, int L, int E>
 __device__ __forceinline__ void k3_store_job(cx<T> (&r)[E], SmPencil<T, L, E> sm, int q, int Kz, cx<T> *A, cx<T> *B,
                                              bool single, bool ok, const cx<T> *__restrict__ tw) {
     constexpr int Q = L / E;
-    pencil_fft<T, L, E, false, (32 % (L / E) == 0)>(r, sm, q, tw);
+    fft<T, L, E, false, SmPencil<T, L, E>, (32 % (L / E) == 0)>(r, sm, q, tw);
     if (single) {
         if (ok) {
 #pragma unroll
@@ -424,6 +424,7 @@ __device__ __forceinline__ void k3_store_job(cx<T> (&r)[E], SmPencil<T, L, E> sm
         }
         return;
     }
+    __syncthreads();
 #pragma unroll
     for (int e = 0; e < E; e++) sm.at(out_row<L, E, false>(q, e)) = r[e];
     __syncthreads();
@@ -503,7 +504,7 @@ __device__ __forceinline__ void k3_z_body(Geo g, cx<T> *__restrict__ buf, const 
     const bool ok = pen < npen;
     const long long base = (ok ? pen : 0) * g.Kp;
     cx<T> *smc = reinterpret_cast<cx<T> *>(smraw);
-    constexpr int PITCH = pencil_pitch<T, L, E>();
+    constexpr int PITCH = SmPencil<T, L, E>::PITCH;
     SmPencil<T, L, E> sm{smc + p * PITCH};
     const T sz = T(g.sz);
     cx<T> *const B0 = buf + base;
@@ -513,9 +514,9 @@ __device__ __forceinline__ void k3_z_body(Geo g, cx<T> *__restrict__ buf, const 
     if constexpr (MODE == MODE_VEL) {
         cx<T> A[E], B[E];
         k3_load_pair<T, L, E>(A, F(0), false, F(1), false, g.Kz, sz, q, ok);
-        pencil_fft<T, L, E, true, (32 % (L / E) == 0)>(A, sm, q, tw);
+        fft<T, L, E, true, SmPencil<T, L, E>, (32 % (L / E) == 0)>(A, sm, q, tw);
         k3_load_pair<T, L, E>(B, F(2), false, nullptr, false, g.Kz, sz, q, ok);
-        pencil_fft<T, L, E, true, (32 % (L / E) == 0)>(B, sm, q, tw);
+        fft<T, L, E, true, SmPencil<T, L, E>, (32 % (L / E) == 0)>(B, sm, q, tw);
         double ss = 0.0;
 #pragma unroll
         for (int e = 0; e < E; e++) {
@@ -581,7 +582,7 @@ __device__ __forceinline__ void k3_z_body(Geo g, cx<T> *__restrict__ buf, const 
                 else if (pi == FIRST + 2) { cp_async_wait<0>(); __syncthreads(); }
             }
             k3_load_pair<T, L, E>(A, src[pi], false, src[pi + 3], false, g.Kz, sz, q, ok);
-            pencil_fft<T, L, E, true, (32 % (L / E) == 0)>(A, sm, q, tw);
+            fft<T, L, E, true, SmPencil<T, L, E>, (32 % (L / E) == 0)>(A, sm, q, tw);
             if (pi == 0) {
 #pragma unroll
                 for (int e = 0; e < E; e++) { rs[0][e] = A[e].x; rs[1][e] = A[e].y; }

@@ -211,6 +211,7 @@ __device__ __forceinline__ void k3_field_body(Geo g, SCx<T> *__restrict__ buf, c
             SmPencil<T, L, E> sm{smc + item * PITCH};
             k3_load_pair<T, L, E>(A, base + pr.a * g.S2, pr.da, pr.b < 0 ? nullptr : base + pr.b * g.S2, pr.db, Kz, sz, q, ok, g.Kp);
             fft<T, L, E, true, SmPencil<T, L, E>, WARP>(A, sm, q, tw);
+            stage_barrier<WARP>();
 #pragma unroll
             for (int e = 0; e < E; e++) sm.at(out_row<L, E, true>(q, e)) = A[e];
         }
@@ -240,8 +241,8 @@ __device__ __forceinline__ void k3_field_body(Geo g, SCx<T> *__restrict__ buf, c
             SCx<T> *oa = base + jb.a * g.S2, *ob = jb.b < 0 ? nullptr : base + jb.b * g.S2;
 #pragma unroll
             for (int e = 0; e < E; e++) A[e] = sm.at(in_row<L, E, false>(q, e));
-            stage_barrier<WARP>();
             fft<T, L, E, false, SmPencil<T, L, E>, WARP>(A, sm, q, tw);
+            stage_barrier<WARP>();
 #pragma unroll
             for (int e = 0; e < E; e++) sm.at(out_row<L, E, false>(q, e)) = A[e];
             stage_barrier<WARP>();

@@ -78,7 +78,7 @@ constexpr int ZS_WAIT_LIMIT = 1 << 22;
 // thread), SLOTS_SM physical slots of L reals per exchange buffer, then the block's mbarrier.
 template <typename T, int L, int E, int PB, int SLOTS_SM> struct ZStagedLayout {
     static constexpr int Q = L / E, W = Arith<T>::W;
-    static constexpr int PITCH = pencil_pitch<T, L, E>();
+    static constexpr int PITCH = SmPencil<T, L, E>::PITCH;
     // staged elements of np pencils of one field (whole 16-byte units, as Kp is)
     __host__ __device__ static int stage_elems(int np, int Kz, int Kp) {
         constexpr int U = 16 / (int)sizeof(SCx<T>);
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(PB *(L / E), MINB) k3_rot_staged(Geo g, SCx<T>
         k3_load_pair<T, L, E>(A, sa, false, sb, false, Kz, sz, q, ok, Kp);
         __syncthreads();
         issue(grp, 1, 4);
-        pencil_fft<T, L, E, true, WARP>(A, sm, q, tw);
+        fft<T, L, E, true, SmPencil<T, L, E>, WARP>(A, sm, q, tw);
 #pragma unroll
         for (int e = 0; e < E; e++) { SL(0, e) = A[e].x; SL(2, e) = A[e].y; }
         // pair 1: v + i w_y; then c_z = w_x v - w_y u, transformed and written over w_x (field 3)
@@ -176,14 +176,14 @@ __global__ void __launch_bounds__(PB *(L / E), MINB) k3_rot_staged(Geo g, SCx<T>
         k3_load_pair<T, L, E>(A, sa, false, sb, false, Kz, sz, q, ok, Kp);
         __syncthreads();
         issue(grp, 2, 5);
-        pencil_fft<T, L, E, true, WARP>(A, sm, q, tw);
+        fft<T, L, E, true, SmPencil<T, L, E>, WARP>(A, sm, q, tw);
 #pragma unroll
         for (int e = 0; e < E; e++) {
             const T vv = A[e].x, oy = A[e].y;
             SL(1, e) = vv; SL(3, e) = oy;
             A[e] = mk<T>(SL(2, e) * vv - oy * SL(0, e), T(0));
         }
-        pencil_fft<T, L, E, false, WARP>(A, sm, q, tw);
+        fft<T, L, E, false, SmPencil<T, L, E>, WARP>(A, sm, q, tw);
         if (ok) {
             SCx<T> *o = FZ(3);
 #pragma unroll
@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(PB *(L / E), MINB) k3_rot_staged(Geo g, SCx<T>
         k3_load_pair<T, L, E>(A, sa, false, sb, false, Kz, sz, q, ok, Kp);
         __syncthreads();
         if (grp + gridDim.x < ngrp) issue(grp + gridDim.x, 0, 3);
-        pencil_fft<T, L, E, true, WARP>(A, sm, q, tw);
+        fft<T, L, E, true, SmPencil<T, L, E>, WARP>(A, sm, q, tw);
 #pragma unroll
         for (int e = 0; e < E; e++) {
             const T ww = A[e].x, oz = A[e].y, uu = SL(0, e), vv = SL(1, e);
@@ -205,7 +205,8 @@ __global__ void __launch_bounds__(PB *(L / E), MINB) k3_rot_staged(Geo g, SCx<T>
             A[e] = mk<T>(SL(3, e) * ww - oz * vv, oz * uu - SL(2, e) * ww);
         }
         // forward transform of c_x + i c_y and extraction of both half spectra, kz < Kz
-        pencil_fft<T, L, E, false, WARP>(A, sm, q, tw);
+        fft<T, L, E, false, SmPencil<T, L, E>, WARP>(A, sm, q, tw);
+        stage_barrier<WARP>();
 #pragma unroll
         for (int e = 0; e < E; e++) sm.at(out_row<L, E, false>(q, e)) = A[e];
         stage_barrier<WARP>();
@@ -218,7 +219,6 @@ __global__ void __launch_bounds__(PB *(L / E), MINB) k3_rot_staged(Geo g, SCx<T>
                 st_pencil(ob, k, Kp, mk<T>(h * (zk.y + zm.y), h * (zm.x - zk.x)));
             }
         }
-        stage_barrier<WARP>();
 #undef SL
 #undef FZ
     }
