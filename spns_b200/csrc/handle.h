@@ -150,51 +150,14 @@ template <typename T, int L, int MODE, int ALT> using ShapeK5A =
 #ifndef SPNS_SPLIT_WAVES
 #define SPNS_SPLIT_WAVES 4       // x/y passes with fewer than 4 blocks per SM spread their fields over blocks
 #endif
-// Rotational z pass with pair-by-pair bulk-copy staging, persistent
-// (k3_rot_staged, zpass_staged.cuh): used at lengths from SPNS_ZS_MIN_L up to 768.
-// Per precision: E values per thread, PB pencils per block, SLOTS physical slots
-// in shared memory (of four), MINB resident blocks per SM for the register budget.
-#ifndef SPNS_ZS_MIN_L
-#define SPNS_ZS_MIN_L 384         // double: measured 14.65 against 14.93 ms at 768, slower at 384
-#endif
-#ifndef SPNS_F32_ZS_MIN_L
-#define SPNS_F32_ZS_MIN_L 100000  // single: off (12.29 against 11.61 ms at 768)
-#endif
-#ifndef SPNS_ZS_E
-#define SPNS_ZS_E 12
-#endif
-// Double at 768, N=512: one pencil per block, two of the four slots in shared memory and
-// 6 blocks per SM (12 warps) 12.97 ms; two pencils per block with one slot and 3 blocks
-// 13.74, with no slot and 2 blocks 13.94; one pencil with one slot 13.19 (6 blocks), 14.42 (7).
-#ifndef SPNS_ZS_PB
-#define SPNS_ZS_PB 1
-#endif
-#ifndef SPNS_ZS_SLOTS
-#define SPNS_ZS_SLOTS 2
-#endif
-#ifndef SPNS_ZS_MINB
-#define SPNS_ZS_MINB 6
-#endif
-#ifndef SPNS_F32_ZS_E
-#define SPNS_F32_ZS_E 12
-#endif
-#ifndef SPNS_F32_ZS_PB
-#define SPNS_F32_ZS_PB 2
-#endif
-#ifndef SPNS_F32_ZS_SLOTS
-#define SPNS_F32_ZS_SLOTS 0
-#endif
-#ifndef SPNS_F32_ZS_MINB
-#define SPNS_F32_ZS_MINB 4
-#endif
-template <typename T, int L> struct ZStagedShape {
-    static constexpr bool D = sizeof(T) == 8;
-    static constexpr int E = D ? SPNS_ZS_E : SPNS_F32_ZS_E;
-    static constexpr int PB = D ? SPNS_ZS_PB : SPNS_F32_ZS_PB;
-    static constexpr int SLOTS = D ? SPNS_ZS_SLOTS : SPNS_F32_ZS_SLOTS;
-    static constexpr int MINB = D ? SPNS_ZS_MINB : SPNS_F32_ZS_MINB;
-    static constexpr bool ON = L >= (D ? SPNS_ZS_MIN_L : SPNS_F32_ZS_MIN_L) && L <= 768 && L % E == 0 && spns::n_stages(L, E) > 0;
-};
+// Rotational z pass with pair-by-pair bulk-copy staging and slots in tensor memory
+// (k3_rot_staged, zpass_staged.cuh): lengths whose pencils, at 12 values per thread, are a
+// part of a warp, one or two warps; k3_z runs the others.
+// Staged against k3_z: double 768 11.5 against 14.9 ms (N=512), 192 0.175 against 0.199 (N=128),
+// 96 0.031 against 0.034 (N=64), 48 0.018 against 0.015 (N=32); single 192 0.121 against 0.125,
+// 96 0.027 against 0.021: short pencils leave too few values per staged pair.
+template <typename T> constexpr bool spns_zstaged_length(int L) { return L == 768 || L == 384 || L == 192 || (L == 96 && sizeof(T) == 8); }
+constexpr int SPNS_ZS_E = 12;
 
 // Velocity and short-length rotational z pass (k3_z): pencils per block limited by the
 // shared memory of the exchange buffers.

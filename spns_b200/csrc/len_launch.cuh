@@ -51,24 +51,18 @@ template <typename T> struct LenLaunch {
         return cudaGetLastError();
     }
     // Rotational z pass staged pair by pair with bulk copies (zpass_staged.cuh),
-    // persistent: one wave of blocks over the SMs.
+    // persistent: one block per SM.
     template <int L> static cudaError_t launch_k3_staged(spns_handle *h) {
-        using ZS = ZStagedShape<A, L>;
-        using LY = spns::ZStagedLayout<A, L, ZS::E, ZS::PB, ZS::SLOTS>;
-        auto kern = spns::k3_rot_staged<A, L, ZS::E, ZS::PB, ZS::SLOTS, ZS::MINB>;
-        const size_t smem = LY::smem_bytes(h->g.Kz, h->g.Kp);
+        using LY = spns::ZStagedLayout<A, L, SPNS_ZS_E>;
+        auto kern = spns::k3_rot_staged<A, L, SPNS_ZS_E>;
+        const long long ngrp = (long long)h->g.Mx * h->g.My / (LY::PPU * LY::W);
+        // as many units as a block holds, or as it takes to spread the pencils over the SMs
+        const int units = (int)std::min<long long>(LY::max_units(h->g.Kz, h->g.Kp), (ngrp + h->sms - 1) / h->sms);
+        const size_t smem = LY::smem_bytes(units, h->g.Kz, h->g.Kp);
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        constexpr int THREADS = ZS::PB * LY::Q;
-        int dev = 0, sms = 0, per_sm = 0;
-        if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-        if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, THREADS, smem)) != cudaSuccess) return e;
-        if (per_sm < 1) return cudaErrorInvalidConfiguration;
-        const long long groups = ((long long)h->g.Mx * h->g.My / LY::W + ZS::PB - 1) / ZS::PB;
-        long long blocks = (long long)sms * per_sm;
-        if (blocks > groups) blocks = groups;
-        kern<<<(unsigned)blocks, THREADS, smem, h->st>>>(h->g, (C *)h->B2, h->c, h->ds, twa(h, L));
+        const unsigned blocks = (unsigned)std::min<long long>((ngrp + units - 1) / units, h->sms);
+        kern<<<blocks, units * LY::U, smem, h->st>>>(h->g, (C *)h->B2, h->c, h->ds, twa(h, L));
         return cudaGetLastError();
     }
     // Persistent launch of k3_field: one wave of blocks.
@@ -95,7 +89,7 @@ template <typename T> struct LenLaunch {
         if constexpr (MODE != spns::MODE_VEL && MODE != spns::MODE_ROT) {
             return launch_k3_field<L, MODE, ALT>(h, phys);
         } else {
-        if constexpr (MODE == spns::MODE_ROT && ALT == 0 && ZStagedShape<A, L>::ON) return launch_k3_staged<L>(h);
+        if constexpr (MODE == spns::MODE_ROT && ALT == 0 && spns_zstaged_length<T>(L)) return launch_k3_staged<L>(h);
         using S3 = Shape3<T, L, ALT>;
         constexpr bool STAGE = MODE == spns::MODE_ROT && ShapeSel<T>::Z_STAGE;
         auto kern = spns::k3_z<T, L, S3::E, S3::P, MODE, STAGE>;

@@ -6,27 +6,29 @@
 // product c = w x u and the CFL maxima on the grid, r2c of c truncated to
 // kz <= hz (src/HIT_LES.cpp:74-125 up to the gradient the projection removes).
 // What differs is the schedule:
-//   * A block of PB pencils (Q = L/E threads each) is persistent: it walks the
-//     groups of PB consecutive pencils with a stride of the grid.  Only the two
-//     fields of the next input pair are staged in shared memory, by
-//     cp.async.bulk (TMA bulk copies global -> shared, completion counted in
-//     bytes on an mbarrier), while the current pair is transformed; the first
-//     pair of the next group is fetched during the two forward transforms.  The
-//     staging takes 2*PB*Kz complex values instead of 6*PB*Kz, so more blocks fit
-//     an SM.  In single precision (T = f2) a thread transforms two neighbouring pencils
-//     with packed arithmetic, so a block is the double-precision block of 2 PB pencils.
-//   * Working set per thread: four physical slots (u, v, w_x, w_y; the last
-//     SLOTS_SM of them in shared memory, own rows only) and one complex register
-//     array.  c_z
-//     is transformed as soon as it is known (after the second pair) and written
+//   * One block per SM, persistent, of independent units: a warp with one or several
+//     pencils (Q = L/E threads each), or the two warps of one pencil.  Each unit walks the
+//     pencils with the stride of the grid, with its own staging, mbarrier and exchange
+//     barrier.  Only the two fields of the next input pair are staged in shared memory, by
+//     cp.async.bulk (TMA bulk copies global -> shared, completion counted in bytes on an
+//     mbarrier), while the current pair is transformed; the first pair of the next pencils
+//     is fetched during the last transforms.
+//     In single precision (T = f2) a thread transforms two neighbouring pencils with
+//     packed arithmetic.
+//   * The four physical slots (u, v, w_x, w_y) are thread-private and live in tensor
+//     memory beside the running CFL maxima (104 columns a warp).  They took 24 of
+//     the 168 registers and 12 KB of shared memory per pencil at length 768, which held the
+//     pass to 12 warps per SM; now it is 16, and the slots' accesses leave the
+//     shared-memory pipe, the busiest one (77 % of its cycles; the FP64 pipe 44 %).
+//     Before and now: double 512^3 13.0 -> 11.5 ms, single 8.5 -> 7.1.
+//   * c_z is transformed as soon as it is known (after the second pair) and written
 //     over the w_x field of the same pencil (S2 field 3, consumed at the first
 //     pair), so the forward y pass reads the nonlinear term from fields 0, 1, 3.
-//   * Pencils of Q <= 32 threads exchange within their warp (__syncwarp).
 //   * CFL maxima accumulate per thread over all pencils and are reduced once per
 //     block at the end.
 // Every mbarrier wait is bounded; a wait that gives up records wait_timeout in
-// the solver scalars (reported as SPNS_ERR_TIMEOUT by the host) and the block
-// skips its remaining pencils; no copy is left in flight.
+// the solver scalars (reported as SPNS_ERR_TIMEOUT by the host) and the pencil's
+// threads skip their remaining pencils; no copy is left in flight.
 #pragma once
 #include "solver_kernels.cuh"
 
@@ -73,119 +75,192 @@ __device__ __forceinline__ bool mbar_wait_bounded(unsigned long long *bar, unsig
 
 constexpr int ZS_WAIT_LIMIT = 1 << 22;
 
-// Shared memory of one block: PB exchange buffers, 2 staging fields of PB * W pencils (rows
-// of the work buffers' pitch Kp, the last without its padding; W = Arith<T>::W pencils to a
-// thread), SLOTS_SM physical slots of L reals per exchange buffer, then the block's mbarrier.
-template <typename T, int L, int E, int PB, int SLOTS_SM> struct ZStagedLayout {
-    static constexpr int Q = L / E, W = Arith<T>::W;
-    static constexpr int PITCH = SmPencil<T, L, E>::PITCH;
-    // staged elements of np pencils of one field (whole 16-byte units, as Kp is)
-    __host__ __device__ static int stage_elems(int np, int Kz, int Kp) {
-        constexpr int U = 16 / (int)sizeof(SCx<T>);
-        return (np - 1) * Kp + (Kz + U - 1) / U * U;
-    }
-    __host__ __device__ static size_t stage_bytes(int Kz, int Kp) { return (size_t)stage_elems(PB * W, Kz, Kp) * sizeof(SCx<T>); }
-    static constexpr size_t EXCH = (size_t)PB * PITCH * sizeof(cx<T>), SLOTS = (size_t)SLOTS_SM * PB * L * sizeof(T);
-    __host__ __device__ static size_t bar_offset(int Kz, int Kp) { return EXCH + 2 * stage_bytes(Kz, Kp) + SLOTS; }
-    __host__ __device__ static size_t smem_bytes(int Kz, int Kp) { return bar_offset(Kz, Kp) + 16; }
-};
-
-// Physical slot S (0 u, 1 v, 2 w_x, 3 w_y) of register slot e (grid row `row`):
-// the first NREG in registers, the rest in shared memory (stride `pitch` reals).
-template <int S, int NREG, typename T, int E>
-__device__ __forceinline__ T &zs_slot(T (&rg)[NREG > 0 ? NREG : 1][E], T *sm_slots, int pitch, int e, int row) {
-    if constexpr (S < NREG) return rg[S][e];
-    else return sm_slots[(S - NREG) * pitch + row];
+// ---------------------------------------------------------------------------
+// Thread-private values in tensor memory.  A warp may store and load 32-bit columns of its
+// own 32 lanes (shape 32x32b: lane i of the warp, its rank in the block modulo 4 selecting
+// the lanes), so an allocation of C columns is C words of storage for each of 128 lanes
+// beside registers and shared memory, with its own path to the SM.
+// ---------------------------------------------------------------------------
+// One whole warp; the address (columns' base) is written to shared memory.
+template <int COLS> __device__ __forceinline__ void tmem_alloc(unsigned *dst) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_addr(dst)), "n"(COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+}
+template <int COLS> __device__ __forceinline__ void tmem_free(unsigned addr) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(addr), "n"(COLS) : "memory");
+}
+__device__ __forceinline__ unsigned long long bits64(double v) { return (unsigned long long)__double_as_longlong(v); }
+__device__ __forceinline__ unsigned long long bits64(f2 v) { return v.v; }
+__device__ __forceinline__ void from_bits64(unsigned long long b, double &v) { v = __longlong_as_double((long long)b); }
+__device__ __forceinline__ void from_bits64(unsigned long long b, f2 &v) { v.v = b; }
+// four 64-bit values of the thread to / from 8 columns; a load's values are defined after tmem_wait_ld
+template <typename T> __device__ __forceinline__ void tmem_st4(unsigned addr, T a, T b, T c, T d) {
+    const unsigned long long v[4] = {bits64(a), bits64(b), bits64(c), bits64(d)};
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n" ::"r"(addr), "r"((unsigned)v[0]),
+                 "r"((unsigned)(v[0] >> 32)), "r"((unsigned)v[1]), "r"((unsigned)(v[1] >> 32)), "r"((unsigned)v[2]),
+                 "r"((unsigned)(v[2] >> 32)), "r"((unsigned)v[3]), "r"((unsigned)(v[3] >> 32))
+                 : "memory");
+}
+struct Tmem4 { unsigned r[8]; };
+__device__ __forceinline__ void tmem_ld4(unsigned addr, Tmem4 &v) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
+                 : "=r"(v.r[0]), "=r"(v.r[1]), "=r"(v.r[2]), "=r"(v.r[3]), "=r"(v.r[4]), "=r"(v.r[5]), "=r"(v.r[6]), "=r"(v.r[7])
+                 : "r"(addr)
+                 : "memory");
+}
+// completes the loads; the values pass through it, so no use moves above
+__device__ __forceinline__ void tmem_wait_ld(Tmem4 &v) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;\n"
+                 : "+r"(v.r[0]), "+r"(v.r[1]), "+r"(v.r[2]), "+r"(v.r[3]), "+r"(v.r[4]), "+r"(v.r[5]), "+r"(v.r[6]), "+r"(v.r[7])::"memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
+template <typename T> __device__ __forceinline__ T tmem_value(const Tmem4 &v, int i) {
+    T x;
+    from_bits64((unsigned long long)v.r[2 * i] | ((unsigned long long)v.r[2 * i + 1] << 32), x);
+    return x;
 }
 
-template <typename T, int L, int E, int PB, int SLOTS_SM, int MINB>
-__global__ void __launch_bounds__(PB *(L / E), MINB) k3_rot_staged(Geo g, SCx<T> *__restrict__ buf, StepConsts c, DevScalars *ds,
-                                                                   const cx<T> *__restrict__ tw) {
-    using LY = ZStagedLayout<T, L, E, PB, SLOTS_SM>;
-    constexpr int Q = LY::Q, THREADS = PB * Q;
-    static_assert(SLOTS_SM >= 0 && SLOTS_SM <= 4, "zero to four slots in shared memory");
-    constexpr bool WARP = (32 % Q == 0);                      // a pencil never leaves its warp
-    constexpr int W = LY::W;
+// One block per SM of up to ZSTAGED_THREADS threads (the runtime places one block with
+// tensor memory per SM, so the SM's warps are one block).  A unit is a warp with 32/Q
+// pencils (pairs of pencils, T = f2), or the two warps of one (Q = 64); each unit has the
+// exchange buffers of its pencils, 2 staging fields (rows of the work buffers' pitch Kp, the
+// last without its padding) and an mbarrier; one word for the block's tensor-memory address.
+constexpr int ZSTAGED_THREADS = 512;
+template <typename T, int L, int E> struct ZStagedLayout {
+    static constexpr int Q = L / E, W = Arith<T>::W, U = Q <= 32 ? 32 : Q, PPU = U / Q;
+    using SM = SmPencil<T, L, E>;
+    static_assert((Q <= 32 && 32 % Q == 0) || Q == 64, "pencils are a part of a warp, one warp or an aligned pair of warps");
+    static_assert(E == 12, "twelve values a thread: three tensor-memory accesses of four per slot");
+    static constexpr unsigned BAR = Q <= 32 ? 1u : GROUP64;
+    static constexpr int COLS = 512;                 // all of the SM's; 128 (of 104 used) for each of the 4 warps of a lane quarter
+    // every compiled length is even, so the rows of a field are a multiple of 4: no unit is partly filled
+    static_assert(4 % (PPU * W) == 0, "rows of a unit");
+    // the unit's rows of one field, the last without its padding (whole 16-byte units, as Kp is)
+    __host__ __device__ static constexpr size_t stage_bytes(int Kz, int Kp) {
+        constexpr int A = 16 / (int)sizeof(SCx<T>);
+        return (size_t)((PPU * W - 1) * Kp + (Kz + A - 1) / A * A) * sizeof(SCx<T>);
+    }
+    static constexpr size_t EXCH = (size_t)PPU * SM::PITCH * sizeof(cx<T>);
+    __host__ __device__ static constexpr size_t unit_bytes(int Kz, int Kp) { return EXCH + 2 * stage_bytes(Kz, Kp) + sizeof(unsigned long long); }
+    __host__ __device__ static constexpr size_t smem_bytes(int units, int Kz, int Kp) { return units * unit_bytes(Kz, Kp) + 16; }
+    // most units of a block
+    __host__ __device__ static constexpr int max_units(int Kz, int Kp) {
+        const int s = (int)((225 * 1024) / unit_bytes(Kz, Kp)), t = ZSTAGED_THREADS / U;
+        return s < t ? s : t;
+    }
+};
+
+// true on every thread of the unit if `ok` is on all of them (a barrier of the group)
+template <int U> __device__ __forceinline__ bool unit_all(bool ok) {
+    if constexpr (U == 32) {
+        return __all_sync(0xffffffffu, ok) != 0;
+    } else {
+        unsigned r;
+        asm volatile("{\n.reg .pred p, r;\nsetp.ne.u32 p, %1, 0;\nbar.red.and.pred r, %2, 64, p;\nselp.u32 %0, 1, 0, r;\n}\n"
+                     : "=r"(r)
+                     : "r"((unsigned)ok), "r"(1 + (threadIdx.x >> 6))
+                     : "memory");
+        return r != 0;
+    }
+}
+
+template <typename T, int L, int E>
+__global__ void __launch_bounds__(ZSTAGED_THREADS, 1) k3_rot_staged(Geo g, SCx<T> *__restrict__ buf, StepConsts c, DevScalars *ds,
+                                                        const cx<T> *__restrict__ tw) {
+    using LY = ZStagedLayout<T, L, E>;
+    constexpr int Q = LY::Q, W = LY::W, U = LY::U, PPU = LY::PPU;
+    constexpr unsigned BAR = LY::BAR;
     extern __shared__ __align__(128) unsigned char smraw_zs[];
-    const int tid = threadIdx.x, sub = tid / Q, q0 = tid % Q;
-    const int Kz = g.Kz;
-    const int Kp = g.Kp;
-    cx<T> *const smc = reinterpret_cast<cx<T> *>(smraw_zs);
-    SmPencil<T, L, E> sm{smc + sub * LY::PITCH};
-    SCx<T> *const stA = reinterpret_cast<SCx<T> *>(smraw_zs + LY::EXCH);                              // staging: field a of the pair
-    SCx<T> *const stB = reinterpret_cast<SCx<T> *>(smraw_zs + LY::EXCH + LY::stage_bytes(Kz, Kp));    // field b
-    T *const slot_sm = reinterpret_cast<T *>(smraw_zs + LY::EXCH + 2 * LY::stage_bytes(Kz, Kp)) + sub * L;   // slot j of this pencil at slot_sm[j*PB*L + row]
-    unsigned long long *const bar = reinterpret_cast<unsigned long long *>(smraw_zs + LY::bar_offset(Kz, Kp));
-    if (tid == 0) {
+    const int tid = threadIdx.x, unit = tid / U, units = blockDim.x / U, sub = tid % U / Q, q0 = tid % Q;
+    const int Kz = g.Kz, Kp = g.Kp;
+    const size_t sb = LY::stage_bytes(Kz, Kp);
+    unsigned char *const mine = smraw_zs + unit * (LY::EXCH + 2 * sb);
+    typename LY::SM sm{reinterpret_cast<cx<T> *>(mine) + sub * LY::SM::PITCH};
+    SCx<T> *const stA = reinterpret_cast<SCx<T> *>(mine + LY::EXCH);             // staging: field a of the pair
+    SCx<T> *const stB = reinterpret_cast<SCx<T> *>(mine + LY::EXCH + sb);        // field b
+    unsigned long long *const bars = reinterpret_cast<unsigned long long *>(smraw_zs + units * (LY::EXCH + 2 * sb)), *const bar = bars + unit;
+    unsigned *const taddr = reinterpret_cast<unsigned *>(bars + units);
+    if (tid < 32) tmem_alloc<LY::COLS>(taddr);
+    if (tid % U == 0) {
         mbar_init(bar, 1);
         fence_mbar_init();
     }
     __syncthreads();
+    // this warp's lanes and columns; slots of 24 columns: 0 u, 1 v, 2 w_x, 3 w_y
+    const unsigned tbase = *taddr;
+    const unsigned slots = tbase + ((unsigned)(tid >> 5 & 3) << 21) + (unsigned)(tid >> 7) * 128u;
 
-    // npen is even (every compiled length is), so W = 2 leaves no single pencil
-    const long long npen = (long long)g.Mx * g.My / W;
-    const long long ngrp = (npen + PB - 1) / PB;
+    const long long ngrp = (long long)g.Mx * g.My / (PPU * W), step = (long long)gridDim.x * units;
     const T sz = T(g.sz);
     unsigned parity = 0;
     bool bad = false;
-    double mx[4] = {0.0, 0.0, 0.0, 0.0};
+    // running CFL maxima of the thread: four doubles in columns 96..103
+    tmem_st4<double>(slots + 96, 0.0, 0.0, 0.0, 0.0);
+    tmem_wait_st();
 
-    // stage fields fa, fb of group grp (its pencils' rows are contiguous in each field)
+    // stage fields fa, fb of the PPU pencils of group grp (their rows are contiguous in each field)
     auto issue = [&](long long grp, int fa, int fb) {
-        if (tid != 0) return;
-        const long long p0 = grp * PB;
-        const int np = (int)(npen - p0 < PB ? npen - p0 : PB) * W;
-        const SCx<T> *A = buf + (long long)fa * g.S2 + p0 * W * Kp, *B = buf + (long long)fb * g.S2 + p0 * W * Kp;
-        const unsigned bytes = (unsigned)(LY::stage_elems(np, Kz, Kp) * sizeof(SCx<T>));
+        if (tid % U != 0) return;
+        const unsigned bytes = (unsigned)sb;
+        const SCx<T> *p = buf + grp * (PPU * W) * Kp;
         fence_proxy_async_smem();
         mbar_arrive_expect_tx(bar, 2 * bytes);
-        bulk_copy_g2s(stA, A, bytes, bar);
-        bulk_copy_g2s(stB, B, bytes, bar);
+        bulk_copy_g2s(stA, p + fa * g.S2, bytes, bar);
+        bulk_copy_g2s(stB, p + fb * g.S2, bytes, bar);
     };
-    // the staged pair is complete and visible to every thread of the block
+    // the staged pair is complete and visible to every thread of the unit
     auto wait_stage = [&]() -> bool {
         const bool ok = mbar_wait_bounded(bar, parity, ZS_WAIT_LIMIT);
         parity ^= 1u;
-        return __syncthreads_and(ok ? 1 : 0) != 0;
+        return unit_all<U>(ok);
     };
 
-    long long grp = blockIdx.x;
+    long long grp = (long long)blockIdx.x * units + unit;
     if (grp < ngrp) issue(grp, 0, 3);
-    for (; grp < ngrp; grp += gridDim.x) {
+    for (; grp < ngrp; grp += step) {
         const int q = opaque(q0);
-        const long long pen = grp * PB + sub;
-        const bool ok = pen < npen;
-        SCx<T> *const B0 = buf + (ok ? pen : 0) * W * Kp;
-#define FZ(i) (B0 + (long long)(i) * g.S2)
-        const SCx<T> *sa = stA + sub * W * Kp, *sb = stB + sub * W * Kp;
+        SCx<T> *const B0 = buf + (grp * PPU + sub) * W * Kp;
+        const SCx<T> *const sa = stA + sub * W * Kp, *const sb_ = stB + sub * W * Kp;
         cx<T> A[E];
-        constexpr int NREG = 4 - SLOTS_SM;
-        T r_sl[NREG > 0 ? NREG : 1][E];
-        // physical slot j (0 u, 1 v, 2 w_x, 3 w_y) of register slot e
-#define SL(j, e) zs_slot<(j), NREG, T, E>(r_sl, slot_sm, PB * L, (e), out_row<L, E, true>(q, (e)))
         // pair 0: u + i w_x
         if (!wait_stage()) { bad = true; break; }
-        k3_load_pair<T, L, E>(A, sa, false, sb, false, Kz, sz, q, ok, Kp);
-        __syncthreads();
+        k3_load_pair<T, L, E>(A, sa, false, sb_, false, Kz, sz, q, true, Kp);
+        stage_barrier<BAR>();
         issue(grp, 1, 4);
-        fft<T, L, E, true, SmPencil<T, L, E>, WARP>(A, sm, q, tw);
+        fft<T, L, E, true, typename LY::SM, BAR>(A, sm, q, tw);
+        __syncwarp();
 #pragma unroll
-        for (int e = 0; e < E; e++) { SL(0, e) = A[e].x; SL(2, e) = A[e].y; }
+        for (int i = 0; i < 3; i++) {
+            tmem_st4<T>(slots + 8 * i, A[4 * i].x, A[4 * i + 1].x, A[4 * i + 2].x, A[4 * i + 3].x);
+            tmem_st4<T>(slots + 48 + 8 * i, A[4 * i].y, A[4 * i + 1].y, A[4 * i + 2].y, A[4 * i + 3].y);
+        }
+        tmem_wait_st();
         // pair 1: v + i w_y; then c_z = w_x v - w_y u, transformed and written over w_x (field 3)
         if (!wait_stage()) { bad = true; break; }
-        k3_load_pair<T, L, E>(A, sa, false, sb, false, Kz, sz, q, ok, Kp);
-        __syncthreads();
+        k3_load_pair<T, L, E>(A, sa, false, sb_, false, Kz, sz, q, true, Kp);
+        stage_barrier<BAR>();
         issue(grp, 2, 5);
-        fft<T, L, E, true, SmPencil<T, L, E>, WARP>(A, sm, q, tw);
+        fft<T, L, E, true, typename LY::SM, BAR>(A, sm, q, tw);
+        __syncwarp();
 #pragma unroll
-        for (int e = 0; e < E; e++) {
-            const T vv = A[e].x, oy = A[e].y;
-            SL(1, e) = vv; SL(3, e) = oy;
-            A[e] = mk<T>(SL(2, e) * vv - oy * SL(0, e), T(0));
+        for (int i = 0; i < 3; i++) {
+            Tmem4 tu, tx;
+            tmem_ld4(slots + 8 * i, tu);
+            tmem_ld4(slots + 48 + 8 * i, tx);
+            tmem_st4<T>(slots + 24 + 8 * i, A[4 * i].x, A[4 * i + 1].x, A[4 * i + 2].x, A[4 * i + 3].x);
+            tmem_st4<T>(slots + 72 + 8 * i, A[4 * i].y, A[4 * i + 1].y, A[4 * i + 2].y, A[4 * i + 3].y);
+            tmem_wait_ld(tu);
+            tmem_wait_ld(tx);
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int e = 4 * i + k;
+                A[e] = mk<T>(tmem_value<T>(tx, k) * A[e].x - A[e].y * tmem_value<T>(tu, k), T(0));
+            }
         }
-        fft<T, L, E, false, SmPencil<T, L, E>, WARP>(A, sm, q, tw);
-        if (ok) {
-            SCx<T> *o = FZ(3);
+        tmem_wait_st();
+        fft<T, L, E, false, typename LY::SM, BAR>(A, sm, q, tw);
+        {
+            SCx<T> *o = B0 + 3 * g.S2;
 #pragma unroll
             for (int e = 0; e < E; e++) {
                 const int row = out_row<L, E, false>(q, e);
@@ -194,36 +269,60 @@ __global__ void __launch_bounds__(PB *(L / E), MINB) k3_rot_staged(Geo g, SCx<T>
         }
         // pair 2: w + i w_z; then (c_x, c_y) and the CFL maxima
         if (!wait_stage()) { bad = true; break; }
-        k3_load_pair<T, L, E>(A, sa, false, sb, false, Kz, sz, q, ok, Kp);
-        __syncthreads();
-        if (grp + gridDim.x < ngrp) issue(grp + gridDim.x, 0, 3);
-        fft<T, L, E, true, SmPencil<T, L, E>, WARP>(A, sm, q, tw);
+        k3_load_pair<T, L, E>(A, sa, false, sb_, false, Kz, sz, q, true, Kp);
+        stage_barrier<BAR>();
+        if (grp + step < ngrp) issue(grp + step, 0, 3);
+        fft<T, L, E, true, typename LY::SM, BAR>(A, sm, q, tw);
+        __syncwarp();
+        Tmem4 tm;
+        tmem_ld4(slots + 96, tm);
+        tmem_wait_ld(tm);
+        double mx[4] = {tmem_value<double>(tm, 0), tmem_value<double>(tm, 1), tmem_value<double>(tm, 2), tmem_value<double>(tm, 3)};
 #pragma unroll
-        for (int e = 0; e < E; e++) {
-            const T ww = A[e].x, oz = A[e].y, uu = SL(0, e), vv = SL(1, e);
-            if (ok) cfl_rows(mx, uu, vv, ww, c);
-            A[e] = mk<T>(SL(3, e) * ww - oz * vv, oz * uu - SL(2, e) * ww);
+        for (int i = 0; i < 3; i++) {
+            Tmem4 tu, tv, tx, ty;
+            tmem_ld4(slots + 8 * i, tu);
+            tmem_ld4(slots + 24 + 8 * i, tv);
+            tmem_ld4(slots + 48 + 8 * i, tx);
+            tmem_ld4(slots + 72 + 8 * i, ty);
+            tmem_wait_ld(tu);
+            tmem_wait_ld(tv);
+            tmem_wait_ld(tx);
+            tmem_wait_ld(ty);
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int e = 4 * i + k;
+                const T ww = A[e].x, oz = A[e].y, uu = tmem_value<T>(tu, k), vv = tmem_value<T>(tv, k);
+                cfl_rows(mx, uu, vv, ww, c);
+                A[e] = mk<T>(tmem_value<T>(ty, k) * ww - oz * vv, oz * uu - tmem_value<T>(tx, k) * ww);
+            }
         }
+        tmem_st4<double>(slots + 96, mx[0], mx[1], mx[2], mx[3]);
+        tmem_wait_st();
         // forward transform of c_x + i c_y and extraction of both half spectra, kz < Kz
-        fft<T, L, E, false, SmPencil<T, L, E>, WARP>(A, sm, q, tw);
-        stage_barrier<WARP>();
+        fft<T, L, E, false, typename LY::SM, BAR>(A, sm, q, tw);
+        stage_barrier<BAR>();
 #pragma unroll
         for (int e = 0; e < E; e++) sm.at(out_row<L, E, false>(q, e)) = A[e];
-        stage_barrier<WARP>();
-        if (ok) {
+        stage_barrier<BAR>();
+        {
             const T h = T(0.5);
-            SCx<T> *oa = FZ(0), *ob = FZ(1);
+            SCx<T> *oa = B0, *ob = B0 + g.S2;
             for (int k = q; k < Kz; k += Q) {
                 const cx<T> zk = sm.at(k), zm = sm.at(k == 0 ? 0 : L - k);
                 st_pencil(oa, k, Kp, mk<T>(h * (zk.x + zm.x), h * (zk.y - zm.y)));
                 st_pencil(ob, k, Kp, mk<T>(h * (zk.y + zm.y), h * (zm.x - zk.x)));
             }
         }
-#undef SL
-#undef FZ
     }
-    if (bad && tid == 0) atomicExch(&ds->wait_timeout, 1);
-    block_max4<T>(mx, ds);
+    if (bad && tid % U == 0) atomicExch(&ds->wait_timeout, 1);
+    __syncwarp();
+    Tmem4 tm;
+    tmem_ld4(slots + 96, tm);
+    tmem_wait_ld(tm);
+    const double mx[4] = {tmem_value<double>(tm, 0), tmem_value<double>(tm, 1), tmem_value<double>(tm, 2), tmem_value<double>(tm, 3)};
+    block_max4<T>(mx, ds);   // (a block barrier: every warp is done with the tensor memory)
+    if (tid < 32) tmem_free<LY::COLS>(tbase);
 }
 
 } // namespace spns
