@@ -109,13 +109,36 @@ __host__ __device__ constexpr int greedy_radix(int L, int E, int s) {
     for (int i = 0; i < s; i++) rem /= pick_radix(rem, E);
     return pick_radix(rem, E);
 }
-template <int L, int E, bool INV> struct Plan {
-    static constexpr int NST = n_stages(L, E);
+// Plan with a middle radix that does not divide the values per thread (UNEVEN): 768 = 12 x
+// 16 x 4 at 12 values per thread, two exchanges where the greedy plan 12 x 4 x 4 x 4 takes
+// three.  48 radix-16 butterflies over 64 threads per pencil leave a quarter of them idle in
+// that stage.  For the x/y passes (whole warps idle: inverse x at N=512, double, 4.58 ->
+// 4.14 ms); in the z pass, whose threads hold more beside the transform, the 16 values
+// spilled (13.0 -> 14.0 ms), and with 384 = 12 x 8 x 4, half of each warp taking a second
+// butterfly, it was slower too.  First and last radix, and so the rows of a thread's values,
+// are those of the greedy plan.
+__host__ __device__ constexpr bool has_uneven(int L, int E) { return L == 768 && E == 12; }
+__host__ __device__ constexpr int uneven_radix(int s) { return s == 0 ? 12 : s == 1 ? 16 : 4; }
+template <int L, int E, bool INV, bool UNEVEN = false> struct Plan {
+    static constexpr int NST = UNEVEN ? 3 : n_stages(L, E);
     static_assert(NST > 0, "length not factorable with radices dividing E");
     static_assert(L % E == 0, "E must divide L");
     static constexpr int Q = L / E;
-    __host__ __device__ static constexpr int radix(int s) { return INV ? greedy_radix(L, E, NST - 1 - s) : greedy_radix(L, E, s); }
+    __host__ __device__ static constexpr int radix(int s) { 
+        const int f = INV ? NST - 1 - s : s;
+        return UNEVEN ? uneven_radix(f) : greedy_radix(L, E, f);
+    }
     __host__ __device__ static constexpr int ns(int s) { int p = 1; for (int i = 0; i < s; i++) p *= radix(i); return p; }
+    // butterflies of stage s, and how many a thread takes at most (the last of them where j < NB)
+    __host__ __device__ static constexpr int nb(int s) { return L / radix(s); }
+    __host__ __device__ static constexpr int mb(int s) { return (nb(s) + Q - 1) / Q; }
+    // values a thread holds at most
+    __host__ __device__ static constexpr int width() {
+        int v = E;
+        for (int s = 0; s < NST; s++) v = mb(s) * radix(s) > v ? mb(s) * radix(s) : v;
+        return v;
+    }
+    static_assert(nb(0) % Q == 0 && nb(NST - 1) % Q == 0, "the first and last stage are even");
     static constexpr int R_first = radix(0);
     static constexpr int R_last = radix(NST - 1);
 };
@@ -158,6 +181,44 @@ template <typename T, bool INV> __device__ __forceinline__ void dft8(cx<T> *x) {
     x[1] = e[1] + o1;   x[5] = e[1] - o1;
     x[2] = INV ? a : b; x[6] = INV ? b : a;
     x[3] = e[3] + o3;   x[7] = e[3] - o3;
+}
+// Twiddles and 16-point DFT of one butterfly: x[r] times w^r, then 16 points as 4 x 4.  With
+// r = 4 n1 + n2 the factor w^(4 n1) goes before the DFT4 of column n2 and w^(n2), joined with
+// the inner twiddle w16^(n2 k1), after it: the multipliers of a column or a row are few and
+// short-lived, where the fifteen powers of one pass over x spilled.  w1, w2, w4, w8: powers of
+// the forward twiddle.
+template <typename T, bool INV> __device__ __forceinline__ void dft16_tw(cx<T> *x, cx<T> w1, cx<T> w2, cx<T> w4, cx<T> w8) {
+    const T c1 = T(0.92387953251128675612818318939679), s1 = T(0.38268343236508977172845998403040);   // cos, sin of pi/8
+    const T n_s1 = T(-0.38268343236508977172845998403040), n_c1 = T(-0.92387953251128675612818318939679);
+    const T h = T(0.70710678118654752440084436210485), n_h = T(-0.70710678118654752440084436210485);
+    auto mul = [](cx<T> a, cx<T> w) { return INV ? cmulc(a, w) : cmul(a, w); };
+    {
+        const cx<T> w12 = cmul(w8, w4);
+#pragma unroll
+        for (int n2 = 0; n2 < 4; n2++) {
+            cx<T> c[4] = {x[n2], mul(x[4 + n2], w4), mul(x[8 + n2], w8), mul(x[12 + n2], w12)};
+            dft4<T, INV>(c);
+#pragma unroll
+            for (int k1 = 0; k1 < 4; k1++) x[4 * k1 + n2] = c[k1];
+        }
+    }
+    const cx<T> w3 = cmul(w2, w1);
+    // w times w16^m (forward) = (c - i s), given c, s, -s
+    auto rot = [](cx<T> w, T c, T sn, T ns) { return mk<T>(mad(w.x, c, w.y * sn), mad(w.y, c, w.x * ns)); };
+    cx<T> y[16];
+#pragma unroll
+    for (int k1 = 0; k1 < 4; k1++) {
+        cx<T> m1 = w1, m2 = w2, m3 = w3;
+        if (k1 == 1) { m1 = rot(w1, c1, s1, n_s1); m2 = rot(w2, h, h, n_h); m3 = rot(w3, s1, c1, n_c1); }
+        else if (k1 == 2) { m1 = rot(w1, h, h, n_h); m2 = mk<T>(w2.y, -w2.x); m3 = rot(w3, n_h, h, n_h); }
+        else if (k1 == 3) { m1 = rot(w1, s1, c1, n_c1); m2 = rot(w2, n_h, h, n_h); m3 = rot(w3, n_c1, n_s1, s1); }
+        cx<T> c[4] = {x[4 * k1], mul(x[4 * k1 + 1], m1), mul(x[4 * k1 + 2], m2), mul(x[4 * k1 + 3], m3)};
+        dft4<T, INV>(c);
+#pragma unroll
+        for (int k2 = 0; k2 < 4; k2++) y[k1 + 4 * k2] = c[k2];
+    }
+#pragma unroll
+    for (int r = 0; r < 16; r++) x[r] = y[r];
 }
 // Good-Thomas split of R = A*B (gcd 1): input n = (B a + A b) mod R, output
 // k with k = ka (mod A), k = kb (mod B); DFT_A over a, then DFT_B over b.
@@ -217,6 +278,9 @@ template <class SM, bool INV, int S> __host__ __device__ constexpr int ex_pad() 
     if constexpr (SmPadded<SM>::value) return SM::template Ex<INV, S>::PAD;
     else return 0;
 }
+
+// accessors whose transforms take the uneven plan where there is one
+template <class SM, int L, int E> __host__ __device__ constexpr bool uneven_plan() { return has_uneven(L, E) && !SmPadded<SM>::value; }
 
 // Offset of the sub-table w_n^m (m < n) in a twiddle table of length L: 0 for
 // n = L (the base table), else L plus the sizes of the sub-tables of the divisors
@@ -282,20 +346,31 @@ __device__ __forceinline__ void twiddle_powers(cx<T> (&wp)[R], const cx<T> *__re
 }
 
 template <typename T, int L, int E, bool INV, unsigned WARP, int S, class SM>
-__device__ __forceinline__ void fft_run(cx<T> (&v)[E], SM sm, int q, const cx<T> *__restrict__ tw) {
-    using PL = Plan<L, E, INV>;
+__device__ __forceinline__ void fft_run(cx<T> (&v)[Plan<L, E, INV, uneven_plan<SM, L, E>()>::width()], SM sm, int q, const cx<T> *__restrict__ tw) {
+    using PL = Plan<L, E, INV, uneven_plan<SM, L, E>()>;
     constexpr int R = PL::radix(S);
     constexpr int Ns = PL::ns(S);
     constexpr int Q = PL::Q;
-    constexpr int MB = E / R;
+    constexpr int NB = PL::nb(S), MB = PL::mb(S);
 #pragma unroll
     for (int m = 0; m < MB; m++) {
+        if (NB % Q != 0 && q + Q * m >= NB) continue;
         if constexpr (Ns > 1) {
             const int j = q + Q * m;
             const int k = j % Ns;                  // w^r = w_n^{r k}, n = Ns R, r k < n
             constexpr int TWO = tw_sub_offset(L, Ns * R);
             const cx<T> *__restrict__ twn = tw + TWO;
-            if constexpr (Arith<T>::SINGLE) {
+            if constexpr (R == 16) {
+                constexpr int P2 = tw_pow_offset(L, Ns * R, 2), P4 = tw_pow_offset(L, Ns * R, 4), P8 = tw_pow_offset(L, Ns * R, 8);
+                const cx<T> w1 = twn[k];
+                if constexpr (Arith<T>::SINGLE) {
+                    dft16_tw<T, INV>(&v[m * R], w1, tw[P2 + k], tw[P4 + k], tw[P8 + k]);
+                } else {
+                    const cx<T> w2 = cmul(w1, w1), w4 = cmul(w2, w2);
+                    dft16_tw<T, INV>(&v[m * R], w1, w2, w4, cmul(w4, w4));
+                }
+                continue;
+            } else if constexpr (Arith<T>::SINGLE) {
                 cx<T> wp[R];
                 if constexpr (SPNS_F32_TW_POW) {
                     constexpr int P2 = tw_pow_offset(L, Ns * R, 2), P4 = tw_pow_offset(L, Ns * R, 4),
@@ -331,7 +406,7 @@ __device__ __forceinline__ void fft_run(cx<T> (&v)[E], SM sm, int q, const cx<T>
     }
     if constexpr (S + 1 < PL::NST) {
         constexpr int R2 = PL::radix(S + 1);
-        constexpr int MB2 = E / R2;
+        constexpr int NB2 = PL::nb(S + 1), MB2 = PL::mb(S + 1);
         // every reader of the buffer's last contents is done (waited for here, after this
         // stage's arithmetic, rather than right after the reads)
         stage_barrier<WARP>();
@@ -339,6 +414,7 @@ __device__ __forceinline__ void fft_run(cx<T> (&v)[E], SM sm, int q, const cx<T>
             // XOR-swizzled layout (fewer bank conflicts for this exchange)
 #pragma unroll
             for (int m = 0; m < MB; m++) {
+                if (NB % Q != 0 && q + Q * m >= NB) continue;
                 const int j = q + Q * m;
                 const int base = (j / Ns) * Ns * R + (j % Ns);
 #pragma unroll
@@ -347,6 +423,7 @@ __device__ __forceinline__ void fft_run(cx<T> (&v)[E], SM sm, int q, const cx<T>
             stage_barrier<WARP>();
 #pragma unroll
             for (int m = 0; m < MB2; m++) {
+                if (NB2 % Q != 0 && q + Q * m >= NB2) continue;
                 const int j = q + Q * m;
 #pragma unroll
                 for (int r = 0; r < R2; r++) v[m * R2 + r] = sm.xr(j + r * (L / R2));
@@ -357,6 +434,7 @@ __device__ __forceinline__ void fft_run(cx<T> (&v)[E], SM sm, int q, const cx<T>
             cx<T> *const b = sm.base;
 #pragma unroll
             for (int m = 0; m < MB; m++) {
+                if (NB % Q != 0 && q + Q * m >= NB) continue;
                 cx<T> *w;
                 if constexpr (Q % Ns == 0) {
                     w = b + (q / Ns) * XP + (q % Ns) + m * (Q / Ns) * XP;
@@ -372,6 +450,7 @@ __device__ __forceinline__ void fft_run(cx<T> (&v)[E], SM sm, int q, const cx<T>
             static_assert(STEP % X == 0, "exchange read stride must be a multiple of the pad block");
 #pragma unroll
             for (int m = 0; m < MB2; m++) {
+                if (NB2 % Q != 0 && q + Q * m >= NB2) continue;
                 const cx<T> *rd;
                 if constexpr (Q % X == 0) {
                     rd = b + q + (q / X) * PAD + m * (Q + (Q / X) * PAD);
@@ -385,6 +464,7 @@ __device__ __forceinline__ void fft_run(cx<T> (&v)[E], SM sm, int q, const cx<T>
         } else {
 #pragma unroll
             for (int m = 0; m < MB; m++) {
+                if (NB % Q != 0 && q + Q * m >= NB) continue;
                 const int j = q + Q * m;
                 const int base = (j / Ns) * Ns * R + (j % Ns);
 #pragma unroll
@@ -393,6 +473,7 @@ __device__ __forceinline__ void fft_run(cx<T> (&v)[E], SM sm, int q, const cx<T>
             stage_barrier<WARP>();
 #pragma unroll
             for (int m = 0; m < MB2; m++) {
+                if (NB2 % Q != 0 && q + Q * m >= NB2) continue;
                 const int j = q + Q * m;
 #pragma unroll
                 for (int r = 0; r < R2; r++) v[m * R2 + r] = sm.at(j + r * (L / R2));
@@ -430,7 +511,17 @@ __device__ __forceinline__ int opaque(int q) {
 // pencil-major thread layout).
 template <typename T, int L, int E, bool INV, class SM, unsigned WARP = 0>
 __device__ __forceinline__ void fft(cx<T> (&v)[E], SM sm, int q, const cx<T> *__restrict__ tw) {
-    fft_run<T, L, E, INV, WARP, 0, SM>(v, sm, opaque(q), tw);
+    constexpr int V = Plan<L, E, INV, uneven_plan<SM, L, E>()>::width();
+    if constexpr (V == E) {
+        fft_run<T, L, E, INV, WARP, 0, SM>(v, sm, opaque(q), tw);
+    } else {
+        cx<T> x[V];
+#pragma unroll
+        for (int e = 0; e < E; e++) x[e] = v[e];
+        fft_run<T, L, E, INV, WARP, 0, SM>(x, sm, opaque(q), tw);
+#pragma unroll
+        for (int e = 0; e < E; e++) v[e] = x[e];
+    }
 }
 
 // Accessor: tile of P pencils stored row-major [row][P] (pencil index fastest).

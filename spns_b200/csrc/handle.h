@@ -113,7 +113,15 @@ template <typename T> struct ShapeSel {
     static constexpr int Z_E = D ? SPNS_Z_E : SPNS_F32_Z_E, Z_T = D ? SPNS_Z_THREADS : SPNS_F32_Z_T;
     static constexpr bool Z_STAGE = D ? SPNS_Z_STAGE : SPNS_F32_Z_STAGE;
 };
-template <typename T, int L> using ShapeK1 = ShapeT<T, L, ShapeSel<T>::K1_E, ShapeSel<T>::K1_T>;   // inverse x
+// Inverse x pass: from length 384 on 24 values per thread (one exchange less; a 128-byte or
+// 64-byte row tile) where that is faster than 12: single precision N=512 2.81 -> 2.27 ms,
+// N=256 0.31 -> 0.28 (N=128 0.048 -> 0.058); double N=256 0.56 -> 0.52, while at 768 12 values
+// with the uneven plan take 4.14 ms and 24 values 4.72.
+template <typename T, int L> struct ShapeK1Sel {
+    static constexpr bool D = ShapeSel<T>::D, WIDE = L >= 384 && (!D || L == 384);
+    static constexpr int E = WIDE ? 24 : ShapeSel<T>::K1_E, THR = WIDE && D ? 128 : ShapeSel<T>::K1_T;
+};
+template <typename T, int L> using ShapeK1 = ShapeT<T, L, ShapeK1Sel<T, L>::E, ShapeK1Sel<T, L>::THR>;   // inverse x
 template <typename T, int L> using ShapeK2 = ShapeT<T, L, ShapeSel<T>::K2_E, ShapeSel<T>::K2_T>;   // inverse y (and forward y)
 template <typename T, int L> using ShapeK5 = ShapeT<T, L, ShapeSel<T>::K5_E, ShapeSel<T>::K5_T>;   // forward x
 template <typename T, int L> using Shape = ShapeT<T, L, 24, 128>;                                   // edge planes, test lines
