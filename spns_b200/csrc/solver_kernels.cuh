@@ -168,6 +168,34 @@ __device__ __forceinline__ double col_k(int s, int kz, double *) { return (doubl
 __device__ __forceinline__ float col_k(int s, int kz, float *) { return (float)(s * kz); }
 __device__ __forceinline__ f2 col_k(int s, int kz, f2 *) { return f2((float)(s * kz), (float)(s * kz + s)); }
 
+// The x/y passes wait on the loads of a field with nothing else in flight, so while it is
+// transformed the rows of the block's next field are asked for in L2.  addr(e): the tile's
+// first element in the thread's row e (null: no row); the P threads of a row share its E lines.
+// Without and with, in ms, rotational form, double / single:
+//   N=256  K1 0.516 -> 0.450 / 0.276 -> 0.251     K2 0.915 -> 0.648 / 0.483 -> 0.389
+//          K4 0.324 -> 0.301 / 0.190 -> 0.170     K5 0.223 -> 0.201 / 0.129 -> 0.137
+//   N=512  K1 4.13 -> 4.00 / 2.27 -> 2.21         K2 5.75 -> 5.71 / 2.97 -> 3.01
+//          K4 2.63 -> 2.70 / 1.27 -> 1.43         K5 1.80 -> 1.84 / 1.17 -> 1.22
+// From length 768 on the current and the next tiles of all resident blocks (100 KB each, 58 MB
+// together) with their output do not stay in the near half of L2 until they are used: there K2
+// (input rows below the cut-off only) asks after the transform, before the stores (5.58 /
+// 2.89), and K4 and K5 not at all (K4 so 2.72 / 1.36).  The LES passes write more per read and
+// their forward ones have three blocks per SM to cover each other's loads: K2 0.952 -> 0.977 / 0.672 ->
+// 0.576 (on in single precision), K4 1.04 -> 1.17 / 0.61 -> 0.63, K5 0.56 -> 0.65 / 0.34 -> 0.40.
+template <int L> constexpr bool PREFETCH_LATE = L >= 768;
+template <typename T, int MODE> constexpr bool PREFETCH_2 = MODE != MODE_LES || Arith<T>::SINGLE;
+template <int L, int MODE> constexpr bool PREFETCH_4 = L < 768 && MODE != MODE_LES;
+template <typename T, int L, int MODE> constexpr bool PREFETCH_5 = L < 768 && MODE != MODE_LES && !Arith<T>::SINGLE;
+template <int E, int P, class Addr> __device__ __forceinline__ void prefetch_rows(int p, Addr addr) {
+#pragma unroll
+    for (int i = 0; i < (E + P - 1) / P; i++) {
+        const int e = i * P + p;
+        if (E % P != 0 && e >= E) break;
+        const void *a = addr(e);
+        if (a) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(a));
+    }
+}
+
 // ===========================================================================
 // K1: inverse transform along x.  Block = (kz chunk, iy).
 //   VEL: u,v,w   ROT: u,v,w and the vorticity   ADV/LES: u,v,w, du/dx, dv/dx, dw/dx
@@ -204,6 +232,17 @@ __device__ __forceinline__ void k1_inv_x_body(Geo g, const SCx<T> *__restrict__ 
             for (int e = 0; e < E; e++) r[e] = T(g.sx * ffreq(in_row<L, E, true>(q, e), L)) * r[e];
         }
     };
+    // the first column of each row; a compact row's tile may end in the next line
+    auto prefetch = [&](const SCx<T> *src) {
+        const int last = (g.Kz - (kz - p * Arith<T>::W) < P * Arith<T>::W ? g.Kz - (kz - p * Arith<T>::W) : P * Arith<T>::W) - 1;
+        prefetch_rows<E, P>(p, [&](int e) -> const void * {
+            const int m1 = ffreq(in_row<L, E, true>(q, e), L);
+            if (m1 > g.hx || m1 < -g.hx) return nullptr;
+            const SCx<T> *a = src + (rb - p * Arith<T>::W) + (long long)(m1 >= 0 ? m1 : m1 + g.Kx) * g.Kz;
+            asm volatile("prefetch.global.L2 [%0];\n" ::"l"(a + last));
+            return a;
+        });
+    };
     auto put = [&](int f, auto value) {
         if (!ok) return;
         SCx<T> *o = out + (long long)f * g.S1 + ob;
@@ -234,6 +273,7 @@ __device__ __forceinline__ void k1_inv_x_body(Geo g, const SCx<T> *__restrict__ 
         for (int s = 0; s < 5; s++) {
             cx<T> r[E];
             load(r, s == 2 ? u : (s == 0 || s == 4) ? v : w, s >= 3);
+            if (s < 2) prefetch(s == 0 ? w : u);
             fft<T, L, E, true>(r, sm, q, tw);
             if (s < 3) put(s == 0 ? 1 : s == 1 ? 2 : 0, [&](int e) { return r[e]; });
             if (s == 1) put(3, [&](int e) { return mul_i(kyf * r[e] - kzf * slot[e * THREADS]); });
@@ -249,6 +289,7 @@ __device__ __forceinline__ void k1_inv_x_body(Geo g, const SCx<T> *__restrict__ 
         for (int f = f0; f < Fields<MODE>::K1; f += fs) {
             cx<T> r[E];
             load(r, f % 3 == 0 ? u : f % 3 == 1 ? v : w, f >= 3);
+            if (f + fs < 3) prefetch(f + fs == 1 ? v : w);
             fft<T, L, E, true>(r, sm, q, tw);
             if (f < 3) put(f, [&](int e) { return r[e]; });
             else put(f, [&](int e) { return mul_i(r[e]); });
@@ -272,22 +313,37 @@ __device__ __forceinline__ void k2_inv_y_body(Geo g, const SCx<T> *__restrict__ 
     // row offsets in 32 bits (a field has fewer than 2^31 elements at every compiled length):
     // one register and one multiply-add per address instead of a 64-bit chain
     const unsigned col = (unsigned)x * g.Kp + kz, rs = (unsigned)g.Mx * g.Kp;
+    // Nine fields: d/dy of u, v, w follow right after their own transforms, whose input is
+    // then still in L2 (u, d/dy u, v, ..., then the x derivatives).
+    constexpr bool DERIV = Fields<MODE>::K2 == 9;
+    auto field = [](int i) { return !DERIV ? i : i >= 6 ? i - 3 : i & 1 ? 6 + i / 2 : i / 2; };
+    auto source = [](int f) { return f >= 6 ? f - 6 : f; };
 #pragma unroll 1
-    for (int f = f0; f < Fields<MODE>::K2; f += fs) {
-        const int q = opaque(q0);
+    for (int i = f0; i < Fields<MODE>::K2; i += fs) {
+        const int q = opaque(q0), f = field(i);
         cx<T> r[E];
-        const bool deriv = (MODE == MODE_ADV || MODE == MODE_LES || MODE == MODE_INV) && f >= 6;
-        const SCx<T> *F = in + (long long)(deriv ? f - 6 : f) * g.S1;
+        const bool deriv = f >= 6;
+        const SCx<T> *F = in + (long long)source(f) * g.S1;
 #pragma unroll
         for (int e = 0; e < E; e++) {
             const int m2 = ffreq(in_row<L, E, true>(q, e), L);
             r[e] = (ok && m2 <= g.hy && m2 >= -g.hy) ? ld_work(F + (col + (unsigned)(m2 >= 0 ? m2 : m2 + g.Ky) * rs), (cx<T> *)nullptr) : zero<T>();
         }
+        auto prefetch = [&] {
+            if (!PREFETCH_2<T, MODE> || i + fs >= Fields<MODE>::K2 || source(field(i + fs)) == source(f)) return;
+            const SCx<T> *N = in + (long long)source(field(i + fs)) * g.S1;
+            prefetch_rows<E, P>(p, [&](int e) -> const void * {
+                const int m2 = ffreq(in_row<L, E, true>(q, e), L);
+                return m2 <= g.hy && m2 >= -g.hy ? N + (col - p * Arith<T>::W + (unsigned)(m2 >= 0 ? m2 : m2 + g.Ky) * rs) : nullptr;
+            });
+        };
+        if constexpr (!PREFETCH_LATE<L>) prefetch();
         if (deriv) {
 #pragma unroll
             for (int e = 0; e < E; e++) r[e] = mul_i(T(g.sy * ffreq(in_row<L, E, true>(q, e), L)) * r[e]);
         }
         fft<T, L, E, true>(r, sm, q, tw);
+        if constexpr (PREFETCH_LATE<L>) prefetch();
         if (ok) {
             SCx<T> *o = out + (long long)f * g.S2;
 #pragma unroll
@@ -635,11 +691,16 @@ __device__ __forceinline__ void k4_fwd_y_body(Geo g, const SCx<T> *__restrict__ 
     //       out (S1): 0 G_x + i ky t12, 1 G_y + i ky t22, 2 G_z + i ky t23, 3 t11, 4 t12, 5 t13
     // Groups: (t12, G_x), (t22, G_y), (t23, G_z), then t11 and t13 alone.
     constexpr int NG = LES ? 5 : Fields<MODE>::NOUT;
-    auto load_fft = [&](cx<T>(&r)[E], int f) {
+    // (next: the field read after this one, -1 for none)
+    auto load_fft = [&](cx<T>(&r)[E], int f, int next) {
         const int q = opaque(q0);
         const SCx<T> *src = in + (long long)f * g.S2;
 #pragma unroll
         for (int e = 0; e < E; e++) r[e] = ok ? ld_work(src + (col + (unsigned)in_row<L, E, false>(q, e) * rs), (cx<T> *)nullptr) : zero<T>();
+        if (PREFETCH_4<L, MODE> && next >= 0) {
+            const SCx<T> *N = in + (long long)next * g.S2;
+            prefetch_rows<E, P>(p, [&](int e) -> const void * { return N + (col - p * Arith<T>::W + (unsigned)in_row<L, E, false>(q, e) * rs); });
+        }
         fft<T, L, E, false>(r, sm, q, tw);
     };
     auto store = [&](int f, auto value) {
@@ -652,18 +713,20 @@ __device__ __forceinline__ void k4_fwd_y_body(Geo g, const SCx<T> *__restrict__ 
             if (m2 <= g.hy && m2 >= -g.hy) st_work(o + (col + (unsigned)(m2 >= 0 ? m2 : m2 + g.Ky) * rs), value(e, m2));
         }
     };
+    // first field of a group
+    auto first = [&](int grp) { return grp >= NG ? -1 : !LES ? k4_in_field<MODE>(grp) : grp == 0 ? 4 : grp >= 3 ? 2 * grp - 3 : grp + 5; };
 #pragma unroll 1
     for (int grp = f0; grp < NG; grp += fs) {
         cx<T> r[E];
         if (!LES || grp >= 3) {
-            const int f = !LES ? k4_in_field<MODE>(grp) : 2 * grp - 3;
-            load_fft(r, f);
+            const int f = first(grp);
+            load_fft(r, f, first(grp + fs));
             store(LES ? f : grp, [&](int e, int) { return r[e]; });
         } else {
             cx<T> t[E];
-            load_fft(t, grp == 0 ? 4 : grp + 5);
+            load_fft(t, first(grp), grp);
             if (grp == 0) store(4, [&](int e, int) { return t[e]; });
-            load_fft(r, grp);
+            load_fft(r, grp, first(grp + fs));
             store(grp, [&](int e, int m2) { return r[e] + mul_i(T(g.sy * m2) * t[e]); });
         }
     }
@@ -683,17 +746,22 @@ __device__ __forceinline__ void k5_fwd_x_body(Geo g, const SCx<T> *__restrict__ 
     SmRowMajor<T, P> sm{reinterpret_cast<cx<T> *>(smraw), p};
     const long long col = (long long)iy * g.Mx * g.Kp + kz;
     constexpr bool LES = MODE == MODE_LES;
-    auto load_fft = [&](cx<T>(&r)[E], int f) {
+    auto load_fft = [&](cx<T>(&r)[E], int f, int next) {
         const SCx<T> *src = in + (long long)f * g.S1 + col;
 #pragma unroll
         for (int e = 0; e < E; e++) r[e] = ok ? ld_work(src + (long long)in_row<L, E, false>(q, e) * g.Kp, (cx<T> *)nullptr) : zero<T>();
+        if (PREFETCH_5<T, L, MODE> && next >= 0) {
+            const SCx<T> *N = in + (long long)next * g.S1 + (col - p * Arith<T>::W);
+            prefetch_rows<E, P>(p, [&](int e) -> const void * { return N + (long long)in_row<L, E, false>(q, e) * g.Kp; });
+        }
         fft<T, L, E, false>(r, sm, q, tw);
     };
 #pragma unroll 1
     for (int f = f0; f < Fields<MODE>::NOUT; f += fs) {
         cx<T> r[E], t[LES ? E : 1];
-        load_fft(r, f);
-        if constexpr (LES) load_fft(t, 3 + f);   // t11, t12, t13
+        const int next = f + fs < Fields<MODE>::NOUT ? f + fs : -1;
+        load_fft(r, f, LES ? 3 + f : next);
+        if constexpr (LES) load_fft(t, 3 + f, next);   // t11, t12, t13
         if (!ok) continue;
         SCx<T> *o = G + (long long)f * g.S0 + (long long)iy * g.Kx * g.Kz + kz;
 #pragma unroll
