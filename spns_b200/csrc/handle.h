@@ -138,26 +138,16 @@ template <int L, int MODE> constexpr bool shape_alt_ok() {
 }
 // Forward passes of the LES form hold two arrays of values per thread (G_i and the stress
 // folded into it).
-#ifndef SPNS_LES_E
-#define SPNS_LES_E 12
-#endif
-#ifndef SPNS_LES_T4
-#define SPNS_LES_T4 128
-#endif
-#ifndef SPNS_LES_T5
-#define SPNS_LES_T5 128
-#endif
+constexpr int SPNS_LES_E = 12, SPNS_LES_T = 128;
 template <typename T, int L, int ALT> using ShapeK1A = typename std::conditional<ALT != 0, ShapeT<T, L, SPNS_ALT_E, ShapeSel<T>::K1_T>, ShapeK1<T, L>>::type;
 template <typename T, int L, int ALT> using ShapeK2A = typename std::conditional<ALT != 0, ShapeT<T, L, SPNS_ALT_E, ShapeSel<T>::K2_T>, ShapeK2<T, L>>::type;
 template <typename T, int L, int MODE, int ALT> using ShapeK4A =
-    typename std::conditional<ALT != 0 || MODE != spns::MODE_LES, ShapeK2A<T, L, ALT>, ShapeT<T, L, SPNS_LES_E, SPNS_LES_T4>>::type;
+    typename std::conditional<ALT != 0 || MODE != spns::MODE_LES, ShapeK2A<T, L, ALT>, ShapeT<T, L, SPNS_LES_E, SPNS_LES_T>>::type;
 template <typename T, int L, int MODE, int ALT> using ShapeK5A =
     typename std::conditional<ALT != 0, ShapeT<T, L, SPNS_ALT_E, ShapeSel<T>::K5_T>,
-                              typename std::conditional<MODE != spns::MODE_LES, ShapeK5<T, L>, ShapeT<T, L, SPNS_LES_E, SPNS_LES_T5>>::type>::type;
+                              typename std::conditional<MODE != spns::MODE_LES, ShapeK5<T, L>, ShapeT<T, L, SPNS_LES_E, SPNS_LES_T>>::type>::type;
 
-#ifndef SPNS_SPLIT_WAVES
-#define SPNS_SPLIT_WAVES 4       // x/y passes with fewer than 4 blocks per SM spread their fields over blocks
-#endif
+constexpr int SPNS_SPLIT_WAVES = 4;   // x/y passes with fewer than 4 blocks per SM spread their fields over blocks
 // Rotational z pass with pair-by-pair bulk-copy staging and slots in tensor memory
 // (k3_rot_staged, zpass_staged.cuh): lengths whose pencils, at 12 values per thread, are a
 // part of a warp, one or two warps; k3_z runs the others.
@@ -184,39 +174,8 @@ template <typename T, int L, int ALT = 0> struct Shape3 {
 // z pass with the fields transformed side by side (k3_field, zpass_field.cuh).  E values
 // per thread, NT teams of Q = L/E threads (a whole number of warps), PB pencils per block,
 // and the register budget that sets the resident blocks.
-#ifndef SPNS_ZF_E_LONG
-#define SPNS_ZF_E_LONG 12
-#endif
-#ifndef SPNS_ZF_R24
-#define SPNS_ZF_R24 168
-#endif
-#ifndef SPNS_ZF_R12
-#define SPNS_ZF_R12 84
-#endif
-#ifndef SPNS_ZF_R6
-#define SPNS_ZF_R6 80
-#endif
-#ifndef SPNS_F32_ZF_E_LONG
-#define SPNS_F32_ZF_E_LONG 12
-#endif
-#ifndef SPNS_ZF_E144
-#define SPNS_ZF_E144 12
-#endif
-#ifndef SPNS_F32_ZF_R24
-#define SPNS_F32_ZF_R24 104
-#endif
-#ifndef SPNS_F32_ZF_R12
-#define SPNS_F32_ZF_R12 80
-#endif
-#ifndef SPNS_F32_ZF_R6
-#define SPNS_F32_ZF_R6 64
-#endif
-#ifndef SPNS_ZF_ROT
-#define SPNS_ZF_ROT 0
-#endif
 template <typename T, int L, int MODE, int ALT = 0> struct ZFieldShape {
-    static constexpr bool D = sizeof(T) == 8;
-    static constexpr int E = ALT ? SPNS_ALT_E : L >= 768 ? 24 : L == 384 ? (D ? SPNS_ZF_E_LONG : SPNS_F32_ZF_E_LONG) : L == 144 ? SPNS_ZF_E144 : 12;
+    static constexpr int E = ALT ? SPNS_ALT_E : L >= 768 ? 24 : 12;
     static constexpr int Q = L / E;
     static constexpr int NPAIR = spns::ZFieldForm<MODE>::NPAIR;
     static constexpr bool INV = MODE == spns::MODE_INV;
@@ -227,7 +186,7 @@ template <typename T, int L, int MODE, int ALT = 0> struct ZFieldShape {
     static constexpr int PB = lcm(NT, NPAIR) / NPAIR;
     using LY = spns::ZFieldLayout<T, L, E, PB, NT, MODE>;
     static constexpr int THREADS = LY::THREADS;
-    static constexpr int REGS = E == 24 ? (D ? SPNS_ZF_R24 : SPNS_F32_ZF_R24) : E == 12 ? (D ? SPNS_ZF_R12 : SPNS_F32_ZF_R12) : (D ? SPNS_ZF_R6 : SPNS_F32_ZF_R6);
+    static constexpr int REGS = E == 24 ? 168 : E == 12 ? 84 : 80;   // (T = f2: values of 64 bits too)
     static constexpr int B0 = 65536 / (REGS * THREADS);
     static constexpr int MINB = B0 < 1 ? 1 : B0;
     static_assert(THREADS % 32 == 0 && LY::SMEM <= 227 * 1024, "whole warps and at most 227 KB of shared memory");

@@ -88,8 +88,9 @@ template <typename T> struct LenLaunch {
     template <int L, int MODE, int ALT = 0> static cudaError_t launch_k3(spns_handle *h, double *phys) {
         if constexpr (MODE != spns::MODE_VEL && MODE != spns::MODE_ROT) {
             return launch_k3_field<L, MODE, ALT>(h, phys);
+        } else if constexpr (MODE == spns::MODE_ROT && ALT == 0 && spns_zstaged_length<T>(L)) {
+            return launch_k3_staged<L>(h);
         } else {
-        if constexpr (MODE == spns::MODE_ROT && ALT == 0 && spns_zstaged_length<T>(L)) return launch_k3_staged<L>(h);
         using S3 = Shape3<T, L, ALT>;
         constexpr bool STAGE = MODE == spns::MODE_ROT && ShapeSel<T>::Z_STAGE;
         auto kern = spns::k3_z<T, L, S3::E, S3::P, MODE, STAGE>;

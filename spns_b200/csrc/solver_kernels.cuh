@@ -106,11 +106,12 @@ __device__ __forceinline__ int ffreq(int a, int M) { return a <= M / 2 ? a : a -
 #ifndef SPNS_F32_AX_MINB
 #define SPNS_F32_AX_MINB 2
 #endif
-#ifndef SPNS_LES_MINB
-#define SPNS_LES_MINB 3
-#endif
-template <typename T, int PASS, int MODE> struct AxisMinBlocks {
-    static constexpr int N = MODE == 3 /* LES */ && PASS >= 4 ? SPNS_LES_MINB : sizeof(T) == 8 ? ((PASS == 2 || PASS == 4) ? SPNS_K2_MINB : PASS == 1 ? SPNS_K1_MINB : SPNS_K5_MINB)
+// The LES forward passes hold two arrays of 12 values per thread: three blocks of 128 threads.
+// Blocks of 256 threads (length 768), LES N=512, double / single: y two blocks 10.0 / 5.2 ms, one 11.0 /
+// 5.5; x two 5.1 / 3.0, one 4.0 / 2.65.
+template <typename T, int PASS, int MODE, int THREADS> struct AxisMinBlocks {
+    static constexpr int N = MODE == 3 /* LES */ && PASS >= 4 ? (THREADS <= 128 ? 3 : THREADS <= 256 && PASS == 4 ? 2 : 1)
+                             : sizeof(T) == 8 ? ((PASS == 2 || PASS == 4) ? SPNS_K2_MINB : PASS == 1 ? SPNS_K1_MINB : SPNS_K5_MINB)
                                             : SPNS_F32_AX_MINB;
 };
 
@@ -1371,14 +1372,14 @@ static __global__ void k_dft_axis(const double2 *__restrict__ in, double2 *__res
 // come from a device table (BatchMember).  The arithmetic is the one-box kernel's.
 // ===========================================================================
 template <typename T, int L, int E, int P, int MODE>
-__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 1, MODE>::N) k1_inv_x(Geo g, const SCx<T> *__restrict__ u, const SCx<T> *__restrict__ v,
+__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 1, MODE, P *(L / E)>::N) k1_inv_x(Geo g, const SCx<T> *__restrict__ u, const SCx<T> *__restrict__ v,
                                                                            const SCx<T> *__restrict__ w, SCx<T> *__restrict__ out,
                                                                            const cx<T> *__restrict__ tw, DevScalars *reset) {
     if (blockIdx.z == 0) reset_maxima(reset);
     k1_inv_x_body<T, L, E, P, MODE>(g, u, v, w, out, tw, blockIdx.z, gridDim.z);
 }
 template <typename T, int L, int E, int P, int MODE>
-__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 2, MODE>::N) k2_inv_y(Geo g, const SCx<T> *__restrict__ in, SCx<T> *__restrict__ out,
+__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 2, MODE, P *(L / E)>::N) k2_inv_y(Geo g, const SCx<T> *__restrict__ in, SCx<T> *__restrict__ out,
                                                                            const cx<T> *__restrict__ tw) {
     k2_inv_y_body<T, L, E, P, MODE>(g, in, out, tw, blockIdx.z, gridDim.z);
 }
@@ -1389,12 +1390,12 @@ __global__ void __launch_bounds__(P *(L / E), K3MinBlocks<T, P *(L / E)>::N) k3_
     k3_z_body<T, L, E, P, MODE, STAGE>(g, buf, c, ds, phys, tw);
 }
 template <typename T, int L, int E, int P, int MODE>
-__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 4, MODE>::N) k4_fwd_y(Geo g, const SCx<T> *__restrict__ in, SCx<T> *__restrict__ out,
+__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 4, MODE, P *(L / E)>::N) k4_fwd_y(Geo g, const SCx<T> *__restrict__ in, SCx<T> *__restrict__ out,
                                                                            const cx<T> *__restrict__ tw) {
     k4_fwd_y_body<T, L, E, P, MODE>(g, in, out, tw, blockIdx.z, gridDim.z);
 }
 template <typename T, int L, int E, int P, int MODE>
-__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 5, MODE>::N) k5_fwd_x(Geo g, const SCx<T> *__restrict__ in, SCx<T> *__restrict__ G,
+__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 5, MODE, P *(L / E)>::N) k5_fwd_x(Geo g, const SCx<T> *__restrict__ in, SCx<T> *__restrict__ G,
                                                                            const cx<T> *__restrict__ tw) {
     k5_fwd_x_body<T, L, E, P, MODE>(g, in, G, tw, blockIdx.z, gridDim.z);
 }
@@ -1414,7 +1415,7 @@ struct BatchMember {
     StepConsts c;
 };
 template <typename T, int L, int E, int P, int MODE>
-__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 1, MODE>::N) k1_inv_x_batch(Geo g, const BatchMember *__restrict__ tab,
+__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 1, MODE, P *(L / E)>::N) k1_inv_x_batch(Geo g, const BatchMember *__restrict__ tab,
                                                                                  const cx<T> *__restrict__ tw) {
     const BatchMember &m = tab[blockIdx.z];
     reset_maxima(m.ds);
@@ -1422,19 +1423,19 @@ __global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 1, MODE>::N) k1_i
     k1_inv_x_body<T, L, E, P, MODE>(g, U, U + g.S0, U + 2 * g.S0, static_cast<SCx<T> *>(m.B1), tw, 0, 1);
 }
 template <typename T, int L, int E, int P, int MODE>
-__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 2, MODE>::N) k2_inv_y_batch(Geo g, const BatchMember *__restrict__ tab,
+__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 2, MODE, P *(L / E)>::N) k2_inv_y_batch(Geo g, const BatchMember *__restrict__ tab,
                                                                                  const cx<T> *__restrict__ tw) {
     const BatchMember &m = tab[blockIdx.z];
     k2_inv_y_body<T, L, E, P, MODE>(g, static_cast<const SCx<T> *>(m.B1), static_cast<SCx<T> *>(m.B2), tw, 0, 1);
 }
 template <typename T, int L, int E, int P, int MODE>
-__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 4, MODE>::N) k4_fwd_y_batch(Geo g, const BatchMember *__restrict__ tab,
+__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 4, MODE, P *(L / E)>::N) k4_fwd_y_batch(Geo g, const BatchMember *__restrict__ tab,
                                                                                  const cx<T> *__restrict__ tw) {
     const BatchMember &m = tab[blockIdx.z];
     k4_fwd_y_body<T, L, E, P, MODE>(g, static_cast<const SCx<T> *>(m.B2), static_cast<SCx<T> *>(m.B1), tw, 0, 1);
 }
 template <typename T, int L, int E, int P, int MODE>
-__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 5, MODE>::N) k5_fwd_x_batch(Geo g, const BatchMember *__restrict__ tab,
+__global__ void __launch_bounds__(P *(L / E), AxisMinBlocks<T, 5, MODE, P *(L / E)>::N) k5_fwd_x_batch(Geo g, const BatchMember *__restrict__ tab,
                                                                                  const cx<T> *__restrict__ tw) {
     const BatchMember &m = tab[blockIdx.z];
     k5_fwd_x_body<T, L, E, P, MODE>(g, static_cast<const SCx<T> *>(m.B1), static_cast<SCx<T> *>(m.B2), tw, 0, 1);

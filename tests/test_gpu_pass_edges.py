@@ -90,3 +90,26 @@ def test_ensemble_names_the_member_that_failed():
     ens.close()
     for h in members:
         h.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_rotational_members_side_by_side(precision):
+    """The persistent z pass takes an SM's tensor memory whole: boxes stepped concurrently, on
+    streams of one ensemble, reach bit for bit the states they reach alone."""
+    from spns_b200.hit import HIT, Ensemble
+    members, alone = [], []
+    for i, N in enumerate([(64, 64, 64), (64, 32, 128), (32, 32, 128), (64, 64, 64)]):
+        args = make_args(0, nu=2e-3, Ns=N)
+        h = HIT(args, precision=precision, k41_ranks=-1)
+        h.seed_field(40 + i, 3.0)
+        a = HIT(args, precision=precision, k41_ranks=-1)
+        a.checkpoint_load(h.checkpoint_save())
+        members.append(h)
+        alone.append(a)
+    for a in alone:
+        a.New_Fractional_Step_Method(4)
+    ens = Ensemble(members)
+    ens.step(4)
+    for h, a in zip(members, alone):
+        assert np.array_equal(h.get_compact(), a.get_compact())
+    ens.close()
