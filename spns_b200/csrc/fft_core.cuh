@@ -312,14 +312,15 @@ __host__ __device__ constexpr int tw_pow_offset(int L, int n, int r) {
 }
 __host__ __device__ constexpr int tw_full_size(int L) { return 4 * tw_table_size(L); }
 
-// Barrier of an exchange: the block's (WARP 0), the whole warp's (1), that of the two warps
-// of an aligned group of 64 threads (GROUP64: named barrier 1 + group), or that of the lanes
-// of the mask WARP, the only ones that run the transform.
-constexpr unsigned GROUP64 = 0x40000000u;
+// Barrier of an exchange: the block's (WARP 0), the whole warp's (1), that of the warps of an
+// aligned group of 64, 96 or 128 threads (GROUP + threads: named barrier 1 + group), or that of the
+// lanes of the mask WARP, the only ones that run the transform.
+constexpr unsigned GROUP = 0x40000000u;
 template <unsigned WARP> __device__ __forceinline__ void stage_barrier() {
     if constexpr (WARP == 0) __syncthreads();
     else if constexpr (WARP == 1) __syncwarp();
-    else if constexpr (WARP == GROUP64) asm volatile("bar.sync %0, 64;\n" ::"r"(1 + (threadIdx.x >> 6)) : "memory");
+    else if constexpr (WARP == GROUP + 64 || WARP == GROUP + 96 || WARP == GROUP + 128)
+        asm volatile("bar.sync %0, %1;\n" ::"r"(1 + threadIdx.x / (WARP - GROUP)), "n"(WARP - GROUP) : "memory");
     else __syncwarp(WARP);
 }
 

@@ -149,12 +149,14 @@ template <typename T, int L, int MODE, int ALT> using ShapeK5A =
 
 constexpr int SPNS_SPLIT_WAVES = 4;   // x/y passes with fewer than 4 blocks per SM spread their fields over blocks
 // Rotational z pass with pair-by-pair bulk-copy staging and slots in tensor memory
-// (k3_rot_staged, zpass_staged.cuh): lengths whose pencils, at 12 values per thread, are a
-// part of a warp, one or two warps; k3_z runs the others.
-// Staged against k3_z: double 768 11.5 against 14.9 ms (N=512), 192 0.175 against 0.199 (N=128),
-// 96 0.031 against 0.034 (N=64), 48 0.018 against 0.015 (N=32); single 192 0.121 against 0.125,
-// 96 0.027 against 0.021: short pencils leave too few values per staged pair.
-template <typename T> constexpr bool spns_zstaged_length(int L) { return L == 768 || L == 384 || L == 192 || (L == 96 && sizeof(T) == 8); }
+// (k3_rot_staged, zpass_staged.cuh): lengths whose pencils, at 12 values per thread, fill one
+// to four warps, in boxes with enough of them (LenLaunch::staged_pays); k3_z runs the others.
+// Staged against k3_z: double 768 11.5 against 14.9 ms (N=512), 288 0.634 against 0.809 (N=192),
+// 192 0.158 against 0.199 (N=128), 144 0.076 against 0.090 (N=96), 96 0.029 against 0.033 (N=64);
+// 1536 2.01 against 2.09 (192 x 192 pencils); single 288 0.371 against 0.460, 192 0.111 against 0.125,
+// 1536 1.17 against 1.39; 48 double 0.018 against 0.015, single 96 0.022 against 0.023, 48 0.023 against
+// 0.014: short pencils leave too few values per staged pair.
+template <typename T> constexpr bool spns_zstaged_length(int L) { return L >= 192 || ((L == 144 || L == 96) && sizeof(T) == 8); }
 constexpr int SPNS_ZS_E = 12;
 
 // Velocity and short-length rotational z pass (k3_z): pencils per block limited by the

@@ -51,13 +51,28 @@ template <typename T> struct LenLaunch {
         return cudaGetLastError();
     }
     // Rotational z pass staged pair by pair with bulk copies (zpass_staged.cuh),
-    // persistent: one block per SM.
+    // persistent: one block per SM.  Units of the box, and units the SMs hold in one round.
+    template <int L> static long long staged_units(const spns_handle *h) {
+        using LY = spns::ZStagedLayout<A, L, SPNS_ZS_E>;
+        return (long long)h->g.Mx * h->g.My / (LY::PPU * LY::W);
+    }
+    template <int L> static long long staged_round(const spns_handle *h) {
+        return (long long)spns::ZStagedLayout<A, L, SPNS_ZS_E>::max_units(h->g.Kz, h->g.Kp) * h->sms;
+    }
+    // A unit's pairs follow one another, so the pass needs rounds to overlap: against k3_z, whose
+    // blocks copy all six fields at their start, it is faster from half a round in double
+    // precision (0.24..0.49 rounds, 48 x 48 pencils of 96..192: 0.020..0.023 against 0.016..0.019 ms;
+    // 0.55, 72 x 72 of 96: 0.023 against 0.029) and from three in single precision (3.5, 144 x 144 of
+    // 288: 0.115 against 0.125; 3.9, 192^3: 0.111 against 0.125; 2.2, 144 x 144 of 192: 0.086 against 0.076).
+    template <int L> static bool staged_pays(const spns_handle *h) {
+        return sizeof(T) == 8 ? 2 * staged_units<L>(h) >= staged_round<L>(h) : staged_units<L>(h) >= 3 * staged_round<L>(h);
+    }
     template <int L> static cudaError_t launch_k3_staged(spns_handle *h) {
         using LY = spns::ZStagedLayout<A, L, SPNS_ZS_E>;
         auto kern = spns::k3_rot_staged<A, L, SPNS_ZS_E>;
-        const long long ngrp = (long long)h->g.Mx * h->g.My / (LY::PPU * LY::W);
-        // as many units as a block holds, or as it takes to spread the pencils over the SMs
-        const int units = (int)std::min<long long>(LY::max_units(h->g.Kz, h->g.Kp), (ngrp + h->sms - 1) / h->sms);
+        const long long ngrp = staged_units<L>(h), per_round = staged_round<L>(h), rounds = (ngrp + per_round - 1) / per_round;
+        // as many units as spread the pencils evenly over the rounds
+        const int units = (int)((ngrp + rounds * h->sms - 1) / (rounds * h->sms));
         const size_t smem = LY::smem_bytes(units, h->g.Kz, h->g.Kp);
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
@@ -88,9 +103,9 @@ template <typename T> struct LenLaunch {
     template <int L, int MODE, int ALT = 0> static cudaError_t launch_k3(spns_handle *h, double *phys) {
         if constexpr (MODE != spns::MODE_VEL && MODE != spns::MODE_ROT) {
             return launch_k3_field<L, MODE, ALT>(h, phys);
-        } else if constexpr (MODE == spns::MODE_ROT && ALT == 0 && spns_zstaged_length<T>(L)) {
-            return launch_k3_staged<L>(h);
         } else {
+        if constexpr (MODE == spns::MODE_ROT && ALT == 0 && spns_zstaged_length<T>(L))
+            if (staged_pays<L>(h)) return launch_k3_staged<L>(h);
         using S3 = Shape3<T, L, ALT>;
         constexpr bool STAGE = MODE == spns::MODE_ROT && ShapeSel<T>::Z_STAGE;
         auto kern = spns::k3_z<T, L, S3::E, S3::P, MODE, STAGE>;

@@ -122,19 +122,20 @@ template <typename T> __device__ __forceinline__ T tmem_value(const Tmem4 &v, in
 
 // One block per SM of up to ZSTAGED_THREADS threads (the runtime places one block with
 // tensor memory per SM, so the SM's warps are one block).  A unit is a warp with 32/Q
-// pencils (pairs of pencils, T = f2), or the two warps of one (Q = 64); each unit has the
+// pencils (pairs of pencils, T = f2), the two warps of one (Q = 64) or three warps of four (Q = 24); each unit has the
 // exchange buffers of its pencils, 2 staging fields (rows of the work buffers' pitch Kp, the
 // last without its padding) and an mbarrier; one word for the block's tensor-memory address.
 constexpr int ZSTAGED_THREADS = 512;
+constexpr int whole_warps(int q) { return q % 32 == 0 ? q : 32 % q == 0 ? 32 : 96; }   // q = 24: four pencils in three warps
 template <typename T, int L, int E> struct ZStagedLayout {
-    static constexpr int Q = L / E, W = Arith<T>::W, U = Q <= 32 ? 32 : Q, PPU = U / Q;
+    static constexpr int Q = L / E, W = Arith<T>::W, U = whole_warps(Q), PPU = U / Q;
     using SM = SmPencil<T, L, E>;
-    static_assert((Q <= 32 && 32 % Q == 0) || Q == 64, "pencils are a part of a warp, one warp or an aligned pair of warps");
+    static_assert((U == 32 || U == 64 || U == 96 || U == 128) && U % Q == 0, "a unit's pencils fill one to four warps");
     static_assert(E == 12, "twelve values a thread: three tensor-memory accesses of four per slot");
-    static constexpr unsigned BAR = Q <= 32 ? 1u : GROUP64;
+    static constexpr unsigned BAR = U == 32 ? 1u : GROUP + U;
     static constexpr int COLS = 512;                 // all of the SM's; 128 (of 104 used) for each of the 4 warps of a lane quarter
-    // every compiled length is even, so the rows of a field are a multiple of 4: no unit is partly filled
-    static_assert(4 % (PPU * W) == 0, "rows of a unit");
+    // every compiled length is a multiple of 8 (and so are the rows of a field, of a slab too): no unit is partly filled
+    static_assert(8 % (PPU * W) == 0, "rows of a unit");
     // the unit's rows of one field, the last without its padding (whole 16-byte units, as Kp is)
     __host__ __device__ static constexpr size_t stage_bytes(int Kz, int Kp) {
         constexpr int A = 16 / (int)sizeof(SCx<T>);
@@ -156,9 +157,9 @@ template <int U> __device__ __forceinline__ bool unit_all(bool ok) {
         return __all_sync(0xffffffffu, ok) != 0;
     } else {
         unsigned r;
-        asm volatile("{\n.reg .pred p, r;\nsetp.ne.u32 p, %1, 0;\nbar.red.and.pred r, %2, 64, p;\nselp.u32 %0, 1, 0, r;\n}\n"
+        asm volatile("{\n.reg .pred p, r;\nsetp.ne.u32 p, %1, 0;\nbar.red.and.pred r, %2, %3, p;\nselp.u32 %0, 1, 0, r;\n}\n"
                      : "=r"(r)
-                     : "r"((unsigned)ok), "r"(1 + (threadIdx.x >> 6))
+                     : "r"((unsigned)ok), "r"(1 + threadIdx.x / U), "n"(U)
                      : "memory");
         return r != 0;
     }
