@@ -32,6 +32,15 @@ BOXES = {
     "y192": ((128, 96, 64), (192, 144, 96)),       # one after another
     "x288": ((192, 32, 33), (288, 48, 72)),
 }
+# boxes with pencils enough for the persistent z pass in single precision too: one to four warps
+# a unit, several pencils of one, a last round that is not full
+STAGED = {
+    "z192": ((128, 128, 125), (192, 192, 192)),
+    "z288": ((96, 96, 191), (144, 144, 288)),
+    "z384": ((96, 96, 256), (144, 144, 384)),
+    "z768": ((64, 64, 511), (96, 96, 768)),
+    "z1536": ((48, 48, 1024), (72, 72, 1536)),
+}
 FORMS = {
     "rotational": (0, dict(self_adaptive=True), dict(eps_forcing=0.1)),
     "advective": (2, dict(), dict()),
@@ -42,7 +51,7 @@ FORMS = {
 def _states(box, form_name, precision):
     import oracle as O
     from spns_b200.hit import HIT
-    N, M = BOXES[box]
+    N, M = {**BOXES, **STAGED}[box]
     form, aopt, hopt = FORMS[form_name]
     args = make_args(0, nu=3.283e-4, Ns=N, **aopt)
     args.Mx, args.My, args.Mz = M
@@ -90,6 +99,13 @@ def test_ensemble_names_the_member_that_failed():
     ens.close()
     for h in members:
         h.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("box", STAGED)
+def test_persistent_z_pass(box, precision):
+    a, b = _states(box, "rotational", precision)
+    assert rel_l2(a, b) <= (5e-6 if precision else 1e-12)
 
 
 @pytest.mark.parametrize("precision", [0, 1])
