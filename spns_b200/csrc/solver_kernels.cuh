@@ -180,11 +180,12 @@ __device__ __forceinline__ f2 col_k(int s, int kz, f2 *) { return f2((float)(s *
 // From length 768 on the current and the next tiles of all resident blocks (100 KB each, 58 MB
 // together) with their output do not stay in the near half of L2 until they are used: there K2
 // (input rows below the cut-off only) asks after the transform, before the stores (5.58 /
-// 2.89), and K4 and K5 not at all (K4 so 2.72 / 1.36).  The LES passes write more per read and
+// 2.89), and K4 and K5 not at all (K4 so 2.72 / 1.36); nor K2 at 1536 (N=1024 single 48.6 -> 59.8).
+// The LES passes write more per read and
 // their forward ones have three blocks per SM to cover each other's loads: K2 0.952 -> 0.977 / 0.672 ->
 // 0.576 (on in single precision), K4 1.04 -> 1.17 / 0.61 -> 0.63, K5 0.56 -> 0.65 / 0.34 -> 0.40.
 template <int L> constexpr bool PREFETCH_LATE = L >= 768;
-template <typename T, int MODE> constexpr bool PREFETCH_2 = MODE != MODE_LES || Arith<T>::SINGLE;
+template <typename T, int L, int MODE> constexpr bool PREFETCH_2 = L <= 768 && (MODE != MODE_LES || Arith<T>::SINGLE);
 template <int L, int MODE> constexpr bool PREFETCH_4 = L < 768 && MODE != MODE_LES;
 template <typename T, int L, int MODE> constexpr bool PREFETCH_5 = L < 768 && MODE != MODE_LES && !Arith<T>::SINGLE;
 template <int E, int P, class Addr> __device__ __forceinline__ void prefetch_rows(int p, Addr addr) {
@@ -331,7 +332,7 @@ __device__ __forceinline__ void k2_inv_y_body(Geo g, const SCx<T> *__restrict__ 
             r[e] = (ok && m2 <= g.hy && m2 >= -g.hy) ? ld_work(F + (col + (unsigned)(m2 >= 0 ? m2 : m2 + g.Ky) * rs), (cx<T> *)nullptr) : zero<T>();
         }
         auto prefetch = [&] {
-            if (!PREFETCH_2<T, MODE> || i + fs >= Fields<MODE>::K2 || source(field(i + fs)) == source(f)) return;
+            if (!PREFETCH_2<T, L, MODE> || i + fs >= Fields<MODE>::K2 || source(field(i + fs)) == source(f)) return;
             const SCx<T> *N = in + (long long)source(field(i + fs)) * g.S1;
             prefetch_rows<E, P>(p, [&](int e) -> const void * {
                 const int m2 = ffreq(in_row<L, E, true>(q, e), L);
