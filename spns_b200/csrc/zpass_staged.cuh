@@ -6,8 +6,8 @@
 // product c = w x u and the CFL maxima on the grid, r2c of c truncated to
 // kz <= hz (src/HIT_LES.cpp:74-125 up to the gradient the projection removes).
 // What differs is the schedule:
-//   * One block per SM, persistent, of independent units: a warp with one or several
-//     pencils (Q = L/E threads each), or the two warps of one pencil.  Each unit walks the
+//   * One block per SM, persistent, of independent units: one or several pencils (Q = L/E
+//     threads each) that fill one to four warps.  Each unit walks the
 //     pencils with the stride of the grid, with its own staging, mbarrier and exchange
 //     barrier.  Only the two fields of the next input pair are staged in shared memory, by
 //     cp.async.bulk (TMA bulk copies global -> shared, completion counted in bytes on an
@@ -20,7 +20,7 @@
 //     the 168 registers and 12 KB of shared memory per pencil at length 768, which held the
 //     pass to 12 warps per SM; now it is 16, and the slots' accesses leave the
 //     shared-memory pipe, the busiest one (77 % of its cycles; the FP64 pipe 44 %).
-//     Before and now: double 512^3 13.0 -> 11.5 ms, single 8.5 -> 7.1.
+//     Before and now: double 512^3 13.0 -> 11.5 ms, single 8.25 -> 7.2.
 //   * c_z is transformed as soon as it is known (after the second pair) and written
 //     over the w_x field of the same pencil (S2 field 3, consumed at the first
 //     pair), so the forward y pass reads the nonlinear term from fields 0, 1, 3.
