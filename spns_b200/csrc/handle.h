@@ -220,8 +220,6 @@ struct spns_handle {
     int forced_cap = 0;
     double *phys = nullptr;
     void *edge = nullptr;                            // edge-correction planes (rotational form)
-    cudaStream_t edge_st = nullptr;                  // their transforms run beside K1..K5: forked from st by
-    cudaEvent_t edge_fork = nullptr, edge_join = nullptr;   // edge_fork, joined to it by edge_join before the sweep
     void *inv_B1 = nullptr, *inv_B2 = nullptr;       // invariant spectra: advective-size work buffers (on first use)
     double *inv_bins = nullptr;                      // 5 spectra, then the nu_t accumulators
     double nut_stats[3] = {0.0, 0.0, 0.0};           // mean, rms, max of nu_t at the last invariant pass
@@ -351,8 +349,8 @@ struct LenTable {
     // the same for the n members of a batched class
     cudaError_t (*batch)(spns_handle *h, const spns::BatchMember *tab, int n, cudaStream_t st, int k, int mode);
     // batched 1-D transforms of contiguous lines / of the strided axis of [nbatch][L][ncols] arrays
-    cudaError_t (*lines)(spns_handle *h, void *data, long long batch, bool inv, cudaStream_t st);
-    cudaError_t (*cols)(spns_handle *h, void *data, int ncols, int nbatch, bool inv, cudaStream_t st);
+    cudaError_t (*lines)(spns_handle *h, void *data, long long batch, bool inv);
+    cudaError_t (*cols)(spns_handle *h, void *data, int ncols, int nbatch, bool inv);
 };
 #define SPNS_LEN_DECL(n) extern const LenTable spns_len_f64_##n, spns_len_f32_##n;
 SPNS_FOR_EACH_LENGTH(SPNS_LEN_DECL)

@@ -155,21 +155,21 @@ template <typename T> struct LenLaunch {
 #undef SPNS_SELECT
 
     // Batched 1-D FFTs for the 2-D edge planes.
-    template <int L, bool INV> static cudaError_t launch_lines(spns_handle *h, C *data, long long batch, cudaStream_t st) {
+    template <int L, bool INV> static cudaError_t launch_lines(spns_handle *h, C *data, long long batch) {
         using S = Shape<T, L>;
         auto kern = spns::k_lines<T, L, S::E, S::P, INV>;
         cudaError_t e = spns_set_smem(kern, S::SMEM_PEN);
         if (e != cudaSuccess) return e;
-        kern<<<(unsigned)((batch + S::P - 1) / S::P), S::THREADS, S::SMEM_PEN, st>>>(data, batch, tw(h, L));
+        kern<<<(unsigned)((batch + S::P - 1) / S::P), S::THREADS, S::SMEM_PEN, h->st>>>(data, batch, tw(h, L));
         return cudaGetLastError();
     }
-    template <int L, bool INV> static cudaError_t launch_cols(spns_handle *h, C *data, int ncols, int nbatch, cudaStream_t st) {
+    template <int L, bool INV> static cudaError_t launch_cols(spns_handle *h, C *data, int ncols, int nbatch) {
         using S = Shape<T, L>;
         auto kern = spns::k_cols<T, L, S::E, S::P, INV>;
         cudaError_t e = spns_set_smem(kern, S::SMEM_ROW);
         if (e != cudaSuccess) return e;
         dim3 grid((ncols + S::P - 1) / S::P, nbatch);
-        kern<<<grid, S::THREADS, S::SMEM_ROW, st>>>(data, ncols, tw(h, L));
+        kern<<<grid, S::THREADS, S::SMEM_ROW, h->st>>>(data, ncols, tw(h, L));
         return cudaGetLastError();
     }
     // ---- batched launches: one per pass for the members of a table, all of h0's class ----
@@ -265,11 +265,11 @@ template <typename T> struct LenLaunch {
             return mode == spns::MODE_LES ? batch_mode<L, spns::MODE_LES>(h, tab, n, st, k) : batch_mode<L, spns::MODE_ADV>(h, tab, n, st, k);
         return cudaErrorNotSupported;
     }
-    template <int L> static cudaError_t lines(spns_handle *h, void *data, long long batch, bool inv, cudaStream_t st) {
-        return inv ? launch_lines<L, true>(h, (C *)data, batch, st) : launch_lines<L, false>(h, (C *)data, batch, st);
+    template <int L> static cudaError_t lines(spns_handle *h, void *data, long long batch, bool inv) {
+        return inv ? launch_lines<L, true>(h, (C *)data, batch) : launch_lines<L, false>(h, (C *)data, batch);
     }
-    template <int L> static cudaError_t cols(spns_handle *h, void *data, int ncols, int nbatch, bool inv, cudaStream_t st) {
-        return inv ? launch_cols<L, true>(h, (C *)data, ncols, nbatch, st) : launch_cols<L, false>(h, (C *)data, ncols, nbatch, st);
+    template <int L> static cudaError_t cols(spns_handle *h, void *data, int ncols, int nbatch, bool inv) {
+        return inv ? launch_cols<L, true>(h, (C *)data, ncols, nbatch) : launch_cols<L, false>(h, (C *)data, ncols, nbatch);
     }
     template <int L> static constexpr LenTable table() { return LenTable{&pass<L>, &batch<L>, &lines<L>, &cols<L>}; }
 };

@@ -134,19 +134,20 @@ template <typename T> struct Passes {
     }
 
     // Exact aliasing correction of the rotational form on the +-N/2 planes
-    // (edge_kernels.cuh).  The aliasing axes are grouped by the size of their 2-D
-    // transforms (one group for a cubic box); each group has its own part of h->edge.
-    struct EdgeGroups { int n; spns::EdgeSet es[3]; C *V[3], *Phi[3]; };
-    static EdgeGroups edge_groups(spns_handle *h) {
+    // (edge_kernels.cuh), added to the compact nonlinear term G held in B2.  Its launches follow
+    // the passes in the stream, though the planes need only the state: as a branch of the
+    // step's graph they took 0.03 ms less of a 64^3 step and 0.26 ms of a 512^3 one, but
+    // destroying a graph with branches waits for all work on the device (closing a box while
+    // another steps: 600 ms against 1), and runs side by side held up each other's copies to the
+    // host (served workload, median of eight: p50 3.1 s against 1.1).
+    static int edge_correction(spns_handle *h) {
         const spns::Geo &g = h->g;
-        EdgeGroups G;
-        G.n = 0;
+        // group the aliasing axes by the size of their 2-D transforms (one group for a cubic box)
         int RC[3][2] = {{g.My, g.Mz}, {g.Mx, g.Mz}, {g.Mx, g.My}};
         bool done[3] = {false, false, false};
-        C *next = (C *)h->edge;
         for (int a0 = 0; a0 < 3; a0++) {
             if (!h->edge_axis[a0] || done[a0]) continue;
-            spns::EdgeSet &es = G.es[G.n];
+            spns::EdgeSet es;
             es.naxes = 0;
             es.R = RC[a0][0];
             es.C = RC[a0][1];
@@ -158,46 +159,23 @@ template <typename T> struct Passes {
                 es.first[es.naxes + 1] = es.first[es.naxes] + (a == 2 ? 1 : 2);
                 es.naxes++;
             }
-            const long long plane = (long long)es.R * es.C * es.first[es.naxes];
-            G.V[G.n] = next;
-            G.Phi[G.n] = next + 3 * plane;
-            next += 4 * plane;
-            G.n++;
-        }
-        return G;
-    }
-    // The planes' transforms need only the state, so they run on a second stream beside
-    // passes K1..K5 (a parallel branch of the step's graph): their six short launches took
-    // 40 of 168 us of the 64^3 step when they stood between K5 and the sweep.
-    static int edge_transforms(spns_handle *h, cudaStream_t st) {
-        const spns::Geo &g = h->g;
-        const EdgeGroups G = edge_groups(h);
-        for (int i = 0; i < G.n; i++) {
-            const spns::EdgeSet &es = G.es[i];
             const int np = es.first[es.naxes];
-            const long long n = (long long)es.R * es.C, nb = n * 3 * np;
+            const long long n = (long long)es.R * es.C;
+            C *V = (C *)h->edge, *Phi = V + 3 * (long long)np * n;
+            const long long nb = n * 3 * np;
             const int blocks = (int)std::min<long long>((nb + 255) / 256, 16LL * h->sms);
-            spns::k_edge_build<T><<<blocks, 256, 0, st>>>(g, U(h), es, G.V[i]);
+            spns::k_edge_build<T><<<blocks, 256, 0, h->st>>>(g, U(h), es, V);
             CKL();
-            LAUNCH(spns_len_table<T>(es.C)->lines(h, G.V[i], (long long)es.R * 3 * np, true, st));
-            LAUNCH(spns_len_table<T>(es.R)->cols(h, G.V[i], es.C, 3 * np, true, st));
-            spns::k_edge_square<T><<<blocks, 256, 0, st>>>(G.V[i], n, np, G.Phi[i]);
+            LAUNCH(spns_len_table<T>(es.C)->lines(h, V, (long long)es.R * 3 * np, true));
+            LAUNCH(spns_len_table<T>(es.R)->cols(h, V, es.C, 3 * np, true));
+            spns::k_edge_square<T><<<blocks, 256, 0, h->st>>>(V, n, np, Phi);
             CKL();
-            LAUNCH(spns_len_table<T>(es.C)->lines(h, G.Phi[i], (long long)es.R * np, false, st));
-            LAUNCH(spns_len_table<T>(es.R)->cols(h, G.Phi[i], es.C, np, false, st));
-            h->edge_launches += 6;
-        }
-        return SPNS_OK;
-    }
-    // Adds the correction to the compact nonlinear term G held in B2.
-    static int edge_apply(spns_handle *h) {
-        const EdgeGroups G = edge_groups(h);
-        for (int i = 0; i < G.n; i++) {
-            const spns::EdgeSet &es = G.es[i];
-            const int ablocks = (int)std::min<long long>(((long long)es.R * es.C * 2 + 255) / 256, 8LL * h->sms);
-            spns::k_edge_apply<T><<<dim3(ablocks, es.naxes), 256, 0, h->st>>>(h->g, (C *)h->B2, es, G.Phi[i]);
+            LAUNCH(spns_len_table<T>(es.C)->lines(h, Phi, (long long)es.R * np, false));
+            LAUNCH(spns_len_table<T>(es.R)->cols(h, Phi, es.C, np, false));
+            const int ablocks = (int)std::min<long long>((n * 2 + 255) / 256, 8LL * h->sms);
+            spns::k_edge_apply<T><<<dim3(ablocks, es.naxes), 256, 0, h->st>>>(g, (C *)h->B2, es, Phi);
             CKL();
-            h->edge_launches += 1;
+            h->edge_launches += 7;
         }
         return SPNS_OK;
     }
@@ -225,14 +203,6 @@ template <typename T> struct Passes {
             nk += 1;
         }
         const int mode = h->a.isLES ? spns::MODE_LES : h->a.nonlinear_form == 2 ? spns::MODE_ADV : spns::MODE_ROT;
-        const bool edge = mode == spns::MODE_ROT && h->edge;
-        if (edge) {
-            CK(cudaEventRecord(h->edge_fork, h->st));
-            CK(cudaStreamWaitEvent(h->edge_st, h->edge_fork, 0));
-            const int r_ = edge_transforms(h, h->edge_st);
-            CK(cudaEventRecord(h->edge_join, h->edge_st));
-            if (r_) return r_;
-        }
         MARK("k1_inv_x");
         LAUNCH(pass(h, 1, mode, true));
         MARK("k2_inv_y");
@@ -243,10 +213,9 @@ template <typename T> struct Passes {
         LAUNCH(pass(h, 4, mode, true));
         MARK("k5_fwd_x");
         LAUNCH(pass(h, 5, mode, true));
-        if (edge) {
+        if (mode == spns::MODE_ROT && h->edge) {
             MARK("edge_correction");
-            CK(cudaStreamWaitEvent(h->st, h->edge_join, 0));
-            const int r_ = edge_apply(h);
+            int r_ = edge_correction(h);
             if (r_) return r_;
         }
         MARK("k6_sweep");
@@ -256,7 +225,7 @@ template <typename T> struct Passes {
         CKL();
         MARK(nullptr);
         if (prof) { if (h->prof_steps == 0) h->prof_nk = slot - 1; h->prof_steps++; }
-        if (edge) nk += h->edge_launches;             // build, 2+2 line FFTs, square, apply per group
+        if (mode == spns::MODE_ROT && h->edge) nk += h->edge_launches;             // build, 2+2 line FFTs, square, apply per group
         h->kernels_per_step = nk + 7;
         return SPNS_OK;
 #undef MARK

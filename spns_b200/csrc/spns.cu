@@ -367,9 +367,6 @@ static void free_handle(spns_handle *h) {
     for (auto &kv : h->tw2) if (kv.second) cudaFreeAsync(kv.second, h->st);
     for (auto ev : h->prof_ev) cudaEventDestroy(ev);
     for (auto &gx : h->graph) if (gx) cudaGraphExecDestroy(gx);
-    if (h->edge_fork) cudaEventDestroy(h->edge_fork);
-    if (h->edge_join) cudaEventDestroy(h->edge_join);
-    if (h->edge_st) cudaStreamDestroy(h->edge_st);
     if (h->st) cudaStreamDestroy(h->st);
     delete h;
 }
@@ -435,14 +432,6 @@ int spns_create(const spns_hit_args *args, const double *file_uvw, spns_handle *
             return cleanup(spns_fail(nullptr, SPNS_ERR_CUDA, "SM count query failed"));
     }
     const BufferPlan bp = buffer_plan(a, g, h->last_rad_max);
-    if (bp.need_edge) {
-        int prio = 0;
-        if (cudaStreamGetPriority(h->st, &prio) != cudaSuccess ||
-            cudaStreamCreateWithPriority(&h->edge_st, cudaStreamNonBlocking, prio) != cudaSuccess ||
-            cudaEventCreateWithFlags(&h->edge_fork, cudaEventDisableTiming) != cudaSuccess ||
-            cudaEventCreateWithFlags(&h->edge_join, cudaEventDisableTiming) != cudaSuccess)
-            return cleanup(spns_fail(nullptr, SPNS_ERR_CUDA, "stream creation failed"));
-    }
     h->nB1 = bp.nB1;
     h->nB2 = bp.nB2;
     for (int i = 0; i < 3; i++) h->edge_axis[i] = bp.edge_axis[i];
@@ -518,7 +507,6 @@ int spns_create(const spns_hit_args *args, const double *file_uvw, spns_handle *
 int spns_destroy(spns_handle *h) {
     if (!h) return SPNS_ERR_INVALID_ARGUMENT;
     cudaSetDevice(h->a.device);
-    if (h->edge_st) cudaStreamSynchronize(h->edge_st);
     cudaStreamSynchronize(h->st);
     free_handle(h);
     return SPNS_OK;
