@@ -50,8 +50,21 @@ template <typename T> struct LenLaunch {
         kern<<<grid, S::THREADS, S::SMEM_ROW, h->st>>>(h->g, (const C *)h->B1, (C *)h->B2, twx<2, L>(h));
         return cudaGetLastError();
     }
+    // Blocks of a z pass over n items whose blocks walk the box, `wave` of them resident at once.
+    // A block holds its place on an SM until it ends, so a run of higher priority on the same
+    // device waits that long: one wave where a block has at most 16 items (14 to 29 us each),
+    // else as many whole waves as leave it 8.  32^3 and 64^3 LES of higher priority beside two
+    // 256^3 LES boxes, us a step, one wave against this: single 209 -> 160 and 443 -> 365, double
+    // 269 -> 192 and 567 -> 430 (with a block for every few pencils 211, 390, 265, 519).  The pass
+    // alone, ms: 256^3 LES single 2.28 -> 2.20, double 4.00 -> 3.82; 512^3 single 7.23 -> 6.80,
+    // double 11.53 -> 11.47; 512 x 512 x 64 LES double 3.61 -> 3.77.  With four items for eight the
+    // waits are 5 to 15 % shorter, 512^3 single 7.6 and 512 x 512 x 64 3.91.
+    static unsigned walking_blocks(long long wave, long long n) {
+        const long long rounds = (n + wave - 1) / wave;
+        return (unsigned)std::min(n, rounds <= 16 ? wave : wave * ((rounds + 7) / 8));
+    }
     // Rotational z pass staged pair by pair with bulk copies (zpass_staged.cuh),
-    // persistent: one block per SM.  Units of the box, and units the SMs hold in one round.
+    // one block per SM at a time.  Units of the box, and units the SMs hold in one round.
     template <int L> static long long staged_units(const spns_handle *h) {
         using LY = spns::ZStagedLayout<A, L, SPNS_ZS_E>;
         return (long long)h->g.Mx * h->g.My / (LY::PPU * LY::W);
@@ -76,28 +89,28 @@ template <typename T> struct LenLaunch {
         const size_t smem = LY::smem_bytes(units, h->g.Kz, h->g.Kp);
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        const unsigned blocks = (unsigned)std::min<long long>((ngrp + units - 1) / units, h->sms);
+        const unsigned blocks = walking_blocks(h->sms, (ngrp + units - 1) / units);
         kern<<<blocks, units * LY::U, smem, h->st>>>(h->g, (C *)h->B2, h->c, h->ds, twa(h, L));
         return cudaGetLastError();
     }
-    // Persistent launch of k3_field: one wave of blocks.
+    // Launch of k3_field: blocks that walk the pencils.
     template <int L, int MODE, int ALT> static cudaError_t launch_k3_field(spns_handle *h, double *nut) {
         using S = ZFieldShape<A, L, MODE, ALT>;
         auto kern = spns::k3_field<A, L, S::E, S::PB, S::NT, MODE, S::MINB>;
         unsigned blocks = 0;
-        cudaError_t e = wave_of_blocks(h, kern, S::THREADS, S::LY::SMEM, ((long long)h->g.Mx * h->g.My / spns::Arith<A>::W + S::PB - 1) / S::PB, &blocks);
+        cudaError_t e = walking_grid(h, kern, S::THREADS, S::LY::SMEM, ((long long)h->g.Mx * h->g.My / spns::Arith<A>::W + S::PB - 1) / S::PB, &blocks);
         if (e != cudaSuccess) return e;
         kern<<<blocks, S::THREADS, S::LY::SMEM, h->st>>>(h->g, (C *)h->B2, h->c, h->ds, nut, twa(h, L));
         return cudaGetLastError();
     }
-    // Shared-memory opt-in and grid of a persistent kernel over n work items.
-    template <class K> static cudaError_t wave_of_blocks(spns_handle *h, K kern, int threads, size_t smem, long long n, unsigned *blocks) {
+    // Shared-memory opt-in and grid of a kernel whose blocks walk n work items.
+    template <class K> static cudaError_t walking_grid(spns_handle *h, K kern, int threads, size_t smem, long long n, unsigned *blocks) {
         cudaError_t e = spns_set_smem(kern, smem);
         if (e != cudaSuccess) return e;
         int per_sm = 0;
         if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem)) != cudaSuccess) return e;
         if (per_sm < 1) return cudaErrorInvalidConfiguration;
-        *blocks = (unsigned)std::min<long long>(n, (long long)h->sms * per_sm);
+        *blocks = walking_blocks((long long)h->sms * per_sm, n);
         return cudaSuccess;
     }
     template <int L, int MODE, int ALT = 0> static cudaError_t launch_k3(spns_handle *h, double *phys) {
@@ -193,7 +206,7 @@ template <typename T> struct LenLaunch {
         using S = ZFieldShape<A, L, MODE, ALT>;
         auto kern = spns::k3_field_batch<A, L, S::E, S::PB, S::NT, MODE, S::MINB>;
         unsigned blocks = 0;
-        cudaError_t e = wave_of_blocks(h, kern, S::THREADS, S::LY::SMEM, ((long long)h->g.Mx * h->g.My / spns::Arith<A>::W + S::PB - 1) / S::PB, &blocks);
+        cudaError_t e = walking_grid(h, kern, S::THREADS, S::LY::SMEM, ((long long)h->g.Mx * h->g.My / spns::Arith<A>::W + S::PB - 1) / S::PB, &blocks);
         if (e != cudaSuccess) return e;
         kern<<<dim3(blocks, n), S::THREADS, S::LY::SMEM, st>>>(h->g, tab, twa(h, L));
         return cudaGetLastError();

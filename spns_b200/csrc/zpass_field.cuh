@@ -19,7 +19,7 @@
 // with up to 12 slots per grid row in the thread that owns the row; what is left is the
 // shared-memory traffic of the exchanges, and E = 24 plans (one exchange less) fit.
 //
-// Persistent: one wave of blocks walks the groups of PB pencils, so the CFL maxima are
+// Blocks walk the groups of PB pencils (LenLaunch::walking_blocks), so the CFL maxima are
 // reduced once per block.
 #pragma once
 #include "solver_kernels.cuh"

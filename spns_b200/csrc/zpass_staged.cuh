@@ -1,4 +1,4 @@
-// zpass_staged.cuh -- the rotational-form z pass, persistent over the grid, with
+// zpass_staged.cuh -- the rotational-form z pass, whose blocks walk the grid, with
 // its input pairs staged by bulk asynchronous copies.
 //
 // Same arithmetic as k3_z<MODE_ROT> (solver_kernels.cuh): c2r of the six real
@@ -6,9 +6,9 @@
 // product c = w x u and the CFL maxima on the grid, r2c of c truncated to
 // kz <= hz (src/HIT_LES.cpp:74-125 up to the gradient the projection removes).
 // What differs is the schedule:
-//   * One block per SM, persistent, of independent units: one or several pencils (Q = L/E
+//   * One block per SM at a time, of independent units: one or several pencils (Q = L/E
 //     threads each) that fill one to four warps.  Each unit walks the
-//     pencils with the stride of the grid, with its own staging, mbarrier and exchange
+//     pencils with the stride of the grid (LenLaunch::walking_blocks), with its own staging, mbarrier and exchange
 //     barrier.  Only the two fields of the next input pair are staged in shared memory, by
 //     cp.async.bulk (TMA bulk copies global -> shared, completion counted in bytes on an
 //     mbarrier), while the current pair is transformed; the first pair of the next pencils

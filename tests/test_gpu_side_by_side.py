@@ -32,3 +32,31 @@ def test_closing_a_box_leaves_the_others_running(les):
         if running:
             return
     pytest.fail("closing a 64^3 box waited for 300 steps of a 256^3 box, three times of three")
+
+
+@pytest.mark.parametrize("N, les, precision", [((256, 256, 512), 0.17, 1), ((256, 256, 512), 0.17, 0), ((512, 256, 512), 0.0, 1)])
+def test_short_steps_do_not_wait_for_whole_z_passes(N, les, precision):
+    """Steps of a 32^3 box of high priority, one after another, beside a box whose z pass takes
+    milliseconds.  If blocks of that pass stayed to its end, one short step in each long one would wait
+    for nearly the whole pass; at most one in four may wait for half of it."""
+    import time
+
+    import numpy as np
+    long_run, short = _box(N, les, precision), _box((32, 32, 32), 0.17, 1, -5)
+    for h in (long_run, short):
+        h.New_Fractional_Step_Method(4)            # captured
+    long_run.profile_begin(3)
+    long_run.New_Fractional_Step_Method(3)
+    names, ms = long_run.profile_read(3)
+    z_pass = 1e-3 * float(np.median(ms[:, names.index("k3_z")]))
+    steps, waits = 40, []
+    long_run.step_async(steps)
+    while not long_run.query():
+        t = time.perf_counter()
+        short.step_async(1)
+        short.synchronize()
+        waits.append(time.perf_counter() - t)
+    long_run.synchronize()
+    short.close()
+    long_run.close()
+    assert len(waits) > steps and np.sum(np.array(waits) > 0.5 * z_pass) <= steps // 4
