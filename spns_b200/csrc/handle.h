@@ -246,6 +246,7 @@ struct spns_handle {
     unsigned char shape_alt[6] = {0, 0, 0, 0, 0, 0};
     void *U0 = nullptr;                              // state buffer of parity 0
     bool use_graphs = true;
+    int stage_polls = spns::ZS_WAIT_LIMIT;           // polls of a wait of the staged z pass; SPNS_STAGE_POLLS lowers it (0: every wait gives up)
     // optional per-kernel event profile of the next steps (spns_profile_*)
     std::vector<cudaEvent_t> prof_ev;
     std::vector<std::string> prof_names;

@@ -90,7 +90,7 @@ template <typename T> struct LenLaunch {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         const unsigned blocks = walking_blocks(h->sms, (ngrp + units - 1) / units);
-        kern<<<blocks, units * LY::U, smem, h->st>>>(h->g, (C *)h->B2, h->c, h->ds, twa(h, L));
+        kern<<<blocks, units * LY::U, smem, h->st>>>(h->g, (C *)h->B2, h->c, h->ds, twa(h, L), h->stage_polls);
         return cudaGetLastError();
     }
     // Launch of k3_field: blocks that walk the pencils.

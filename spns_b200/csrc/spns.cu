@@ -487,6 +487,8 @@ int spns_create(const spns_hit_args *args, const double *file_uvw, spns_handle *
     {
         const char *ng = getenv("SPNS_NO_GRAPHS");
         h->use_graphs = !(ng && ng[0] == '1');
+        const char *sp = getenv("SPNS_STAGE_POLLS");
+        if (sp) h->stage_polls = std::max(0, std::min(spns::ZS_WAIT_LIMIT, atoi(sp)));
     }
     rc = spns_ops(h).run_velocity(h, nullptr);
     if (rc) { g_create_error = h->err; return cleanup(rc); }

@@ -27,8 +27,10 @@
 //   * CFL maxima accumulate per thread over all pencils and are reduced once per
 //     block at the end.
 // Every mbarrier wait is bounded; a wait that gives up records wait_timeout in
-// the solver scalars (reported as SPNS_ERR_TIMEOUT by the host) and the pencil's
-// threads skip their remaining pencils; no copy is left in flight.
+// the solver scalars (reported as SPNS_ERR_TIMEOUT by the host) and the unit
+// skips its remaining pencils.  The copies that it waited for may still be on
+// their way then, into shared memory that the SM hands to its next block, so the
+// unit waits for them once more, as long as a wait may take, before it leaves.
 #pragma once
 #include "solver_kernels.cuh"
 
@@ -73,7 +75,7 @@ __device__ __forceinline__ bool mbar_wait_bounded(unsigned long long *bar, unsig
     return false;
 }
 
-constexpr int ZS_WAIT_LIMIT = 1 << 22;
+constexpr int ZS_WAIT_LIMIT = 1 << 22;   // polls of a wait
 
 // ---------------------------------------------------------------------------
 // Thread-private values in tensor memory.  A warp may store and load 32-bit columns of its
@@ -167,7 +169,7 @@ template <int U> __device__ __forceinline__ bool unit_all(bool ok) {
 
 template <typename T, int L, int E>
 __global__ void __launch_bounds__(ZSTAGED_THREADS, 1) k3_rot_staged(Geo g, SCx<T> *__restrict__ buf, StepConsts c, DevScalars *ds,
-                                                        const cx<T> *__restrict__ tw) {
+                                                        const cx<T> *__restrict__ tw, int polls) {
     using LY = ZStagedLayout<T, L, E>;
     constexpr int Q = LY::Q, W = LY::W, U = LY::U, PPU = LY::PPU;
     constexpr unsigned BAR = LY::BAR;
@@ -211,7 +213,7 @@ __global__ void __launch_bounds__(ZSTAGED_THREADS, 1) k3_rot_staged(Geo g, SCx<T
     };
     // the staged pair is complete and visible to every thread of the unit
     auto wait_stage = [&]() -> bool {
-        const bool ok = mbar_wait_bounded(bar, parity, ZS_WAIT_LIMIT);
+        const bool ok = mbar_wait_bounded(bar, parity, polls);
         parity ^= 1u;
         return unit_all<U>(ok);
     };
@@ -316,7 +318,10 @@ __global__ void __launch_bounds__(ZSTAGED_THREADS, 1) k3_rot_staged(Geo g, SCx<T
             }
         }
     }
-    if (bad && tid % U == 0) atomicExch(&ds->wait_timeout, 1);
+    if (bad) {
+        mbar_wait_bounded(bar, parity ^ 1u, ZS_WAIT_LIMIT);   // the phase that the failed wait was for
+        if (tid % U == 0) atomicExch(&ds->wait_timeout, 1);
+    }
     __syncwarp();
     Tmem4 tm;
     tmem_ld4(slots + 96, tm);
