@@ -319,8 +319,10 @@ template <typename T> inline void *spns_make_twiddles(int L, cudaStream_t st, bo
     return d;
 }
 
-// Opt-in to the dynamic shared memory of a launch.  Set even below 48 KB: the
-// kernel's static shared memory counts against the same 48 KB default limit.
+// Opt-in to the dynamic shared memory of a kernel's launches.  Set even below 48 KB: the
+// kernel's static shared memory counts against the same 48 KB default limit.  The limit
+// belongs to the kernel, for every handle and thread: `bytes` is a constant of the kernel,
+// the most that any box launches it with, never the size of one box.
 template <class K> inline cudaError_t spns_set_smem(K kern, size_t bytes) {
     if (bytes <= 16 * 1024) return cudaSuccess;
     return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);

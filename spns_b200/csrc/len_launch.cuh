@@ -87,7 +87,7 @@ template <typename T> struct LenLaunch {
         // as many units as spread the pencils evenly over the rounds
         const int units = (int)((ngrp + rounds * h->sms - 1) / (rounds * h->sms));
         const size_t smem = LY::smem_bytes(units, h->g.Kz, h->g.Kp);
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = spns_set_smem(kern, LY::SMEM_MAX);
         if (e != cudaSuccess) return e;
         const unsigned blocks = walking_blocks(h->sms, (ngrp + units - 1) / units);
         kern<<<blocks, units * LY::U, smem, h->st>>>(h->g, (C *)h->B2, h->c, h->ds, twa(h, L), h->stage_polls);
@@ -124,10 +124,10 @@ template <typename T> struct LenLaunch {
         auto kern = spns::k3_z<T, L, S3::E, S3::P, MODE, STAGE>;
         constexpr size_t stage_fields = STAGE ? 2 * spns::K3StagePairs<T>::N : 0;
         // the staging is sized by Kz at run time: at most L/2+1 values per field and pencil
-        static_assert(S3::SMEM + (size_t)S3::P * stage_fields * (L / 2 + 1) * sizeof(C) <= 227 * 1024,
-                      "z-pass shared memory (exchange and staging) exceeds 227 KB for this shape");
+        constexpr size_t most = S3::SMEM + (size_t)S3::P * stage_fields * (L / 2 + 1) * sizeof(C);
+        static_assert(most <= 225 * 1024, "z-pass shared memory (exchange and staging) exceeds 227 KB, less the reductions', for this shape");
         const size_t smem = S3::SMEM + (size_t)S3::P * stage_fields * h->g.Kz * sizeof(C);
-        cudaError_t e = spns_set_smem(kern, smem);
+        cudaError_t e = spns_set_smem(kern, most);
         if (e != cudaSuccess) return e;
         const long long npen = (long long)h->g.Mx * h->g.My;
         dim3 grid((unsigned)((npen + S3::P - 1) / S3::P));

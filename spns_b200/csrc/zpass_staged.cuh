@@ -146,9 +146,10 @@ template <typename T, int L, int E> struct ZStagedLayout {
     static constexpr size_t EXCH = (size_t)PPU * SM::PITCH * sizeof(cx<T>);
     __host__ __device__ static constexpr size_t unit_bytes(int Kz, int Kp) { return EXCH + 2 * stage_bytes(Kz, Kp) + sizeof(unsigned long long); }
     __host__ __device__ static constexpr size_t smem_bytes(int units, int Kz, int Kp) { return units * unit_bytes(Kz, Kp) + 16; }
+    static constexpr size_t SMEM_MAX = 225 * 1024 + 16;   // of any box
     // most units of a block
     __host__ __device__ static constexpr int max_units(int Kz, int Kp) {
-        const int s = (int)((225 * 1024) / unit_bytes(Kz, Kp)), t = ZSTAGED_THREADS / U;
+        const int s = (int)((SMEM_MAX - 16) / unit_bytes(Kz, Kp)), t = ZSTAGED_THREADS / U;
         return s < t ? s : t;
     }
 };

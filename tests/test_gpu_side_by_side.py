@@ -60,3 +60,40 @@ def test_short_steps_do_not_wait_for_whole_z_passes(N, les, precision):
     short.close()
     long_run.close()
     assert len(waits) > steps and np.sum(np.array(waits) > 0.5 * z_pass) <= steps // 4
+
+
+@pytest.mark.parametrize("My, Mz, wide", [(48, 384, 256), (48, 192, 128), (72, 384, 256)])
+def test_threads_with_boxes_of_one_z_length(My, Mz, wide, monkeypatch):
+    """Two host threads launch steps of boxes with the same z length and 17 and `wide` / 2 + 1 modes
+    along it (staged z pass, and k3_z at 192): the shared memory that the kernels of the
+    one need does not depend on what the other launched last."""
+    import threading
+
+    import numpy as np
+
+    from spns_b200.hit import HIT
+    monkeypatch.setenv("SPNS_NO_GRAPHS", "1")
+    boxes = []
+    for Nz in (32, wide):
+        args = make_args(0, nu=1e-3, Ns=(32, My * 2 // 3, Nz))
+        args.Mx, args.My, args.Mz = 48, My, Mz
+        h = HIT(args, k41_ranks=-1)
+        h.seed_field(3, 3.0)
+        boxes.append(h)
+    errors = []
+
+    def run(h):
+        try:
+            for _ in range(60):
+                h.step_async(100)
+                h.synchronize()
+        except Exception as e:  # noqa: BLE001
+            errors.append(str(e))
+
+    threads = [threading.Thread(target=run, args=(h,)) for h in boxes]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
+    assert all(np.isfinite(h.get_compact()).all() for h in boxes)
