@@ -91,6 +91,10 @@ template <int COLS> __device__ __forceinline__ void tmem_alloc(unsigned *dst) {
 template <int COLS> __device__ __forceinline__ void tmem_free(unsigned addr) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(addr), "n"(COLS) : "memory");
 }
+// Tensor-memory accesses of different warps are ordered by a barrier only between these two:
+// the one before it after a warp's own accesses, the other after it before what depends on them.
+__device__ __forceinline__ void tmem_fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
+__device__ __forceinline__ void tmem_fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ unsigned long long bits64(double v) { return (unsigned long long)__double_as_longlong(v); }
 __device__ __forceinline__ unsigned long long bits64(f2 v) { return v.v; }
 __device__ __forceinline__ void from_bits64(unsigned long long b, double &v) { v = __longlong_as_double((long long)b); }
@@ -189,7 +193,9 @@ __global__ void __launch_bounds__(ZSTAGED_THREADS, 1) k3_rot_staged(Geo g, SCx<T
         mbar_init(bar, 1);
         fence_mbar_init();
     }
+    tmem_fence_before_sync();
     __syncthreads();
+    tmem_fence_after_sync();
     // this warp's lanes and columns; slots of 24 columns: 0 u, 1 v, 2 w_x, 3 w_y
     const unsigned tbase = *taddr;
     const unsigned slots = tbase + ((unsigned)(tid >> 5 & 3) << 21) + (unsigned)(tid >> 7) * 128u;
@@ -328,7 +334,9 @@ __global__ void __launch_bounds__(ZSTAGED_THREADS, 1) k3_rot_staged(Geo g, SCx<T
     tmem_ld4(slots + 96, tm);
     tmem_wait_ld(tm);
     const double mx[4] = {tmem_value<double>(tm, 0), tmem_value<double>(tm, 1), tmem_value<double>(tm, 2), tmem_value<double>(tm, 3)};
+    tmem_fence_before_sync();
     block_max4<T>(mx, ds);   // (a block barrier: every warp is done with the tensor memory)
+    tmem_fence_after_sync();
     if (tid < 32) tmem_free<LY::COLS>(tbase);
 }
 
