@@ -350,7 +350,12 @@ static BufferPlan buffer_plan(const spns_hit_args &a, const Geo &g, int last_rad
     p.bins = sizeof(double) * 2 * (size_t)(last_rad_max + 1);
     // up to 5 planes of one axis set: 3 components each for V plus one Phi plane each
     p.edge = p.need_edge ? cs * 20 * (size_t)std::max((long long)g.My * g.Mz, std::max((long long)g.Mx * g.Mz, (long long)g.Mx * g.My)) : 0;
-    p.tw = cs * ((size_t)g.Mx + g.My + g.Mz);
+    // one table per length, in single precision once more as pairs (spns_make_twiddles)
+    for (int i = 0; i < 3; i++) {
+        const int L[3] = {g.Mx, g.My, g.Mz};
+        if ((i > 0 && L[i] == L[0]) || (i > 1 && L[i] == L[1])) continue;
+        p.tw += cs * (size_t)spns::tw_full_size(L[i]) * (hilo ? 3 : 1);
+    }
     p.scalars = sizeof(DevScalars);
     return p;
 }
