@@ -13,10 +13,9 @@ the solver has no data-path collective, so `value` is the sum over ranks
 
 --impl reference times the reference solver on the host cores (oracle/_ref:
 src/*.cpp of adalbal/SpNS compiled unchanged against single-process MPI and
-FFTW stand-ins, the oracle's OpenMP FFT in place of FFTW's threads; where it
-was not built, the CPU oracle, a C restatement of the same solver) on a bounded
+FFTW stand-ins, the oracle's OpenMP FFT in place of FFTW's threads) on a bounded
 sample of the same workload, and prints the same JSON line with
-"impl": "reference".
+"impl": "reference"; where it was not built, a line that says so.
 """
 from __future__ import annotations
 
@@ -501,19 +500,16 @@ def run_reference(args):
     rank = int(os.environ.get("RANK", 0))
     if rank != 0:
         return 0
+    if not os.path.exists(REF_EXE):
+        print(json.dumps({"impl": "reference", "unavailable": "oracle/_ref/spns_ref is not built: the reference's sources are not on this machine"}),
+              flush=True)
+        return 0
     threads = os.cpu_count() or 1
     n_sample = args.ref_sample_n
-    if os.path.exists(REF_EXE):
-        # W warm-up steps inside the first (set-up cancelling) run pair, then K timed steps
-        if args.warmup > 0:
-            ref_sample(n_sample, args.warmup, threads)
-        s, kind, desc = cpu_step_seconds(n_sample, max(1, args.steps), threads)
-    else:
-        for _ in range(args.warmup):
-            cpu_sample(n_sample, 1, threads)
-        per = [cpu_sample(n_sample, 1, threads) for _ in range(max(1, args.steps))]
-        s, kind = sum(per) / len(per), "port"
-        desc = f"one CPU-oracle step at N={n_sample} per timed step, {s:.3f} s/step"
+    # W warm-up steps inside the first (set-up cancelling) run pair, then K timed steps
+    if args.warmup > 0:
+        ref_sample(n_sample, args.warmup, threads)
+    s, kind, desc = cpu_step_seconds(n_sample, max(1, args.steps), threads)
     scale = fft_work(N_BOX) / fft_work(n_sample)
     value = 1.0 / (s * scale)
     line = {
