@@ -159,8 +159,8 @@ constexpr int SPNS_SPLIT_WAVES = 4;   // x/y passes with fewer than 4 blocks per
 template <typename T> constexpr bool spns_zstaged_length(int L) { return L >= 192 || ((L == 144 || L == 96) && sizeof(T) == 8); }
 constexpr int SPNS_ZS_E = 12;
 
-// Velocity and short-length rotational z pass (k3_z): pencils per block limited by the
-// shared memory of the exchange buffers.
+// Velocity z pass, and the rotational one of short lengths and of boxes with few pencils (k3_z):
+// pencils per block limited by the shared memory of the exchange buffers.
 template <typename T, int L, int ALT = 0> struct Shape3 {
     static constexpr int E = ALT ? SPNS_ALT_E : ShapeSel<T>::Z_E;
     static constexpr int Q = L / E;

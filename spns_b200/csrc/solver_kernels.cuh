@@ -154,10 +154,6 @@ __device__ __forceinline__ void st_work(cx<float> *p, cx<f2> v) {
 // Compact arrays (S0): rows of Kz elements, so a pair may straddle 16 bytes and the last row end (two: it is whole).
 __device__ __forceinline__ cx<double> ld_compact(const cx<double> *p, bool, cx<double> *) { return *p; }
 __device__ __forceinline__ cx<float> ld_compact(const cx<float> *p, bool, cx<float> *) { return *p; }
-__device__ __forceinline__ cx<f2> ld_compact(const cx<float> *p, bool two, cx<f2> *) {
-    const cx<float> a = p[0], b = two ? p[1] : zero<float>();
-    return mk<f2>(f2(a.x, b.x), f2(a.y, b.y));
-}
 __device__ __forceinline__ void st_compact(cx<double> *p, cx<double> v, bool) { *p = v; }
 __device__ __forceinline__ void st_compact(cx<float> *p, cx<float> v, bool) { *p = v; }
 __device__ __forceinline__ void st_compact(cx<float> *p, cx<f2> v, bool two) {
@@ -167,7 +163,6 @@ __device__ __forceinline__ void st_compact(cx<float> *p, cx<f2> v, bool two) {
 // s kz of the thread's columns
 __device__ __forceinline__ double col_k(int s, int kz, double *) { return (double)(s * kz); }
 __device__ __forceinline__ float col_k(int s, int kz, float *) { return (float)(s * kz); }
-__device__ __forceinline__ f2 col_k(int s, int kz, f2 *) { return f2((float)(s * kz), (float)(s * kz + s)); }
 
 // The x/y passes wait on the loads of a field with nothing else in flight, so while it is
 // transformed the rows of the block's next field are asked for in L2.  addr(e): the tile's

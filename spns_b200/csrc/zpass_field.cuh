@@ -28,18 +28,17 @@ namespace spns {
 
 // Inverse pairs and forward jobs per form.
 template <int MODE> struct ZFieldForm {
-    static constexpr int NPAIR = MODE == MODE_ROT ? 3 : MODE == MODE_INV ? 5 : 6;
+    static_assert(MODE == MODE_ADV || MODE == MODE_LES || MODE == MODE_INV, "the rotational form runs in k3_rot_staged or k3_z");
+    static constexpr int NPAIR = MODE == MODE_INV ? 5 : 6;
     static constexpr int NJOB = MODE == MODE_LES ? 5 : MODE == MODE_INV ? 3 : 2;
 };
 
 // S2 fields of inverse pair p and whether each enters as its z derivative (b < 0: none).
-//   ROT  (u, w_x), (v, w_y), (w, w_z)
 //   ADV, LES  (u, v), (w, du/dz), (du/dx, du/dy), (dv/dx, dv/dy), (dw/dx, dw/dy), (dv/dz, dw/dz)
 //   INV  (du/dx, du/dy), (dv/dx, dv/dy), (dw/dx, dw/dy), (du/dz, dv/dz), (dw/dz, -)
 struct ZPair { int a, b; bool da, db; };
 template <int MODE> __device__ __forceinline__ ZPair zfield_pair(int p) {
-    if constexpr (MODE == MODE_ROT) return ZPair{p, p + 3, false, false};
-    else if constexpr (MODE == MODE_INV) return p < 3 ? ZPair{3 + p, 6 + p, false, false} : p == 3 ? ZPair{0, 1, true, true} : ZPair{2, -1, true, false};
+    if constexpr (MODE == MODE_INV) return p < 3 ? ZPair{3 + p, 6 + p, false, false} : p == 3 ? ZPair{0, 1, true, true} : ZPair{2, -1, true, false};
     else return ZPair{p == 0 ? 0 : p == 1 ? 2 : p == 5 ? 1 : p + 1, p == 0 ? 1 : p == 1 ? 0 : p == 5 ? 2 : p + 4, p == 5, p == 1 || p == 5};
 }
 
@@ -47,8 +46,7 @@ template <int MODE> __device__ __forceinline__ ZPair zfield_pair(int p) {
 // single: one real field, stored without the separation of a pair.
 struct ZJob { int a, b; bool fold, single; };
 template <int MODE> __device__ __forceinline__ ZJob zfield_job(int j) {
-    if constexpr (MODE == MODE_ROT) return j == 0 ? ZJob{0, 1, false, false} : ZJob{3, -1, false, true};   // c_z over w_x (k4_in_field)
-    else if constexpr (MODE == MODE_ADV) return j == 0 ? ZJob{0, 1, false, false} : ZJob{2, -1, false, true};
+    if constexpr (MODE == MODE_ADV) return j == 0 ? ZJob{0, 1, false, false} : ZJob{2, -1, false, true};
     else if constexpr (MODE == MODE_INV) return j < 2 ? ZJob{2 * j, 2 * j + 1, false, false} : ZJob{4, -1, false, true};
     // 0 G_x = conv_x + i kz t13, 1 G_y, 2 G_z, 3 t11, 4 t12, 5 t13, 6 t22, 7 t23
     else return j == 0 ? ZJob{0, 5, true, false} : j == 1 ? ZJob{1, 7, true, false} : j == 2 ? ZJob{2, -1, true, false}
@@ -59,12 +57,7 @@ template <int MODE> __device__ __forceinline__ ZJob zfield_job(int j) {
 // real inputs of job p on return.
 template <typename T, int MODE>
 __device__ __forceinline__ void zfield_row(cx<T> (&v)[ZFieldForm<MODE>::NPAIR], const StepConsts &c, double (&mx)[4], double (&nut)[3]) {
-    if constexpr (MODE == MODE_ROT) {
-        const T uu = v[0].x, ox = v[0].y, vv = v[1].x, oy = v[1].y, ww = v[2].x, oz = v[2].y;
-        cfl_update<T>(mx, uu, vv, ww, c);
-        v[0] = mk<T>(oy * ww - oz * vv, oz * uu - ox * ww);
-        v[1] = mk<T>(ox * vv - oy * uu, T(0));
-    } else if constexpr (MODE == MODE_INV) {
+    if constexpr (MODE == MODE_INV) {
         // Invariants of G_ij = d_j u_i (src/HIT_LES.cpp:1297-1319, definitions
         // src/tensor_algebra.cpp:165-306, 356-358) and the eddy-viscosity statistics, in double.
         double G[3][3], S[3][3], O[3][3];
