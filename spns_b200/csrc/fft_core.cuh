@@ -15,7 +15,7 @@
 // Stockham autosort, stage (R, Ns): butterfly j, k = j mod Ns,
 //   inputs  x_r = in[j + r*L/R],  x_r *= w_L^{r*k*L/(Ns*R)},  y = DFT_R(x),
 //   outputs out[(j/Ns)*Ns*R + k + r*Ns] = y_r.
-// Radices 2, 3, 4, 6, 8, 12: the composite ones with a factor 3 use the
+// Radices 2, 3, 4, 6, 8, 12, and 16 in the uneven plan (has_uneven): those with a factor 3 use the
 // prime-factor (Good-Thomas) split 2x3 / 4x3, which needs no inner twiddles.
 // Twiddles: w^1 of a butterfly is read from a table w_L^m = exp(-2 pi i m/L)
 // computed on the host in extended precision.  Stage (R, Ns) needs w_L^{r k L/(Ns R)}

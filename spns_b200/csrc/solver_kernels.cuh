@@ -21,8 +21,8 @@
 //   K5 forward x : S1 (3)            -> S0 G (3)
 //   K6 sweep     : G, u, R^{n-1} [, u^{n-1}] -> 1/M^3, R, Coriolis, forcing,
 //                  AB2 or kappa-scheme predictor, projection -> u^{n+1}, R^n.
-// The rotational form (opt-in) carries u and the vorticity instead (5, 6 and 6
-// fields in K1, K2, K3).  LES (Smagorinsky) adds the SGS stress, whose
+// The rotational form (the default of DNS) carries u and the vorticity instead: K1 writes
+// six fields from five transforms, K2 six, K3 three over the first of them.  LES (Smagorinsky) adds the SGS stress, whose
 // divergence is folded into the forward passes (i kz t_i3 in K3, i ky t_i2 in
 // K4, i kx t_i1 in K5).
 #pragma once

@@ -16,11 +16,11 @@
 //     In single precision (T = f2) a thread transforms two neighbouring pencils with
 //     packed arithmetic.
 //   * The four physical slots (u, v, w_x, w_y) are thread-private and live in tensor
-//     memory beside the running CFL maxima (104 columns a warp).  They took 24 of
-//     the 168 registers and 12 KB of shared memory per pencil at length 768, which held the
+//     memory beside the running CFL maxima (104 columns a warp).  Two of them took 48 of
+//     the 168 registers and two 12 KB of shared memory per pencil at length 768, which held the
 //     pass to 12 warps per SM; now it is 16, and the slots' accesses leave the
 //     shared-memory pipe, the busiest one (77 % of its cycles; the FP64 pipe 44 %).
-//     Before and now: double 512^3 13.0 -> 11.5 ms, single 8.25 -> 7.2.
+//     Before and now: double 512^3 13.0 -> 11.5 ms, single 8.25 -> 7.2 (6.7 in waves).
 //   * c_z is transformed as soon as it is known (after the second pair) and written
 //     over the w_x field of the same pencil (S2 field 3, consumed at the first
 //     pair), so the forward y pass reads the nonlinear term from fields 0, 1, 3.
