@@ -91,9 +91,10 @@ def test_parity(box, monkeypatch):
 
 
 # several boxes of one z length with other mode and pencil counts (other dynamic shared memory of one
-# kernel), and one of another length
+# kernel), and boxes of other lengths; 72 x 72 pencils of 96 give blocks of half an SM's threads
 SIDE_BY_SIDE = {
-    0: [((128, 96, 125), (192, 144, 192)), ((64, 64, 96), (96, 96, 192)), ((64, 64, 256), (96, 96, 384))],
+    0: [((128, 96, 125), (192, 144, 192)), ((64, 64, 96), (96, 96, 192)), ((64, 64, 256), (96, 96, 384)),
+        ((48, 48, 64), (72, 72, 96)), ((48, 48, 63), (72, 72, 96))],
     1: [((128, 128, 125), (192, 192, 192)), ((128, 192, 96), (192, 288, 192)), ((96, 96, 256), (144, 144, 384))],
 }
 
