@@ -13,6 +13,12 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA GPU (B200, sm_100a)")
 
 
+def pytest_collection_modifyitems(items):
+    # The tests of the reference's driver need its sources and fail without them: they come last, so
+    # that a run that stops at the first failure has been through all the others.
+    items.sort(key=lambda item: item.path.name == "test_gpu_dropin.py")
+
+
 @pytest.fixture(scope="session")
 def oracle_lib():
     import oracle as O
